@@ -1990,7 +1990,7 @@ __device__ __forceinline__ void k_grad4_body(DevMesh m, DevState<R> s, DevParams
         const Grad4Stage st{sgeo + cl, sgat + tid, slim + tid, slimc + cl};
         if constexpr (HP_FAST(1)) {
             const unsigned bad = grad4_body<1>(m, s, P, i, q, active, &st);
-            if (__any_sync(0xffffffffu, bad)) grad4_body<0>(m, s, P, i, q, active, &st);
+            if (__any_sync(0xffffffffu, bad && active)) grad4_body<0>(m, s, P, i, q, active, &st);
         } else {
             grad4_body<0>(m, s, P, i, q, active, &st);
         }
@@ -2003,7 +2003,7 @@ __device__ __forceinline__ void k_grad4_body(DevMesh m, DevState<R> s, DevParams
         // the outputs are not inputs of this kernel, so a warp that flagged
         // an operand simply recomputes and overwrites them
         const unsigned bad = grad4_body<1>(m, s, P, i, q, active, nullptr);
-        if (__any_sync(0xffffffffu, bad)) grad4_body<0>(m, s, P, i, q, active, nullptr);
+        if (__any_sync(0xffffffffu, bad && active)) grad4_body<0>(m, s, P, i, q, active, nullptr);
     } else {
         grad4_body<0>(m, s, P, i, q, active, nullptr);
     }
@@ -2216,8 +2216,13 @@ __device__ __forceinline__ bool flux4_body(const DevMesh& m, const DevState<R>& 
 #pragma unroll
             for (int c = 0; c < 3; c++) rhs[6 + c] = rhs[6 + c] + (S)COL(s.qdrag, 3 * d + c)[i];
     }
+    // only lanes that store count: a lane past the last cell has read
+    // whatever follows the mesh in the columns (zero LSQ weights), and its
+    // flag would send the last warp of every mesh whose cell count is no
+    // multiple of 8 through the hardware-division body, which then is the
+    // whole launch's tail (2,058 cells: 26 -> 16 us a launch, between events)
     if constexpr (F == 1) {
-        if (__any_sync(0xffffffffu, bad)) return false;
+        if (__any_sync(0xffffffffu, bad && active)) return false;
     }
     if (!active) return true;
     const S dtbyvol = (S)s.s[case_of(m, i)].dt / TLS(TAIL_VOL, ldg(m.vol + i));
