@@ -172,7 +172,9 @@ int hp_step_timed(hp_handle *h, int32_t nsteps, double *device_ms);
 /* nsteps launched eagerly with a CUDA event between every two kernels;
  * accumulates device time and launch counts per kernel kind (nkinds >= 16:
  * prim_start, step_begin, smooth1, smooth2, bc_visc, visc, prim_stage, bc,
- * grad, flux, prim_end, step_end, serial, overset, halo, qrs). */
+ * grad, flux, prim_end, step_end, serial, overset, halo, qrs; step_begin runs
+ * inside smooth1, and step_end and the next step's prim_start inside
+ * prim_end, so the first two stay zero and prim_start counts none). */
 int hp_profile_steps(hp_handle *h, int32_t nsteps, double *ms_per_kind,
                      int64_t *launches_per_kind, int32_t nkinds);
 

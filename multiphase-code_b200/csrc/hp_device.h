@@ -131,6 +131,7 @@ struct DevScalars {
     double fcarry[10];                // stale-flux carry (aliased meshes)
     int err_flags;
     int cell1;                        // internal id of the case's cell 1
+    unsigned blocks_done;             // case 0: finished blocks of the step's closing pass
 };
 
 // R values per face record of the face-based variants: 48 bytes in FP32, read

@@ -1702,18 +1702,17 @@ extern "C" int hp_device_state(hp_handle* h, double** cu_dev, int64_t* ld) {
 extern "C" int hp_info(const hp_handle* h, int64_t* kernels_per_step, int64_t* device_bytes, int64_t* aliased) {
     if (!h) return HP_E_ARG;
     if (kernels_per_step) {
-        // k_step_begin, smooth x2, bc, visc, stages x (prim, bc, grad, flux), prim end,
-        // k_step_end, prim start
+        // smooth x2, bc, visc, stages x (prim, bc, grad, flux), closing prim
         // (the Jameson flux, myflux 3, computes no gradients)
         const int grad = h->prm.myorder == 2 && h->prm.myflux != 3 ? 1 : 0;
-        int64_t n = 1 + 2 + (h->nghosts ? 1 : 0) + (h->prm.inviscid ? 0 : 1);
+        int64_t n = 2 + (h->nghosts ? 1 : 0) + (h->prm.inviscid ? 0 : 1);
         int64_t per_stage = 1 + (h->nghosts ? 1 : 0) + grad + 1;
         if (h->aliased) per_stage += grad + 1;
         if (h->dm.nfringe > 0) per_stage += 1;
         if (h->dm.nface > 0)   // k_faceflux; or the scatter kernels of face modes 2 (one per colour), 3
             per_stage += h->dm.face_mode == 2 ? h->dm.ncolor : 1;
         if (h->dm.nface > 0 && !h->prm.inviscid && h->var->face_visc) n += 1;   // k_vis_gather
-        n += (int64_t)h->dp.nstage * per_stage + 3;
+        n += (int64_t)h->dp.nstage * per_stage + 1;
         if (h->aliased) n += 2;
         if (h->neq == 22) n += 2 + (int64_t)h->dp.nstage * (2 + (h->nghosts ? 1 : 0));   // k_qrs_*
         if (h->nwall > 0)   // FP64 wall layers: viscous once, gradients and fluxes per stage

@@ -319,26 +319,41 @@ __device__ __forceinline__ unsigned long long warp_max_u64(unsigned long long v)
     return v;
 }
 
-enum { PM_STAGE = 0, PM_START = 1, PM_END = 2 };
+enum { PM_STAGE = 0, PM_START = 1, PM_NEXT = 2 };
 
-// Element primitive pass.  PM_START adds the dt contribution of
-// src/main.F90:529-546; PM_END adds the max-norm residual of :605-611, the
-// cu = cn copy of :619-625 and |u_g(1)| of :641.
+// bit pattern of a cell's dt contribution (src/main.F90:529-546), ~0 for NaN
+__device__ __forceinline__ unsigned long long dt_key(const DevParams& P, const PrimV& q, double dl) {
+    const S ag = sqrt(((S)P.gamag * q.pg) / q.rog);
+    const S ap = sqrt(((S)P.gamap * (q.pp + (S)P.pinf)) / q.rop);
+    const S qg = sqrt(q.ug * q.ug + q.vg * q.vg + q.wg * q.wg);
+    const S qp = sqrt(q.up * q.up + q.vp * q.vp + q.wp * q.wp);
+    const S x = (S)dl / (mx2(ag, ap) + mx2(qg, qp));
+    return x == x ? (unsigned long long)__double_as_longlong((double)x) : ~0ull;
+}
+
+// Element primitive pass.  PM_STAGE: the recovery alone.  PM_START: with the
+// dt contribution of src/main.F90:529-546.  PM_NEXT: the end of a step and
+// the start of the next in one pass: the recovery, the max-norm residual of
+// src/main.F90:605-611, the cu = cn copy of :619-625 and |u_g(1)| of :641,
+// then the recovery of that state once more, as the next step opens
+// (:515-546).  The pass is bound by HBM; two passes wrote the primitives and
+// the state twice and read the state back in between (983,040 cells, between
+// events: FP64 parity 53 + 87 -> 92 us, mixed 62 + 95 -> 101 us).
 template <int MODE>
 __device__ __forceinline__ void k_prim_body(DevMesh m, DevState<R> s, DevParams P, int bid) {
-    __shared__ unsigned long long red[4][16];
+    __shared__ unsigned long long red[MODE == PM_NEXT ? 6 : 1][16];
     int i = bid * blockDim.x + threadIdx.x;
     unsigned long long kmin = ~0ull, kd[4] = {0, 0, 0, 0}, nanc = 0;
     if (i < m.neles) {
-        double c[10], u[10];
+        double c[10], u[4];
 #pragma unroll
         for (int k = 0; k < 10; k++) c[k] = COL(s.cn, k)[i];
         // cu is read before any store of this thread: the compiler cannot
         // prove cn, cu and the primitive columns disjoint, so a load after a
         // store would wait for it
-        if (MODE == PM_END) {
+        if (MODE == PM_NEXT) {
 #pragma unroll
-            for (int k = 0; k < 10; k++) u[k] = COL(s.cu, k)[i];
+            for (int k = 0; k < 4; k++) u[k] = COL(s.cu, k)[i];
         }
         PrimV q;
         double qm[3];
@@ -346,19 +361,7 @@ __device__ __forceinline__ void k_prim_body(DevMesh m, DevState<R> s, DevParams 
             qm[0] = COL(s.cn, 10)[i]; qm[1] = COL(s.cn, 14)[i]; qm[2] = COL(s.cn, 18)[i];
         }
         prim_full(c, q, P, P.five_phase ? qm : nullptr);
-#pragma unroll
-        for (int k = 0; k < 10; k++) COL(s.cn, k)[i] = c[k];
-        store_prims(m, s.pr, i, q);
-        if constexpr (sizeof(R) != sizeof(double)) store_prims(m, s.prr, i, q);
-        if (MODE == PM_START) {
-            S ag = sqrt(((S)P.gamag * q.pg) / q.rog);
-            S ap = sqrt(((S)P.gamap * (q.pp + (S)P.pinf)) / q.rop);
-            S qg = sqrt(q.ug * q.ug + q.vg * q.vg + q.wg * q.wg);
-            S qp = sqrt(q.up * q.up + q.vp * q.vp + q.wp * q.wp);
-            S x = (S)ldg(m.dl + i) / (mx2(ag, ap) + mx2(qg, qp));
-            if (x == x) kmin = (unsigned long long)__double_as_longlong((double)x);
-        }
-        if (MODE == PM_END) {
+        if (MODE == PM_NEXT) {
             bool bad = false;
 #pragma unroll
             for (int k = 0; k < 10; k++) {
@@ -380,7 +383,13 @@ __device__ __forceinline__ void k_prim_body(DevMesh m, DevState<R> s, DevParams 
             nanc = (bad && ldg(m.iblank + i) < HP_IBLANK_HALO1) ? 1 : 0;
             DevScalars& sc = s.s[case_of(m, i)];
             if (i == sc.cell1) sc.velmag = sqrt(q.ug * q.ug + q.vg * q.vg + q.wg * q.wg);
+            prim_full(c, q, P, P.five_phase ? qm : nullptr);
         }
+#pragma unroll
+        for (int k = 0; k < 10; k++) COL(s.cn, k)[i] = c[k];
+        store_prims(m, s.pr, i, q);
+        if constexpr (sizeof(R) != sizeof(double)) store_prims(m, s.prr, i, q);
+        if (MODE != PM_STAGE) kmin = dt_key(P, q, ldg(m.dl + i));
     }
     if (MODE == PM_STAGE) return;
     // a block whose cells belong to two cases of a batch reduces per thread
@@ -390,9 +399,8 @@ __device__ __forceinline__ void k_prim_body(DevMesh m, DevState<R> s, DevParams 
     if (c0 != c1) {
         if (i < m.neles) {
             DevScalars& sc = s.s[case_of(m, i)];
-            if (MODE == PM_START) {
-                if (kmin != ~0ull) atomicMin(&sc.dtmin_bits, kmin);
-            } else {
+            if (kmin != ~0ull) atomicMin(&sc.dtmin_bits, kmin);
+            if (MODE == PM_NEXT) {
                 for (int k = 0; k < 4; k++)
                     if (kd[k]) atomicMax(&sc.diff_bits[k], kd[k]);
                 if (nanc) atomicAdd(&sc.nan_count, nanc);
@@ -401,45 +409,40 @@ __device__ __forceinline__ void k_prim_body(DevMesh m, DevState<R> s, DevParams 
         return;
     }
     DevScalars* const S0 = s.s + c0;
-    int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    if (MODE == PM_START) {
-        kmin = warp_min_u64(kmin);
-        if (lane == 0) red[0][wid] = kmin;
-        __syncthreads();
-        if (wid == 0) {
-            unsigned long long v = lane < (int)(blockDim.x >> 5) ? red[0][lane] : ~0ull;
-            v = warp_min_u64(v);
-            if (lane == 0 && v != ~0ull) atomicMin(&S0->dtmin_bits, v);
-        }
-    } else {
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    constexpr int NR = MODE == PM_NEXT ? 6 : 1;   // dt, then the residuals and the NaN count
+    kmin = warp_min_u64(kmin);
+    if (MODE == PM_NEXT) {
 #pragma unroll
         for (int k = 0; k < 4; k++) kd[k] = warp_max_u64(kd[k]);
         for (int o = 16; o > 0; o >>= 1) nanc += __shfl_xor_sync(0xffffffffu, nanc, o);
-        if (lane == 0) {
-            for (int k = 0; k < 4; k++) red[k][wid] = kd[k];
+    }
+    if (lane == 0) {
+        red[0][wid] = kmin;
+        if (MODE == PM_NEXT) {
+#pragma unroll
+            for (int k = 0; k < 4; k++) red[1 + k][wid] = kd[k];
+            red[5][wid] = nanc;
         }
-        __shared__ unsigned long long nred[16];
-        if (lane == 0) nred[wid] = nanc;
-        __syncthreads();
-        if (wid == 0) {
-            int nw = blockDim.x >> 5;
-            for (int k = 0; k < 4; k++) {
-                unsigned long long v = lane < nw ? red[k][lane] : 0ull;
-                v = warp_max_u64(v);
-                if (lane == 0 && v) atomicMax(&S0->diff_bits[k], v);
-            }
-            unsigned long long c = lane < nw ? nred[lane] : 0ull;
-            for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
-            if (lane == 0 && c) atomicAdd(&S0->nan_count, c);
+    }
+    __syncthreads();
+    // warp r reduces value r over the block's warps (a block has at least
+    // two warps)
+    for (int r = wid; r < NR; r += nw) {
+        unsigned long long v = lane < nw ? red[r][lane] : (r == 0 ? ~0ull : 0ull);
+        if (r == 0) {
+            v = warp_min_u64(v);
+            if (lane == 0 && v != ~0ull) atomicMin(&S0->dtmin_bits, v);
+        } else if (r < 5) {
+            v = warp_max_u64(v);
+            if (lane == 0 && v) atomicMax(&S0->diff_bits[r - 1], v);
+        } else {
+            for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+            if (lane == 0 && v) atomicAdd(&S0->nan_count, v);
         }
     }
 }
-template <int MODE>
-__global__ void __launch_bounds__(512) k_prim(DevMesh m, DevState<R> s, DevParams P) {
-    k_prim_body<MODE>(m, s, P, blockIdx.x);
-}
-
-// dt = cfl * dtmin, time += dt (src/main.F90:521-556); one thread per case.
+// dt = cfl * dtmin, time += dt (src/main.F90:521-556).
 __device__ __forceinline__ void step_begin_case(DevScalars* sc, const DevParams& P, unsigned long long bits) {
     double dtmin = __longlong_as_double((long long)bits);
     sc->dt = dtmin * P.cfl;
@@ -448,29 +451,23 @@ __device__ __forceinline__ void step_begin_case(DevScalars* sc, const DevParams&
     sc->dtmin_bits = (unsigned long long)__double_as_longlong(1.0e8);
 }
 
-// One thread per case.  coupled: the cases are the parts of one mesh and all
-// take the minimum over all of them (the positive dt contributions order as
-// their bit patterns); launched as one block, which reads every case before
-// any is reset.
-__global__ void k_step_begin(DevState<R> s, DevParams P, int ncase, int coupled) {
+// Every case, by one block.  coupled: the cases are the parts of one mesh and
+// all take the minimum over all of them (the positive dt contributions order
+// as their bit patterns), read before any is reset.
+__device__ __forceinline__ void step_begin_block(DevScalars* s, const DevParams& P, int ncase, bool coupled) {
+    unsigned long long bits = ~0ull;
     if (coupled) {
-        unsigned long long bits = ~0ull;
-        for (int k = 0; k < ncase; k++) bits = min(bits, s.s[k].dtmin_bits);
+        for (int k = 0; k < ncase; k++) bits = min(bits, s[k].dtmin_bits);
         __syncthreads();
-        for (int c = threadIdx.x; c < ncase; c += blockDim.x) step_begin_case(s.s + c, P, bits);
-        return;
     }
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c < ncase) step_begin_case(s.s + c, P, s.s[c].dtmin_bits);
+    for (int c = threadIdx.x; c < ncase; c += blockDim.x) step_begin_case(s + c, P, coupled ? bits : s[c].dtmin_bits);
 }
 
-// per-step diagnostics and reset of the residual accumulators; one thread
-// per case (diag rows of case c start at c * max_diag).
-__device__ __forceinline__ void k_step_end_body(DevState<R> s, int ncase, int bid) {
-    const int c = bid * blockDim.x + threadIdx.x;
-    if (c >= ncase) return;
-    DevScalars* sc = s.s + c;
-    int k = sc->step_in_call;
+// per-step diagnostics and reset of the residual accumulators of one case
+// (diag rows of case c start at c * max_diag).
+__device__ __forceinline__ void step_end_case(const DevState<R>& s, int c) {
+    volatile DevScalars* sc = s.s + c;
+    const int k = sc->step_in_call;
     if (k < s.max_diag) {
         double* d = s.diag + 8 * ((size_t)c * s.max_diag + k);
         d[0] = sc->time; d[1] = sc->dt; d[2] = sc->velmag;
@@ -481,8 +478,25 @@ __device__ __forceinline__ void k_step_end_body(DevState<R> s, int ncase, int bi
     for (int j = 0; j < 4; j++) sc->diff_bits[j] = 0ull;
     sc->nan_count = 0ull;
 }
-__global__ void k_step_end(DevState<R> s, int ncase) {
-    k_step_end_body(s, ncase, blockIdx.x);
+
+// PM_NEXT: the block that finishes last writes the step's diagnostics (the
+// residuals are complete then), in place of a launch of its own, whose
+// fixed cost a small mesh pays on every step.  The counter of finished blocks
+// is case 0's, and that block leaves it at zero.
+template <int MODE>
+__global__ void __launch_bounds__(512) k_prim(DevMesh m, DevState<R> s, DevParams P) {
+    k_prim_body<MODE>(m, s, P, blockIdx.x);
+    if constexpr (MODE == PM_NEXT) {
+        __shared__ int last;
+        __threadfence();
+        __syncthreads();
+        if (threadIdx.x == 0) last = atomicAdd(&s.s->blocks_done, 1u) == gridDim.x - 1;
+        __syncthreads();
+        if (!last) return;
+        __threadfence();
+        for (int c = threadIdx.x; c < m.ncase; c += blockDim.x) step_end_case(s, c);
+        if (threadIdx.x == 0) s.s->blocks_done = 0u;
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -780,7 +794,10 @@ __device__ __forceinline__ void k_smooth1_body(DevMesh m, DevState<R> s, int bid
     COL(s.anu, 0)[i] = anu1;
     COL(s.anu, 1)[i] = anu2;
 }
-__global__ void __launch_bounds__(512) k_smooth1(DevMesh m, DevState<R> s) {
+// Block 0 also forms the step's dt, which no smoothing switch reads and every
+// later kernel of the step does.
+__global__ void __launch_bounds__(512) k_smooth1(DevMesh m, DevState<R> s, DevParams P) {
+    if (blockIdx.x == 0) step_begin_block(s.s, P, m.ncase, m.nhalo > 0);
 #if HP_JST_SETS
     const int half = (int)blockDim.x >> 1, set = (int)threadIdx.x >= half;
     const int i = blockIdx.x * half + ((int)threadIdx.x - set * half);
@@ -3068,14 +3085,11 @@ static void enqueue_step(const DevMesh& m, const void* stp, const DevParams& P, 
     const unsigned ge = grid_for(m.neles, cb), gf = grid_for(m.neles, b);
     const unsigned gg = grid_for(m.nghosts > 0 ? m.nghosts : 1, cb);
     EXCHANGE(HP_X_DT);
-    MARK(KK_STEP_BEGIN);
-    if (m.nhalo > 0) k_step_begin<<<1, 128, 0, st>>>(s, P, m.ncase, 1);
-    else k_step_begin<<<grid_for(m.ncase, 128), 128, 0, st>>>(s, P, m.ncase, 0);
-    // JST dissipation, src/sr_smooth.F90 (once per step)
+    // dt and time of every case (in k_smooth1), and JST dissipation, src/sr_smooth.F90 (once per step)
     if (m.aliased) { MARK(KK_SERIAL); k_smooth_copy_serial<<<1, 1, 0, st>>>(m, s, 0); }
     MARK(KK_SMOOTH1);
     const unsigned gj = HP_JST_SETS ? grid_for(2ll * m.neles, cb) : ge;   // two threads per cell
-    k_smooth1<<<gj, cb, 0, st>>>(m, s);
+    k_smooth1<<<gj, cb, 0, st>>>(m, s, P);
     if (m.aliased) { MARK(KK_SERIAL); k_smooth_copy_serial<<<1, 1, 0, st>>>(m, s, 1); }
     MARK(KK_SMOOTH2);
     k_smooth2<<<ge, cb, 0, st>>>(m, s, P);
@@ -3150,14 +3164,10 @@ static void enqueue_step(const DevMesh& m, const void* stp, const DevParams& P, 
         }
         EXCHANGE(HP_X_HALO);
     }
-    // src/main.F90:595-641: primitive, residual norms, cu = cn
+    // src/main.F90:595-641: primitive, residual norms, cu = cn, and the start
+    // of the next step: primitive + dt contributions
     MARK(KK_PRIM_END);
-    k_prim<PM_END><<<ge, cb, 0, st>>>(m, s, P);
-    MARK(KK_STEP_END);
-    k_step_end<<<grid_for(m.ncase, 128), 128, 0, st>>>(s, m.ncase);
-    // start of the next step: primitive + dt contributions
-    MARK(KK_PRIM_START);
-    k_prim<PM_START><<<ge, cb, 0, st>>>(m, s, P);
+    k_prim<PM_NEXT><<<ge, cb, 0, st>>>(m, s, P);
     MARK(KK_COUNT);
 }
 #undef MARK
@@ -3225,7 +3235,7 @@ __global__ void __launch_bounds__(128, HP_FUSED_MINB) k_step_fused(DevMesh m, De
 #define SYNC \
     if (!grid_sync(g)) return;
     // src/main.F90:521-556: dt and time of every case
-    PHASE(m.ncase, { const int c = vb * 128 + threadIdx.x; if (c < m.ncase) step_begin_case(s.s + c, P, s.s[c].dtmin_bits); })
+    if (blockIdx.x == 0) step_begin_block(s.s, P, m.ncase, false);
     SYNC
     PHASE(m.neles, k_smooth1_body(m, s, vb))
     SYNC
@@ -3273,11 +3283,10 @@ __global__ void __launch_bounds__(128, HP_FUSED_MINB) k_step_fused(DevMesh m, De
         }
         SYNC
     }
-    PHASE(m.neles, { k_prim_body<PM_END>(m, s, P, vb); __syncthreads(); })
+    PHASE(m.neles, { k_prim_body<PM_NEXT>(m, s, P, vb); __syncthreads(); })
     SYNC
-    PHASE(m.ncase, k_step_end_body(s, m.ncase, vb))
-    SYNC
-    PHASE(m.neles, { k_prim_body<PM_START>(m, s, P, vb); __syncthreads(); })
+    if (blockIdx.x == 0)
+        for (int c = threadIdx.x; c < m.ncase; c += blockDim.x) step_end_case(s, c);
 #undef PHASE
 #undef SYNC
 }
