@@ -28,6 +28,10 @@ enum { G_UG = 0, G_VG = 3, G_WG = 6, G_TG = 9, G_UP = 12, G_VP = 15,
 // face kind bits per cell, 4 bits per face: bit 0 = wall (ghost type 5),
 // bit 1 = MUSCL-reconstruct across the face (interior or partition ghost).
 enum { FK_WALL = 1, FK_RECON = 2 };
+// cell bits of the same word, set by the host where a least-squares weight,
+// determinant or centroid difference of the cell lies outside the range in
+// which the kernels' shared-reciprocal division is exact (LSQA, LSQB tables)
+enum { FK_LSQA_RANGE = 1 << 16, FK_LSQB_RANGE = 1 << 17 };
 
 struct DevParams {
     double gamag, gamap, pinf, cpp, cpg, prg, rrg, prp;
@@ -63,7 +67,13 @@ struct DevMesh {
     // once at set-up with the host's pow, as the reference evaluates it
     const double* eps2;     // [ld]
     const double* sc;       // [12][ld] face area vectors sc1x..sc4z
-    const double* fch;      // [12][ld] face centroids, 0.3333 factor (HLLC, VK)
+    // face centroids (0.3333 factor: HLLC, VK) minus the cell's centroid and
+    // minus the centroid of the face's neighbour: x of faces 1-4, then y, z
+    const double *fxo, *fxn;   // [12][ld]
+    // unit normal (x, y, z) and area of face 1, then 2, 3, 4; formed on the
+    // device by the variant that reads them (Variant::setup), null when the
+    // handle runs no FP64 flux kernel
+    const double* nrm;      // [16][ld]
     const double* fcv;      // [12][ld] face centroids, /3 (viscous)
     // geometry-only least-squares terms, evaluated once at set-up with the
     // reference's expressions: [0..3] weights, [4..9] a1 a2 a3 b1 b2 b3,
@@ -181,6 +191,7 @@ inline DevState<double> fp64_view(const DevState<R>& s) {
 // FP64 kernels over the wall-layer lists, provided by the FP64 variant and
 // called by the FP32-arithmetic variants' step.
 struct WallFp64 {
+    void (*setup)(const DevMesh&, cudaStream_t);
     void (*visc)(const DevMesh&, const DevState<double>&, const DevParams&, cudaStream_t);
     void (*grad)(const DevMesh&, const DevState<double>&, const DevParams&, cudaStream_t);
     void (*flux)(const DevMesh&, const DevState<double>&, const DevParams&, cudaStream_t, int stage);
@@ -227,6 +238,8 @@ struct Variant {
     // 1 when the viscous fluxes are evaluated once per face on meshes with a
     // face list (k_facevisc + k_vis_gather instead of one kernel)
     int face_visc;
+    // fills the tables that the flux kernels read (m.nrm), once per handle
+    void (*setup)(const DevMesh&, cudaStream_t);
     // fused step (one cooperative launch per step): the grid it runs with on
     // this device (blocks of 128 threads), and the launch of one step
     int (*fused_grid)(const DevMesh&, const DevParams&);

@@ -186,7 +186,9 @@ static void plan_arena(hp_handle* h, Arena& a, int neles, int nghosts, long long
     m.xc = (double*)a.take(ld * D); m.yc = (double*)a.take(ld * D); m.zc = (double*)a.take(ld * D);
     m.vol = (double*)a.take(ld * D); m.dl = (double*)a.take(ld * D); m.dd = (double*)a.take(ld * D);
     m.eps2 = (double*)a.take(ld * D);
-    m.sc = (double*)a.take(12 * ld * D); m.fch = (double*)a.take(12 * ld * D);
+    m.sc = (double*)a.take(12 * ld * D); m.fxo = (double*)a.take(12 * ld * D);
+    m.fxn = (double*)a.take(12 * ld * D);
+    m.nrm = gb == D || h->nwall > 0 ? (double*)a.take(16 * ld * D) : nullptr;
     m.fcv = (double*)a.take(12 * ld * D);
     m.dxn = (double*)a.take(12 * ld * D);
     m.lsqa = (double*)a.take(NLSQ * ld * D);
@@ -630,6 +632,44 @@ static int fill_case(const hp_mesh* mesh, const hp_params* params, Layout& L, Ca
 }
 
 
+namespace {
+inline unsigned blocks_for(long long n, int b) { return (unsigned)((n + b - 1) / b); }
+
+// Set-up, one thread per cell: the neighbour centroid differences of the
+// gradient and source LSQ (m.dxn), the face centroids (in m.fxn on entry)
+// minus the centroids of both sides (m.fxo, m.fxn), the subtractions that the
+// step's kernels would do on gathered centroids; and the range bits of m.fk:
+// weights and determinants in [2^-100, 2^101), centroid differences zero or
+// in [2^-100, 2^100).
+__global__ void __launch_bounds__(128) k_offsets(DevMesh m) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= m.neles) return;
+    const long long ld = m.ld;
+    double *dxn = const_cast<double*>(m.dxn), *fxo = const_cast<double*>(m.fxo), *fxn = const_cast<double*>(m.fxn);
+    const double* x[3] = {m.xc, m.yc, m.zc};
+    unsigned out = 0;
+    for (int f = 0; f < 4; f++) {
+        const int j = m.nc[f * ld + i];
+        for (int d = 0; d < 3; d++) {
+            const double xi = x[d][i], xj = x[d][j], fc = fxn[(4 * d + f) * ld + i];
+            const double dx = xj - xi;
+            dxn[(3 * f + d) * ld + i] = dx;
+            fxo[(4 * d + f) * ld + i] = fc - xi;
+            fxn[(4 * d + f) * ld + i] = fc - xj;
+            const double a = fabs(dx);
+            if (a != 0.0 && !(a >= 0x1p-100 && a < 0x1p100)) out = FK_LSQA_RANGE | FK_LSQB_RANGE;
+        }
+    }
+    for (int t = 0; t < 5; t++) {
+        const int k = t < 4 ? t : 10;
+        const double a = m.lsqa[k * ld + i], b = m.lsqb[k * ld + i];
+        if (!(a >= 0x1p-100 && a < 0x1p101)) out |= FK_LSQA_RANGE;
+        if (!(b >= 0x1p-100 && b < 0x1p101)) out |= FK_LSQB_RANGE;
+    }
+    if (out) const_cast<unsigned*>(m.fk)[i] |= out;
+}
+}  // namespace
+
 extern "C" int hp_create_batch(const hp_mesh* meshes, int32_t ncase, const hp_params* params, hp_handle** out) {
     g_create_error.clear();
     if (!meshes || !params || !out || ncase < 1) return fail(nullptr, HP_E_ARG, "null argument or no case");
@@ -869,7 +909,6 @@ extern "C" int hp_create_batch(const hp_mesh* meshes, int32_t ncase, const hp_pa
     cudaError_t e = cudaMemsetAsync(A.base, 0, A.size, st);
     if (e == cudaSuccess) e = up(m.nc, L.nc.data(), 4 * ld * I);
     if (e == cudaSuccess) e = up(m.snb, L.snb.data(), 4 * ld * I);
-    if (e == cudaSuccess) e = up(m.fk, L.fk.data(), ld * sizeof(unsigned));
     if (e == cudaSuccess) e = up(m.iblank, L.ib.data(), ld * I);
     if (e == cudaSuccess) e = up(m.xc, L.x.data(), ld * D);
     if (e == cudaSuccess) e = up(m.yc, L.y.data(), ld * D);
@@ -883,22 +922,17 @@ extern "C" int hp_create_batch(const hp_mesh* meshes, int32_t ncase, const hp_pa
     if (e == cudaSuccess) e = up(m.eps2, L.eps2.data(), ld * D);
     if (e == cudaSuccess) e = up(m.dd, L.dd.data(), ld * D);
     if (e == cudaSuccess) e = up(m.sc, L.sc.data(), 12 * ld * D);
-    if (e == cudaSuccess) e = up(m.fch, L.fch.data(), 12 * ld * D);
     if (e == cudaSuccess) e = up(m.fcv, L.fcv.data(), 12 * ld * D);
-    // neighbour centroid differences of the FP64 gradient and source LSQ
-    // (the subtraction the kernels would do on the gathered centroids)
-    std::vector<double> hdxn(12 * (size_t)ld, 0.0);
-#pragma omp parallel for schedule(static)
-    for (long long t = 0; t < neles; t++)
-        for (int f = 0; f < 4; f++) {
-            const int j = L.nc[(size_t)f * ld + t];
-            hdxn[(size_t)(3 * f) * ld + t] = L.x[j] - L.x[t];
-            hdxn[(size_t)(3 * f + 1) * ld + t] = L.y[j] - L.y[t];
-            hdxn[(size_t)(3 * f + 2) * ld + t] = L.z[j] - L.z[t];
-        }
-    if (e == cudaSuccess) e = up(m.dxn, hdxn.data(), 12 * ld * D);
     if (e == cudaSuccess) e = up(m.lsqa, L.la.data(), NLSQ * ld * D);
     if (e == cudaSuccess) e = up(m.lsqb, L.lb.data(), NLSQ * ld * D);
+    if (e == cudaSuccess) e = up(m.fk, L.fk.data(), ld * sizeof(unsigned));
+    if (e == cudaSuccess) e = up(m.fxn, L.fch.data(), 12 * ld * D);
+    if (e == cudaSuccess) {
+        k_offsets<<<blocks_for(neles, 128), 128, 0, st>>>(m);
+        if (gb == D) h->var->setup(m, st);
+        else wall_fp64.setup(m, st);
+        e = cudaGetLastError();
+    }
     if (e == cudaSuccess && nghosts) e = up(m.g_par, L.gpar.data(), nghosts * (size_t)I);
     if (e == cudaSuccess && nghosts) e = up(m.g_id, L.gid.data(), nghosts * (size_t)I);
     if (e == cudaSuccess && nghosts) e = up(m.g_type, L.gtyp.data(), nghosts * (size_t)I);
@@ -1061,7 +1095,6 @@ __global__ void k_copy_cols(double* __restrict__ dst, const double* __restrict__
     int k = (int)(t / count), i = (int)(t - (long long)k * count);
     dst[(size_t)k * ld + start + i] = src[(size_t)k * ld + start + i];
 }
-inline unsigned blocks_for(long long n, int b) { return (unsigned)((n + b - 1) / b); }
 const Cols6 GHOST_COLS = {{P_UG, P_VG, P_WG, P_PG, P_TG, P_ROG}};
 }  // namespace
 

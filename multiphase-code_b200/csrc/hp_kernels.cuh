@@ -139,6 +139,61 @@ __device__ __forceinline__ double mrcp_tab(double b, double rbt, unsigned& bad) 
 template <int F> __device__ __forceinline__ float mrcp_tab(float b, float, unsigned& bad) {
     return mrcp<F>(b, bad);
 }
+// The quotient of mdiv for a positive divisor whose range the caller knows
+// (b in [2^-100, 2^101), rb = RN(1/b)), with the dividend's range tested
+// apart (mout, mpos: |a| in [2^-800, 2^801) puts the quotient and both
+// residuals inside the normal range).  The residuals are taken with the
+// other sign, b q - a: an exact zero then keeps the dividend's sign through
+// both corrections (a = -0: q0 = -0, residual +0, correction -0), so no
+// select is needed.  Quotients that share a dividend share its test, and a
+// value that is positive by nature needs no test for zero.
+template <int F>
+__device__ __forceinline__ double mquo(double a, double b, double rb) {
+    if constexpr (F == 0) {
+        (void)rb;
+        return a / b;
+    } else {
+        const double q0 = a * rb;
+        const double q1 = fma(-fma(b, q0, -a), rb, q0);
+        double q2 = fma(-fma(b, q1, -a), rb, q1);
+        // opaque to the compiler, as mdiv's selected result is: in the
+        // variant built with contraction the caller's sums then contract
+        // as they do around mdiv
+        asm("" : "+d"(q2));
+        return q2;
+    }
+}
+template <int F> __device__ __forceinline__ float mquo(float a, float, float rb) { return a * rb; }
+// flags a dividend that is neither zero nor within 2^[lo, hi) in magnitude
+template <int F, int LO = -800, int HI = 801>
+__device__ __forceinline__ void mout(double a, unsigned& bad) {
+    if constexpr (F != 0) {
+        const unsigned h = (unsigned)__double2hiint(a), l = (unsigned)__double2loint(a);
+        const bool nz = ((h & 0x7fffffffu) | l) != 0u;
+        bad |= (unsigned)(nz && (h << 1) - ((unsigned)(LO + 1023) << 21) >= ((unsigned)(HI - LO) << 21));
+    }
+}
+template <int F, int LO = -800, int HI = 801> __device__ __forceinline__ void mout(float, unsigned&) {}
+// flags a value that is not within [2^lo, 2^hi): zero and negative ones too
+template <int F, int LO = -800, int HI = 801>
+__device__ __forceinline__ void mpos(double a, unsigned& bad) {
+    if constexpr (F != 0)
+        bad |= (unsigned)((unsigned)__double2hiint(a) - ((unsigned)(LO + 1023) << 20) >= ((unsigned)(HI - LO) << 20));
+}
+template <int F, int LO = -800, int HI = 801> __device__ __forceinline__ void mpos(float, unsigned&) {}
+// a quotient with its dividend's test
+template <int F, class T>
+__device__ __forceinline__ T star_quo(T a, T b, T rb, unsigned& bad) {
+    mout<F>(a, bad);
+    return mquo<F>(a, b, rb);
+}
+// RN(1/b) of a positive divisor in [2^-100, 2^101); any other is flagged
+template <int F> __device__ __forceinline__ double mrcpp(double b, unsigned& bad) {
+    if constexpr (F == 0) return 0.0;
+    mpos<F, -100, 101>(b, bad);
+    return 1.0 / b;
+}
+template <int F> __device__ __forceinline__ float mrcpp(float b, unsigned&) { return 1.0f / b; }
 // the mixed variant divides approximately
 template <int F> __device__ __forceinline__ float mdiv(float a, float b, float rb, unsigned&) { return a * rb; }
 template <int F> __device__ __forceinline__ float mrcp(float b, unsigned&) { return 1.0f / b; }
@@ -980,9 +1035,9 @@ __device__ __forceinline__ void k_grad_body(DevMesh m, DevState<R> s, DevParams 
     R fx[4], fy[4], fz[4];
 #pragma unroll
     for (int f = 0; f < 4; f++) {
-        fx[f] = (R)(ldg(COL(m.fch, f) + i) - x0);
-        fy[f] = (R)(ldg(COL(m.fch, 4 + f) + i) - y0);
-        fz[f] = (R)(ldg(COL(m.fch, 8 + f) + i) - z0);
+        fx[f] = (R)ldg(COL(m.fxo, f) + i);
+        fy[f] = (R)ldg(COL(m.fxo, 4 + f) + i);
+        fz[f] = (R)ldg(COL(m.fxo, 8 + f) + i);
     }
     const int lv[4] = {8, 9, 11, 12};   // pg, pp, rog, rop rows of gv
     R phi = R(0);
@@ -1187,12 +1242,24 @@ __device__ __forceinline__ void face_eval(const DevMesh& m, const DevState<R>& s
                                           int i, int f, FaceOut& o, unsigned& bad, const PT* pr) {
     const int neigh = ldg(COL(m.nc, f) + i);
     const unsigned kind = (ldg(m.fk + i) >> (4 * f)) & 0xFu;
-    const double scxd = ldg(COL(m.sc, 3 * f) + i), scyd = ldg(COL(m.sc, 3 * f + 1) + i),
-                 sczd = ldg(COL(m.sc, 3 * f + 2) + i);
-    const R scx = (R)scxd, scy = (R)scyd, scz = (R)sczd;
-    const R area = sqrt(scx * scx + scy * scy + scz * scz);
-    const R rarea = mrcp<F>(area, bad);
-    const R enx = mdiv<F>(scx, area, rarea, bad), eny = mdiv<F>(scy, area, rarea, bad), enz = mdiv<F>(scz, area, rarea, bad);
+    // FP64: unit normal and area from the set-up table (the square root and
+    // the three divisions were 7% of the FP64 flux kernel's instructions);
+    // FP32: formed here, where its approximate divisions cost little
+    R area, enx, eny, enz;
+    if constexpr (sizeof(R) == 8) {
+        enx = ldg(COL(m.nrm, 4 * f) + i);
+        eny = ldg(COL(m.nrm, 4 * f + 1) + i);
+        enz = ldg(COL(m.nrm, 4 * f + 2) + i);
+        area = ldg(COL(m.nrm, 4 * f + 3) + i);
+    } else {
+        const R scx = (R)ldg(COL(m.sc, 3 * f) + i), scy = (R)ldg(COL(m.sc, 3 * f + 1) + i),
+                scz = (R)ldg(COL(m.sc, 3 * f + 2) + i);
+        area = sqrt(scx * scx + scy * scy + scz * scz);
+        const R rarea = mrcp<F>(area, bad);
+        enx = mdiv<F>(scx, area, rarea, bad);
+        eny = mdiv<F>(scy, area, rarea, bad);
+        enz = mdiv<F>(scz, area, rarea, bad);
+    }
     R ugL = (R)PLD(COL(pr, P_UG) + i), vgL = (R)PLD(COL(pr, P_VG) + i), wgL = (R)PLD(COL(pr, P_WG) + i);
     R tgL = (R)PLD(COL(pr, P_TG) + i), phigL = (R)PLD(COL(pr, P_PHIG) + i);
     R upL = (R)PLD(COL(pr, P_UP) + i), vpL = (R)PLD(COL(pr, P_VP) + i), wpL = (R)PLD(COL(pr, P_WP) + i);
@@ -1282,11 +1349,12 @@ __device__ __forceinline__ void face_eval(const DevMesh& m, const DevState<R>& s
     }
     if (P.myorder == 2 && (kind & FK_RECON)) {
         const R phimin = (R)mn2(PLD(s.phi + i), PLD(s.phi + neigh));
-        const double xf = ldg(COL(m.fch, f) + i), yf = ldg(COL(m.fch, 4 + f) + i),
-                     zf = ldg(COL(m.fch, 8 + f) + i);
-        const R xf0 = (R)(xf - ldg(m.xc + i)), yf0 = (R)(yf - ldg(m.yc + i)), zf0 = (R)(zf - ldg(m.zc + i));
-        const R xfn = (R)(xf - ldg(m.xc + neigh)), yfn = (R)(yf - ldg(m.yc + neigh)),
-                zfn = (R)(zf - ldg(m.zc + neigh));
+        // face centroid minus each side's centroid (set-up tables: the
+        // neighbour's centroid would be three more gathers)
+        const R xf0 = (R)ldg(COL(m.fxo, f) + i), yf0 = (R)ldg(COL(m.fxo, 4 + f) + i),
+                zf0 = (R)ldg(COL(m.fxo, 8 + f) + i);
+        const R xfn = (R)ldg(COL(m.fxn, f) + i), yfn = (R)ldg(COL(m.fxn, 4 + f) + i),
+                zfn = (R)ldg(COL(m.fxn, 8 + f) + i);
         const R* g = s.gr;
 #define REC(v, X, Y, Z, G, c) \
     v = v + phimin * (X * PLD(COL(g, G) + c) + Y * PLD(COL(g, G + 1) + c) + Z * PLD(COL(g, G + 2) + c))
@@ -1342,27 +1410,37 @@ __device__ __forceinline__ void face_eval(const DevMesh& m, const DevState<R>& s
     // the gas phase's wave speeds and HLLC first, then the liquid's: each
     // phase's quantities are live only while it is evaluated (the values and
     // their order of evaluation are those of src/sr_hllcbatten.F90:338-529)
-    R egL = mdiv<F>(rrg * tgL, gamag - R(1), rgm1, bad) + R(0.5) * (ugL * ugL + vgL * vgL + wgL * wgL);
-    const R rrogL = mrcp<F>(rogL, bad), rrogR = mrcp<F>(rogR, bad);
-    R hgL = egL + mdiv<F>(pgL, rogL, rrogL, bad);
+    // (dividends are tested once each: the pressures and temperatures, times
+    // a constant of order one, serve two quotients, and a gas pressure or a
+    // temperature that is not positive is left to hardware division)
+    const R gm1 = gamag - R(1);
+    mpos<F, -100, 101>(gm1, bad);
+    mpos<F, -800, 600>(tgL, bad); mpos<F, -800, 600>(pgL, bad);
+    mpos<F, -800, 600>(tgR, bad); mpos<F, -800, 600>(pgR, bad);
+    R egL = mquo<F>(rrg * tgL, gm1, rgm1) + R(0.5) * (ugL * ugL + vgL * vgL + wgL * wgL);
+    const R rrogL = mrcpp<F>(rogL, bad), rrogR = mrcpp<F>(rogR, bad);
+    R hgL = egL + mquo<F>(pgL, rogL, rrogL);
     R qgL = ugL * enx + vgL * eny + wgL * enz;
-    R agL = sqrt(mdiv<F>(gamag * pgL, rogL, rrogL, bad));
-    R egR = mdiv<F>(rrg * tgR, gamag - R(1), rgm1, bad) + R(0.5) * (ugR * ugR + vgR * vgR + wgR * wgR);
-    R hgR = egR + mdiv<F>(pgR, rogR, rrogR, bad);
+    R agL = sqrt(mquo<F>(gamag * pgL, rogL, rrogL));
+    R egR = mquo<F>(rrg * tgR, gm1, rgm1) + R(0.5) * (ugR * ugR + vgR * vgR + wgR * wgR);
+    R hgR = egR + mquo<F>(pgR, rogR, rrogR);
     R qgR = ugR * enx + vgR * eny + wgR * enz;
-    R agR = sqrt(mdiv<F>(gamag * pgR, rogR, rrogR, bad));
+    R agR = sqrt(mquo<F>(gamag * pgR, rogR, rrogR));
 #define HP_LIQUID_WAVES \
-    const R rropL = mrcp<F>(ropL, bad), rropR = mrcp<F>(ropR, bad); \
-    R epL = mdiv<F>(cpp * tpL, gamap, rgamap, bad) + mdiv<F>(pinf, ropL, rropL, bad) + \
+    mpos<F, -100, 101>(gamap, bad); mout<F>(pinf, bad); \
+    mpos<F>(cpp * tpL, bad); mpos<F, -800, 600>(ppL + pinf, bad); mout<F>(ppL, bad); \
+    mpos<F>(cpp * tpR, bad); mpos<F, -800, 600>(ppR + pinf, bad); mout<F>(ppR, bad); \
+    const R rropL = mrcpp<F>(ropL, bad), rropR = mrcpp<F>(ropR, bad); \
+    R epL = mquo<F>(cpp * tpL, gamap, rgamap) + mquo<F>(pinf, ropL, rropL) + \
             R(0.5) * (upL * upL + vpL * vpL + wpL * wpL); \
-    R hpL = epL + mdiv<F>(ppL, ropL, rropL, bad); \
+    R hpL = epL + mquo<F>(ppL, ropL, rropL); \
     R qpL = upL * enx + vpL * eny + wpL * enz; \
-    R apL = sqrt(mdiv<F>(gamap * (ppL + pinf), ropL, rropL, bad)); \
-    R epR = mdiv<F>(cpp * tpR, gamap, rgamap, bad) + mdiv<F>(pinf, ropR, rropR, bad) + \
+    R apL = sqrt(mquo<F>(gamap * (ppL + pinf), ropL, rropL)); \
+    R epR = mquo<F>(cpp * tpR, gamap, rgamap) + mquo<F>(pinf, ropR, rropR) + \
             R(0.5) * (upR * upR + vpR * vpR + wpR * wpR); \
-    R hpR = epR + mdiv<F>(ppR, ropR, rropR, bad); \
+    R hpR = epR + mquo<F>(ppR, ropR, rropR); \
     R qpR = upR * enx + vpR * eny + wpR * enz; \
-    R apR = sqrt(mdiv<F>(gamap * (ppR + pinf), ropR, rropR, bad));
+    R apR = sqrt(mquo<F>(gamap * (ppR + pinf), ropR, rropR));
     if constexpr (Z == 1) {
         HP_LIQUID_WAVES
         zien_flux<F>(o, bad, area, enx, eny, enz, phigL, phipL, rogL, ropL, ugL, vgL, wgL, upL, vpL, wpL, pgL,
@@ -1392,13 +1470,13 @@ __device__ __forceinline__ void face_eval(const DevMesh& m, const DevState<R>& s
                 o.F[0] = fl0 * area; o.F[1] = fl1 * area; o.F[2] = fl2 * area;
                 o.F[3] = fl3 * area; o.F[4] = fl4 * area;
             } else {
-                R dnrg = (sgstar - sgl) + eps6;
-                const R rd = mrcp<F>(dnrg, bad);
-                R cs0 = mdiv<F>((qgL - sgl) * cn0, dnrg, rd, bad);
-                R cs1 = mdiv<F>((qgL - sgl) * cn1 + phigL * (pgL * enx - pgstar * enx), dnrg, rd, bad);
-                R cs2 = mdiv<F>((qgL - sgl) * cn2 + phigL * (pgL * eny - pgstar * eny), dnrg, rd, bad);
-                R cs3 = mdiv<F>((qgL - sgl) * cn3 + phigL * (pgL * enz - pgstar * enz), dnrg, rd, bad);
-                R cs4 = mdiv<F>((qgL - sgl) * cn4 + phigL * (pgL * qgL - pgstar * sgstar), dnrg, rd, bad);
+                const R dnrg = (sgstar - sgl) + eps6;
+                const R rd = mrcpp<F>(dnrg, bad);
+                R cs0 = star_quo<F>((qgL - sgl) * cn0, dnrg, rd, bad);
+                R cs1 = star_quo<F>((qgL - sgl) * cn1 + phigL * (pgL * enx - pgstar * enx), dnrg, rd, bad);
+                R cs2 = star_quo<F>((qgL - sgl) * cn2 + phigL * (pgL * eny - pgstar * eny), dnrg, rd, bad);
+                R cs3 = star_quo<F>((qgL - sgl) * cn3 + phigL * (pgL * enz - pgstar * enz), dnrg, rd, bad);
+                R cs4 = star_quo<F>((qgL - sgl) * cn4 + phigL * (pgL * qgL - pgstar * sgstar), dnrg, rd, bad);
                 o.F[0] = (fl0 + sgl * (cs0 - cn0)) * area;
                 o.F[1] = (fl1 + sgl * (cs1 - cn1)) * area;
                 o.F[2] = (fl2 + sgl * (cs2 - cn2)) * area;
@@ -1417,13 +1495,14 @@ __device__ __forceinline__ void face_eval(const DevMesh& m, const DevState<R>& s
                 o.F[0] = fr0 * area; o.F[1] = fr1 * area; o.F[2] = fr2 * area;
                 o.F[3] = fr3 * area; o.F[4] = fr4 * area;
             } else {
-                R dnrg = (sgstar - sgr) + eps6;
-                const R rd = mrcp<F>(dnrg, bad);
-                R cs0 = mdiv<F>((qgR - sgr) * cn0, dnrg, rd, bad);
-                R cs1 = mdiv<F>((qgR - sgr) * cn1 + phigR * (pgR * enx - pgstar * enx), dnrg, rd, bad);
-                R cs2 = mdiv<F>((qgR - sgr) * cn2 + phigR * (pgR * eny - pgstar * eny), dnrg, rd, bad);
-                R cs3 = mdiv<F>((qgR - sgr) * cn3 + phigR * (pgR * enz - pgstar * enz), dnrg, rd, bad);
-                R cs4 = mdiv<F>((qgR - sgr) * cn4 + phigR * (pgR * qgR - pgstar * sgstar), dnrg, rd, bad);
+                // a negative divisor: minus the quotient by its opposite
+                const R dnrg = -((sgstar - sgr) + eps6);
+                const R rd = mrcpp<F>(dnrg, bad);
+                R cs0 = -star_quo<F>((qgR - sgr) * cn0, dnrg, rd, bad);
+                R cs1 = -star_quo<F>((qgR - sgr) * cn1 + phigR * (pgR * enx - pgstar * enx), dnrg, rd, bad);
+                R cs2 = -star_quo<F>((qgR - sgr) * cn2 + phigR * (pgR * eny - pgstar * eny), dnrg, rd, bad);
+                R cs3 = -star_quo<F>((qgR - sgr) * cn3 + phigR * (pgR * enz - pgstar * enz), dnrg, rd, bad);
+                R cs4 = -star_quo<F>((qgR - sgr) * cn4 + phigR * (pgR * qgR - pgstar * sgstar), dnrg, rd, bad);
                 o.F[0] = (fr0 + sgr * (cs0 - cn0)) * area;
                 o.F[1] = (fr1 + sgr * (cs1 - cn1)) * area;
                 o.F[2] = (fr2 + sgr * (cs2 - cn2)) * area;
@@ -1456,13 +1535,13 @@ __device__ __forceinline__ void face_eval(const DevMesh& m, const DevState<R>& s
                 o.F[5] = fl0 * area; o.F[6] = fl1 * area; o.F[7] = fl2 * area;
                 o.F[8] = fl3 * area; o.F[9] = fl4 * area;
             } else {
-                R dnrp = (spstar - spl) + eps6;
-                const R rd = mrcp<F>(dnrp, bad);
-                R cs0 = mdiv<F>((qpL - spl) * cn0, dnrp, rd, bad);
-                R cs1 = mdiv<F>((qpL - spl) * cn1 + phipL * (ppL * enx - ppstar * enx), dnrp, rd, bad);
-                R cs2 = mdiv<F>((qpL - spl) * cn2 + phipL * (ppL * eny - ppstar * eny), dnrp, rd, bad);
-                R cs3 = mdiv<F>((qpL - spl) * cn3 + phipL * (ppL * enz - ppstar * enz), dnrp, rd, bad);
-                R cs4 = mdiv<F>((qpL - spl) * cn4 + phipL * (ppL * qpL - ppstar * spstar), dnrp, rd, bad);
+                const R dnrp = (spstar - spl) + eps6;
+                const R rd = mrcpp<F>(dnrp, bad);
+                R cs0 = star_quo<F>((qpL - spl) * cn0, dnrp, rd, bad);
+                R cs1 = star_quo<F>((qpL - spl) * cn1 + phipL * (ppL * enx - ppstar * enx), dnrp, rd, bad);
+                R cs2 = star_quo<F>((qpL - spl) * cn2 + phipL * (ppL * eny - ppstar * eny), dnrp, rd, bad);
+                R cs3 = star_quo<F>((qpL - spl) * cn3 + phipL * (ppL * enz - ppstar * enz), dnrp, rd, bad);
+                R cs4 = star_quo<F>((qpL - spl) * cn4 + phipL * (ppL * qpL - ppstar * spstar), dnrp, rd, bad);
                 o.F[5] = (fl0 + spl * (cs0 - cn0)) * area;
                 o.F[6] = (fl1 + spl * (cs1 - cn1)) * area;
                 o.F[7] = (fl2 + spl * (cs2 - cn2)) * area;
@@ -1481,13 +1560,14 @@ __device__ __forceinline__ void face_eval(const DevMesh& m, const DevState<R>& s
                 o.F[5] = fr0 * area; o.F[6] = fr1 * area; o.F[7] = fr2 * area;
                 o.F[8] = fr3 * area; o.F[9] = fr4 * area;
             } else {
-                R dnrp = (spstar - spr) + eps6;
-                const R rd = mrcp<F>(dnrp, bad);
-                R cs0 = mdiv<F>((qpR - spr) * cn0, dnrp, rd, bad);
-                R cs1 = mdiv<F>((qpR - spr) * cn1 + phipR * (ppR * enx - ppstar * enx), dnrp, rd, bad);
-                R cs2 = mdiv<F>((qpR - spr) * cn2 + phipR * (ppR * eny - ppstar * eny), dnrp, rd, bad);
-                R cs3 = mdiv<F>((qpR - spr) * cn3 + phipR * (ppR * enz - ppstar * enz), dnrp, rd, bad);
-                R cs4 = mdiv<F>((qpR - spr) * cn4 + phipR * (ppR * qpR - ppstar * spstar), dnrp, rd, bad);
+                // a negative divisor: minus the quotient by its opposite
+                const R dnrp = -((spstar - spr) + eps6);
+                const R rd = mrcpp<F>(dnrp, bad);
+                R cs0 = -star_quo<F>((qpR - spr) * cn0, dnrp, rd, bad);
+                R cs1 = -star_quo<F>((qpR - spr) * cn1 + phipR * (ppR * enx - ppstar * enx), dnrp, rd, bad);
+                R cs2 = -star_quo<F>((qpR - spr) * cn2 + phipR * (ppR * eny - ppstar * eny), dnrp, rd, bad);
+                R cs3 = -star_quo<F>((qpR - spr) * cn3 + phipR * (ppR * enz - ppstar * enz), dnrp, rd, bad);
+                R cs4 = -star_quo<F>((qpR - spr) * cn4 + phipR * (ppR * qpR - ppstar * spstar), dnrp, rd, bad);
                 o.F[5] = (fr0 + spr * (cs0 - cn0)) * area;
                 o.F[6] = (fr1 + spr * (cs1 - cn1)) * area;
                 o.F[7] = (fr2 + spr * (cs2 - cn2)) * area;
@@ -1741,12 +1821,12 @@ __global__ void __launch_bounds__(128) k_flux(DevMesh m, DevState<R> s, DevParam
 // another lane), over its four faces; lane 0 stores the cell's minimum.
 // lp, lc (the staged kernel, below): the limiter field of the lane's cell
 // and of its four neighbours (lp[k * LIM_LD], k = 0 the cell) and the cell's
-// face centroids and epsilon^2 (lc[k * LIMC_LD], k = 0..11 fch, 12 eps2),
+// face centroid offsets and epsilon^2 (lc[k * LIMC_LD], k = 0..11 fxo, 12 eps2),
 // copied to shared memory when the kernel started; null: read from global
 // memory
 __device__ __forceinline__ unsigned grad4_limiter(const DevMesh& m, const DevState<R>& s, const DevParams& P,
-                                                  int i, int q, bool active, const int n[4], double x0,
-                                                  double y0, double z0, R lg[3], const R sg[3],
+                                                  int i, int q, bool active, const int n[4], R lg[3],
+                                                  const R sg[3],
                                                   const double* lp, const double* lc) {
     // lane 2 takes rog from lane 3, lane 3 takes rop from lane 0
     const int src = q == 2 ? 3 : (q == 3 ? 0 : q);
@@ -1768,9 +1848,9 @@ __device__ __forceinline__ unsigned grad4_limiter(const DevMesh& m, const DevSta
     R phl = R(0);
 #pragma unroll
     for (int f = 0; f < 4; f++) {
-        R fx = (R)((lc ? lc[f * LIMC_LD] : ldg(COL(m.fch, f) + i)) - x0);
-        R fy = (R)((lc ? lc[(4 + f) * LIMC_LD] : ldg(COL(m.fch, 4 + f) + i)) - y0);
-        R fz = (R)((lc ? lc[(8 + f) * LIMC_LD] : ldg(COL(m.fch, 8 + f) + i)) - z0);
+        R fx = (R)(lc ? lc[f * LIMC_LD] : ldg(COL(m.fxo, f) + i));
+        R fy = (R)(lc ? lc[(4 + f) * LIMC_LD] : ldg(COL(m.fxo, 4 + f) + i));
+        R fz = (R)(lc ? lc[(8 + f) * LIMC_LD] : ldg(COL(m.fxo, 8 + f) + i));
         R d = fx * lg[0] + fy * lg[1] + fz * lg[2];
         R ph;
         if (d > R(0)) ph = fvenkat(dmax, d, epssq);
@@ -1820,7 +1900,6 @@ __device__ __forceinline__ unsigned grad4_body(const DevMesh& m, const DevState<
     int n[4];
 #pragma unroll
     for (int f = 0; f < 4; f++) n[f] = ldg(COL(m.nc, f) + i);
-    const double x0 = ldg(m.xc + i), y0 = ldg(m.yc + i), z0 = ldg(m.zc + i);
 #if GRAD4_STAGED
     if constexpr (sizeof(R) == sizeof(double)) {
         const double* geo = st->geo;
@@ -1831,10 +1910,14 @@ __device__ __forceinline__ unsigned grad4_body(const DevMesh& m, const DevState<
 #define GZ(f) geo[(3 * (f) + 2) * GEO_LD]
 #define GT(j) geo[(12 + (j)) * GEO_LD]
 #undef DW
-#define DW(x, f) mdiv<F>((x), GT(f), GT(11 + (f)), bad)
-#pragma unroll
-        for (int f = 0; f < 4; f++) (void)mrcp_tab<F>(GT(f), GT(11 + f), bad);
-        (void)mrcp_tab<F>(GT(10), GT(15), bad);
+#define DW(x, f) mquo<F>((x), GT(f), GT(11 + (f)))
+        // the weights, the determinant and the centroid differences were
+        // tested at set-up, so a field needs tests of its four differences
+        // and of the three determinants, in place of one per quotient (a
+        // difference in 2^[-800, 700) times a centroid difference in
+        // 2^[-100, 100) stays in 2^[-900, 800), where the quotient and the
+        // residuals are still normal numbers)
+        if (F != 0) bad |= ldg(m.fk + i) & FK_LSQA_RANGE;
         R lg[3] = {R(0), R(0), R(0)};
         R sg[3] = {R(0), R(0), R(0)};
 #pragma unroll
@@ -1849,6 +1932,8 @@ __device__ __forceinline__ unsigned grad4_body(const DevMesh& m, const DevState<
             const R qi = (R)g[0];
             const R qa = (R)(g[LIM_LD] - qi), qb = (R)(g[2 * LIM_LD] - qi);
             const R qc = (R)(g[3 * LIM_LD] - qi), qd = (R)(g[4 * LIM_LD] - qi);
+            mout<F, -800, 700>(qa, bad); mout<F, -800, 700>(qb, bad);
+            mout<F, -800, 700>(qc, bad); mout<F, -800, 700>(qd, bad);
             R c1 = DW(qa * GX(0), 0) + DW(qb * GX(1), 1) + DW(qc * GX(2), 2) + DW(qd * GX(3), 3);
             R c2;
             if (v == 7)   // cTp2 lacks the /wt4 (src/sr_derivative.F90:225)
@@ -1858,9 +1943,11 @@ __device__ __forceinline__ unsigned grad4_body(const DevMesh& m, const DevState<
             R c3 = DW(qa * GZ(0), 0) + DW(qb * GZ(1), 1) + DW(qc * GZ(2), 2) + DW(qd * GZ(3), 3);
             const R a1 = GT(4), a2 = GT(5), a3 = GT(6), b1 = GT(7), b2 = GT(8), b3 = GT(9);
             const R dnr = GT(10), rdnr = GT(15);
-            R gx = mdiv<F>(det3(c1, c2, c3, b1, a2, b3, b2, b3, a3), dnr, rdnr, bad);
-            R gy = mdiv<F>(det3(a1, b1, b2, c1, c2, c3, b2, b3, a3), dnr, rdnr, bad);
-            R gz = mdiv<F>(det3(a1, b1, b2, b1, a2, b3, c1, c2, c3), dnr, rdnr, bad);
+            const R dx = det3(c1, c2, c3, b1, a2, b3, b2, b3, a3);
+            const R dy = det3(a1, b1, b2, c1, c2, c3, b2, b3, a3);
+            const R dz = det3(a1, b1, b2, b1, a2, b3, c1, c2, c3);
+            mout<F>(dx, bad); mout<F>(dy, bad); mout<F>(dz, bad);
+            const R gx = mquo<F>(dx, dnr, rdnr), gy = mquo<F>(dy, dnr, rdnr), gz = mquo<F>(dz, dnr, rdnr);
             if (v < 11 && active) {
                 COL(s.gr, 3 * v + 0)[i] = gx;
                 COL(s.gr, 3 * v + 1)[i] = gy;
@@ -1875,10 +1962,13 @@ __device__ __forceinline__ unsigned grad4_body(const DevMesh& m, const DevState<
 #undef GZ
 #undef GT
 #define DW(x, f) div_rn((x), wt[f], rw[f])
-        return bad | grad4_limiter(m, s, P, i, q, active, n, x0, y0, z0, lg, sg, st->lim, st->limc);
+        return bad | grad4_limiter(m, s, P, i, q, active, n, lg, sg, st->lim, st->limc);
     }
 #endif
     (void)st;
+#if !HP_DXN_TABLE
+    const double x0 = ldg(m.xc + i), y0 = ldg(m.yc + i), z0 = ldg(m.zc + i);
+#endif
     R xa[4], ya[4], za[4];
 #pragma unroll
     for (int f = 0; f < 4; f++) {
@@ -1955,7 +2045,7 @@ __device__ __forceinline__ unsigned grad4_body(const DevMesh& m, const DevState<
     }
 #undef DW
 #define DW(x, f) div_rn((x), wt[f], rw[f])
-    return bad | grad4_limiter(m, s, P, i, q, active, n, x0, y0, z0, lg, sg, nullptr, nullptr);
+    return bad | grad4_limiter(m, s, P, i, q, active, n, lg, sg, nullptr, nullptr);
 }
 
 
@@ -2008,7 +2098,7 @@ __device__ __forceinline__ void k_grad4_body(DevMesh m, DevState<R> s, DevParams
 #pragma unroll
         for (int f = 0; f < 4; f++) cp_async8(slim + (1 + f) * LIM_LD + tid, ql + nn[f]);
 #pragma unroll
-        for (int d = 0; d < 3; d++) cp_async8(slimc + (4 * d + q) * LIMC_LD + cl, COL(m.fch, 4 * d + q) + i);
+        for (int d = 0; d < 3; d++) cp_async8(slimc + (4 * d + q) * LIMC_LD + cl, COL(m.fxo, 4 * d + q) + i);
         if (q == 0) cp_async8(slimc + 12 * LIMC_LD + cl, m.eps2 + i);
         cp_async_commit();
         const Grad4Stage st{sgeo + cl, sgat + tid, slim + tid, slimc + cl};
@@ -2173,20 +2263,24 @@ __device__ __forceinline__ bool flux4_body(const DevMesh& m, const DevState<R>& 
         const R pq_ = q == 0 ? up : (q == 1 ? vp : wp);
         const R vq_int = (phig * rog * gq + omg * rop * pq_) / den;
         const R uint_ = qshfl(vq_int, 0), vint = qshfl(vq_int, 1), wint = qshfl(vq_int, 2);
-        // geometry-only terms (src/sr_source.F90:100-117), evaluated at set-up
+        // geometry-only terms (src/sr_source.F90:100-117), evaluated (and
+        // their ranges tested) at set-up
         R wt[4], rw[4];
 #undef DW
-#define DW(x, f) mdiv<F>((x), wt[f], rw[f], bad)
 #if HP_LSQ_TABLE
+#define DW(x, f) mquo<F>((x), wt[f], rw[f])
 #define LB(k) TL(TAIL_LSQB + (k), ldg(COL(m.lsqb, k) + i))
+        if (F != 0) bad |= ldg(m.fk + i) & FK_LSQB_RANGE;
 #pragma unroll
         for (int f = 0; f < 4; f++) {
+            mout<F, -800, 700>(pa[f], bad);
             wt[f] = LB(f);
-            rw[f] = mrcp_tab<F>(wt[f], LB(11 + f), bad);
+            rw[f] = LB(11 + f);
         }
         const R a1 = LB(4), a2 = LB(5), a3 = LB(6);
         const R b1 = LB(7), b2 = LB(8), b3 = LB(9);
 #else
+#define DW(x, f) mdiv<F>((x), wt[f], rw[f], bad)
 #pragma unroll
         for (int f = 0; f < 4; f++) { wt[f] = sqrt(xa[f] * xa[f] + ya[f] * ya[f] + za[f] * za[f]); rw[f] = mrcp<F>(wt[f], bad); }
         const R a1 = DW(xa[0] * xa[0], 0) + DW(xa[1] * xa[1], 1) + DW(xa[2] * xa[2], 2) + DW(xa[3] * xa[3], 3);
@@ -2212,9 +2306,9 @@ __device__ __forceinline__ bool flux4_body(const DevMesh& m, const DevState<R>& 
         const R A12 = q == 1 ? c1 : b1, A22 = q == 1 ? c2 : a2, A32 = q == 1 ? c3 : b3;
         const R A13 = q >= 2 ? c1 : b2, A23 = q >= 2 ? c2 : b3, A33 = q >= 2 ? c3 : a3;
 #if HP_LSQ_TABLE
-        const R rdnr = mrcp_tab<F>(dnr, LB(15), bad);
+        const R rdnr = LB(15);
 #undef LB
-        const R dq = mdiv<F>(det3(A11, A21, A31, A12, A22, A32, A13, A23, A33), dnr, rdnr, bad);
+        const R dq = star_quo<F>(det3(A11, A21, A31, A12, A22, A32, A13, A23, A33), dnr, rdnr, bad);
 #else
         const R dq = det3(A11, A21, A31, A12, A22, A32, A13, A23, A33) / dnr;
 #endif
@@ -3029,8 +3123,31 @@ __global__ void __launch_bounds__(128) k_qrs_flux(DevMesh m, DevState<R> s, DevP
     }
 }
 
+// Set-up: unit normals and areas of the cells' faces (m.nrm), by the
+// expressions that the flux kernel would otherwise evaluate per face and
+// stage, compiled with the same flags.
+__global__ void __launch_bounds__(128) k_face_normals(DevMesh m) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= m.neles) return;
+    double* out = const_cast<double*>(m.nrm);
+#pragma unroll
+    for (int f = 0; f < 4; f++) {
+        const double scx = ldg(COL(m.sc, 3 * f) + i), scy = ldg(COL(m.sc, 3 * f + 1) + i),
+                     scz = ldg(COL(m.sc, 3 * f + 2) + i);
+        const double area = sqrt(scx * scx + scy * scy + scz * scz);
+        COL(out, 4 * f)[i] = scx / area;
+        COL(out, 4 * f + 1)[i] = scy / area;
+        COL(out, 4 * f + 2)[i] = scz / area;
+        COL(out, 4 * f + 3)[i] = area;
+    }
+}
+
 static inline unsigned grid_for(long long n, int block) {
     return (unsigned)((n + block - 1) / block);
+}
+
+static void setup(const DevMesh& m, cudaStream_t st) {
+    if (m.nrm) k_face_normals<<<grid_for(m.neles, 128), 128, 0, st>>>(m);
 }
 
 #define MARK(k) do { if (hook && hook->mark) hook->mark(hook->ctx, (k)); } while (0)

@@ -34,7 +34,7 @@
 #include "hp_kernels.cuh"
 
 namespace hp {
-const Variant variant_fp64 = {"fp64", sizeof(double), &v_fp64::enqueue_start, &v_fp64::enqueue_step, (HP_FACE_VISC && sizeof(HP_R) != sizeof(double)) ? 1 : 0,
+const Variant variant_fp64 = {"fp64", sizeof(double), &v_fp64::enqueue_start, &v_fp64::enqueue_step, (HP_FACE_VISC && sizeof(HP_R) != sizeof(double)) ? 1 : 0, &v_fp64::setup,
     &v_fp64::fused_grid, &v_fp64::enqueue_fused};
 
 // The FP64 (FMA) kernels over the wall-layer cell lists, for the steps of the
@@ -73,5 +73,5 @@ static void wall_flux(const DevMesh& m, const DevState<double>& s, const DevPara
     else wall_flux_z<0>(m, s, P, st, stage);
 }
 }  // namespace v_fp64
-const WallFp64 wall_fp64 = {&v_fp64::wall_visc, &v_fp64::wall_grad, &v_fp64::wall_flux};
+const WallFp64 wall_fp64 = {&v_fp64::setup, &v_fp64::wall_visc, &v_fp64::wall_grad, &v_fp64::wall_flux};
 }
