@@ -763,17 +763,22 @@ __global__ void k_phi_copy_serial(DevMesh m, DevState<R> s) {
 // ---------------------------------------------------------------------------
 // JST dissipation, src/sr_smooth.F90:52-154: switches anu and Laplacian d2q.
 //
-// The standalone k_smooth1 (HP_JST_SETS) runs two threads per cell: the
-// first half of a block takes variables 1-5 and the gas-pressure switch of
-// its cells, the second half variables 6-10 and the liquid-pressure switch,
-// so each warp still reads one column for 32 consecutive cells and every
-// thread has half the neighbour gathers in flight.  The values are those of
-// the one-thread form (the fused step's).  (The same split of k_smooth2
-// measured 16% slower: each thread repeats its volume gathers and
-// divisions.)
-#ifndef HP_JST_SETS
-#define HP_JST_SETS 1
+// k_smooth1 and k_smooth2 run two threads per cell: the first JST_CELLS
+// threads of a block take variables 1-5 and the gas-pressure switch of its
+// cells, the others variables 6-10 and the liquid-pressure switch, so a warp
+// reads one column for 32 consecutive cells.  Both wait on gathers, so what
+// counts is the loads in flight: all of a thread's stand before its
+// arithmetic, and the register caps (HP_JST1_MINB, HP_JST2_MINB blocks of 128
+// threads per SM) are as wide as that needs (k_smooth2 with 4 or 5 blocks:
+// 128 or 174 us).  983,040 cells, FP64: k_smooth1 75 -> 63 us, k_smooth2
+// 154 -> 115 us (between events); 2,058 cells: k_smooth2 14 -> 8 us.
+#ifndef HP_JST1_MINB
+#define HP_JST1_MINB 8
 #endif
+#ifndef HP_JST2_MINB
+#define HP_JST2_MINB 3
+#endif
+enum { JST_CELLS = 64 };
 // set 0: variables 1-5, anu(:,1); set 1: variables 6-10, anu(:,2)
 __device__ __forceinline__ void smooth1_set(const DevMesh& m, const DevState<R>& s, int i, int set) {
     const int a = ldg(COL(m.snb, 0) + i), b = ldg(COL(m.snb, 1) + i);
@@ -808,118 +813,101 @@ __device__ __forceinline__ void smooth1_set(const DevMesh& m, const DevState<R>&
     for (int k = 0; k < 5; k++) COL(s.d2q, 5 * set + k)[i] = lap[k];
     COL(s.anu, set)[i] = anu;
 }
+// the fused step's form: one thread per cell
 __device__ __forceinline__ void k_smooth1_body(DevMesh m, DevState<R> s, int bid) {
-    int i = bid * blockDim.x + threadIdx.x;
+    const int i = bid * blockDim.x + threadIdx.x;
     if (i >= m.neles) return;
-    const int a = ldg(COL(m.snb, 0) + i), b = ldg(COL(m.snb, 1) + i);
-    const int c = ldg(COL(m.snb, 2) + i), d = ldg(COL(m.snb, 3) + i);
-    const double* pg = COL(s.pr, P_PG);
-    const double* pp = COL(s.pr, P_PP);
-    const S e6 = (S)(double)1.0e-6f;
-    // the switch sums of variables 1, 5, 6, 10 (sw[0..3]) and the Laplacian
-    // d2q of every variable, one variable at a time
-    S swn[4], swd[4], lap[10];
-#pragma unroll
-    for (int k = 0; k < 10; k++) {
-        const double* col = COL(s.cn, k);
-        const S v0 = (S)col[i], v1 = (S)col[a], v2 = (S)col[b], v3 = (S)col[c], v4 = (S)col[d];
-        const int slot = k == 0 ? 0 : k == 4 ? 1 : k == 5 ? 2 : k == 9 ? 3 : -1;
-        if (slot >= 0) {
-            swn[slot] = fabs(v1 - v0) + fabs(v2 - v0) + fabs(v3 - v0) + fabs(v4 - v0);
-            swd[slot] = fabs(v1 + v0) + fabs(v2 + v0) + fabs(v3 + v0) + fabs(v4 + v0);
-        }
-        lap[k] = v1 - v0 + v2 - v0 + v3 - v0 + v4 - v0;
-    }
-    const S pgi = (S)pg[i], pga = (S)pg[a], pgb = (S)pg[b], pgc = (S)pg[c], pgd = (S)pg[d];
-    S anun = fabs(pga - pgi) + fabs(pgb - pgi) + fabs(pgc - pgi) + fabs(pgd - pgi);
-    S anud = fabs(pga + pgi) + fabs(pgb + pgi) + fabs(pgc + pgi) + fabs(pgd + pgi);
-    S anupg = anun / anud;
-    S anu1 = anupg + swn[1] / (swd[1] + e6);
-    anu1 = anu1 + swn[0] / (swd[0] + e6);
-    const S ppi = (S)pp[i], ppa = (S)pp[a], ppb = (S)pp[b], ppc = (S)pp[c], ppd = (S)pp[d];
-    anun = fabs(ppa - ppi) + fabs(ppb - ppi) + fabs(ppc - ppi) + fabs(ppd - ppi);
-    anud = fabs(ppa + ppi) + fabs(ppb + ppi) + fabs(ppc + ppi) + fabs(ppd + ppi);
-    S anupp = anun / anud;
-    S anu2 = anupp + swn[2] / (swd[2] + e6);
-    anu2 = anu2 + swn[3] / (swd[3] + e6);
-    // all stores after all loads (the output columns may alias the inputs
-    // as far as the compiler can tell)
-#pragma unroll
-    for (int k = 0; k < 10; k++) COL(s.d2q, k)[i] = lap[k];
-    COL(s.anu, 0)[i] = anu1;
-    COL(s.anu, 1)[i] = anu2;
+    smooth1_set(m, s, i, 0);
+    smooth1_set(m, s, i, 1);
 }
 // Block 0 also forms the step's dt, which no smoothing switch reads and every
 // later kernel of the step does.
-__global__ void __launch_bounds__(512) k_smooth1(DevMesh m, DevState<R> s, DevParams P) {
+__global__ void __launch_bounds__(2 * JST_CELLS, HP_JST1_MINB) k_smooth1(DevMesh m, DevState<R> s, DevParams P) {
     if (blockIdx.x == 0) step_begin_block(s.s, P, m.ncase, m.nhalo > 0);
-#if HP_JST_SETS
-    const int half = (int)blockDim.x >> 1, set = (int)threadIdx.x >= half;
-    const int i = blockIdx.x * half + ((int)threadIdx.x - set * half);
+    const int set = (int)threadIdx.x >= JST_CELLS;
+    const int i = blockIdx.x * JST_CELLS + ((int)threadIdx.x - set * JST_CELLS);
     if (i < m.neles) smooth1_set(m, s, i, set);
-#else
-    k_smooth1_body(m, s, blockIdx.x);
-#endif
 }
 
-// src/sr_smooth.F90:200-374: blended 2nd/4th difference d24.  F selects the
-// division form (see mdiv); returns the fast form's out-of-range flag.
+// src/sr_smooth.F90:200-374: blended 2nd/4th difference d24 of the variables
+// of one set (1-5 or 6-10).  F selects the division form (see mdiv); returns
+// the fast form's out-of-range flag.  Every load of the set stands before the
+// arithmetic: the kernel's time is the latency of its gathers, and with one
+// variable loaded at a time a cell waited for ten of them in a row.
 template <int F>
-__device__ __forceinline__ unsigned smooth2_body(const DevMesh& m, const DevState<R>& s, const DevParams& P, int i) {
+__device__ __forceinline__ unsigned smooth2_set(const DevMesh& m, const DevState<R>& s, const DevParams& P, int i,
+                                                int set) {
     unsigned bad = 0;
-    const S dt = (S)s.s[case_of(m, i)].dt;
-    const S rdt = mrcp<F>(dt, bad);
     int nb[4];
 #pragma unroll
     for (int f = 0; f < 4; f++) nb[f] = ldg(COL(m.snb, f) + i);
-    const S vi = mdiv<F>((S)ldg(m.vol + i), dt, rdt, bad);
-    S d24nc[4], out[10];
+    const S dt = (S)s.s[case_of(m, i)].dt;
+    const double* anu = COL(s.anu, set);
+    const S ai = (S)anu[i], voli = (S)ldg(m.vol + i);
+    S an[4], vn[4], c[5][5], q[5][5];
 #pragma unroll
-    for (int f = 0; f < 4; f++) d24nc[f] = S(0.5) * (vi + mdiv<F>((S)ldg(m.vol + nb[f]), dt, rdt, bad));
+    for (int f = 0; f < 4; f++) {
+        an[f] = (S)anu[nb[f]];
+        vn[f] = (S)ldg(m.vol + nb[f]);
+    }
 #pragma unroll
-    for (int set = 0; set < 2; set++) {
-        const double* anu = COL(s.anu, set);
-        S ai = (S)anu[i];
-        S d2c[4], d4c[4];
+    for (int k = 0; k < 5; k++) {
+        const double* cn = COL(s.cn, 5 * set + k);
+        const double* dq = COL(s.d2q, 5 * set + k);
+        c[k][4] = (S)cn[i];
+        q[k][4] = (S)dq[i];
 #pragma unroll
         for (int f = 0; f < 4; f++) {
-            S e2 = (S)P.co2 * mx2(ai, (S)anu[nb[f]]);
-            S e4 = mx2(S(0.0), (S)P.co4 - e2);
-            d2c[f] = e2 * d24nc[f];
-            d4c[f] = e4 * d24nc[f];
-        }
-#pragma unroll
-        for (int k = 5 * set; k < 5 * set + 5; k++) {
-            const double* cn = COL(s.cn, k);
-            const double* dq = COL(s.d2q, k);
-            S ci = (S)cn[i], qi = (S)dq[i];
-            S d2 = d2c[0] * ((S)cn[nb[0]] - ci) + d2c[1] * ((S)cn[nb[1]] - ci) +
-                   d2c[2] * ((S)cn[nb[2]] - ci) + d2c[3] * ((S)cn[nb[3]] - ci);
-            S d4 = d4c[0] * ((S)dq[nb[0]] - qi) + d4c[1] * ((S)dq[nb[1]] - qi) +
-                   d4c[2] * ((S)dq[nb[2]] - qi) + d4c[3] * ((S)dq[nb[3]] - qi);
-            out[k] = d2 - d4;
+            c[k][f] = (S)cn[nb[f]];
+            q[k][f] = (S)dq[nb[f]];
         }
     }
-    // all stores after all loads (see k_smooth1)
+    const S rdt = mrcpp<F>(dt, bad);
+    mpos<F>(voli, bad);
+    const S vi = mquo<F>(voli, dt, rdt);
+    S d2c[4], d4c[4];
 #pragma unroll
-    for (int k = 0; k < 10; k++) COL(s.d24, k)[i] = out[k];
+    for (int f = 0; f < 4; f++) {
+        mpos<F>(vn[f], bad);
+        const S d24nc = S(0.5) * (vi + mquo<F>(vn[f], dt, rdt));
+        const S e2 = (S)P.co2 * mx2(ai, an[f]);
+        const S e4 = mx2(S(0.0), (S)P.co4 - e2);
+        d2c[f] = e2 * d24nc;
+        d4c[f] = e4 * d24nc;
+    }
+#pragma unroll
+    for (int k = 0; k < 5; k++) {
+        const S ci = c[k][4], qi = q[k][4];
+        const S d2 = d2c[0] * (c[k][0] - ci) + d2c[1] * (c[k][1] - ci) + d2c[2] * (c[k][2] - ci) +
+                     d2c[3] * (c[k][3] - ci);
+        const S d4 = d4c[0] * (q[k][0] - qi) + d4c[1] * (q[k][1] - qi) + d4c[2] * (q[k][2] - qi) +
+                     d4c[3] * (q[k][3] - qi);
+        COL(s.d24, 5 * set + k)[i] = d2 - d4;
+    }
     return bad;
 }
 
-__device__ __forceinline__ void k_smooth2_body(DevMesh m, DevState<R> s, DevParams P, int bid) {
-    int i = bid * blockDim.x + threadIdx.x;
-    const bool valid = i < m.neles;
-    if (!valid) i = m.neles - 1;      // keep the warp whole for the vote below
+// one set of cell i (a lane with valid = false only votes)
+__device__ __forceinline__ void smooth2_cell(const DevMesh& m, const DevState<R>& s, const DevParams& P, int i,
+                                             int set, bool valid) {
     if constexpr (HP_FAST(8)) {
         unsigned bad = 0;
-        if (valid) bad = smooth2_body<1>(m, s, P, i);
-        if (__any_sync(0xffffffffu, bad) && valid) smooth2_body<0>(m, s, P, i);
+        if (valid) bad = smooth2_set<1>(m, s, P, i, set);
+        if (__any_sync(0xffffffffu, bad) && valid) smooth2_set<0>(m, s, P, i, set);
     } else {
-        if (valid) smooth2_body<0>(m, s, P, i);
+        if (valid) smooth2_set<0>(m, s, P, i, set);
     }
 }
-__global__ void __launch_bounds__(512) k_smooth2(DevMesh m, DevState<R> s, DevParams P) {
-    k_smooth2_body(m, s, P, blockIdx.x);
+// the fused step's form: one thread per cell
+__device__ __forceinline__ void k_smooth2_body(DevMesh m, DevState<R> s, DevParams P, int bid) {
+    const int i = bid * blockDim.x + threadIdx.x;
+    smooth2_cell(m, s, P, i, 0, i < m.neles);
+    smooth2_cell(m, s, P, i, 1, i < m.neles);
+}
+__global__ void __launch_bounds__(2 * JST_CELLS, HP_JST2_MINB) k_smooth2(DevMesh m, DevState<R> s, DevParams P) {
+    const int set = (int)threadIdx.x >= JST_CELLS;
+    const int i = blockIdx.x * JST_CELLS + ((int)threadIdx.x - set * JST_CELLS);
+    smooth2_cell(m, s, P, i, set, i < m.neles);
 }
 
 // Cells whose gradients and limiter are evaluated: active cells and the
@@ -3182,11 +3170,21 @@ static void enqueue_flux(const DevMesh& m, const DevState<R>& s, const DevParams
     }
 }
 
+// Threads per block of the one-thread-per-cell kernels where the caller leaves
+// the choice (block_size 0): 256, or fewer where that would leave SMs without
+// a block (148 of them).  These kernels wait on gathers, and the warps of one
+// SM queue for its load unit: a 2,058-cell step takes 86 us with 9 blocks of
+// 256 threads in the primitive passes and 82 us with 33 of 64.
+static int cell_block(const DevMesh& m, int block) {
+    if (block > 0) return block;
+    return m.neles >= 148 * 256 ? 256 : m.neles >= 148 * 128 ? 128 : 64;
+}
+
 static void enqueue_start(const DevMesh& m, const void* stp, const DevParams& P, cudaStream_t st,
                           int block, const StepHook* hook) {
     const DevState<R>& s = *static_cast<const DevState<R>*>(stp);
     MARK(KK_PRIM_START);
-    const int cb = block > 0 ? block : 256;
+    const int cb = cell_block(m, block);
     k_prim<PM_START><<<grid_for(m.neles, cb), cb, 0, st>>>(m, s, P);
     MARK(KK_COUNT);
 }
@@ -3198,18 +3196,18 @@ static void enqueue_step(const DevMesh& m, const void* stp, const DevParams& P, 
     // one-thread-per-cell kernels: `block` threads per block (64..512,
     // 0 = 256); four-lane kernels and the one-thread kernels of aliased
     // meshes: 128 (their launch bounds)
-    const int cb = block > 0 ? block : 256, b = 128;
+    const int cb = cell_block(m, block), b = 128;
     const unsigned ge = grid_for(m.neles, cb), gf = grid_for(m.neles, b);
     const unsigned gg = grid_for(m.nghosts > 0 ? m.nghosts : 1, cb);
     EXCHANGE(HP_X_DT);
     // dt and time of every case (in k_smooth1), and JST dissipation, src/sr_smooth.F90 (once per step)
     if (m.aliased) { MARK(KK_SERIAL); k_smooth_copy_serial<<<1, 1, 0, st>>>(m, s, 0); }
     MARK(KK_SMOOTH1);
-    const unsigned gj = HP_JST_SETS ? grid_for(2ll * m.neles, cb) : ge;   // two threads per cell
-    k_smooth1<<<gj, cb, 0, st>>>(m, s, P);
+    const unsigned gj = grid_for(m.neles, JST_CELLS);
+    k_smooth1<<<gj, 2 * JST_CELLS, 0, st>>>(m, s, P);
     if (m.aliased) { MARK(KK_SERIAL); k_smooth_copy_serial<<<1, 1, 0, st>>>(m, s, 1); }
     MARK(KK_SMOOTH2);
-    k_smooth2<<<ge, cb, 0, st>>>(m, s, P);
+    k_smooth2<<<gj, 2 * JST_CELLS, 0, st>>>(m, s, P);
     if (P.five_phase) {   // src/main.F90:570-572
         MARK(KK_QRS);
         k_qrs_diss1<<<grid_for(m.neles, 256), 256, 0, st>>>(m, s);
