@@ -95,6 +95,16 @@ struct DevMesh {
     long long fld;          // leading dimension of the face-flux columns
     const int* f_i;
     const int* f_code;      // local face of the owner (bits 0-1)
+    // what the face kernels read of a face, in face order: the cell on its
+    // other side, the owner's area vector and the face centroid minus the
+    // centroids of owner and neighbour in the arithmetic of the fluxes, and
+    // the viscous face centroid; filled on the device from the cell columns
+    const int* f_j;
+    const float* fgeo;      // [9][fld] area vector, offset from owner, from neighbour
+    const double* fgcv;     // [3][fld]
+    // centroid differences and face centroid offsets in float for the FP32
+    // gradients (FP32-arithmetic variants, no aliased ghosts; else null)
+    const float *dxnf, *fxof;   // [12][ld] as dxn, fxo
     const int* cface;       // [4][ld]
     // face modes 2 (colouring) and 3 (atomics): the face fluxes are added
     // to a per-cell accumulator instead of stored as records.  Mode 2 takes

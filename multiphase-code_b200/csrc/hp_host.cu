@@ -227,6 +227,11 @@ static void plan_arena(hp_handle* h, Arena& a, int neles, int nghosts, long long
         m.wclass = nullptr;
         s.gr64 = nullptr;
     }
+    m.dxnf = m.fxof = nullptr;
+    if (gb != D && !h->aliased) {
+        m.dxnf = (const float*)a.take(12 * (size_t)ld * sizeof(float));
+        m.fxof = (const float*)a.take(12 * (size_t)ld * sizeof(float));
+    }
     m.nface = nface;
     m.fld = ((long long)nface + 63) / 64 * 64;
     s.racc = nullptr;
@@ -235,13 +240,18 @@ static void plan_arena(hp_handle* h, Arena& a, int neles, int nghosts, long long
         m.f_i = (const int*)a.take((size_t)nface * I);
         m.f_code = (const int*)a.take((size_t)nface * I);
         m.cface = (const int*)a.take(4 * (size_t)ld * I);
+        m.f_j = (const int*)a.take((size_t)nface * I);
+        m.fgeo = (const float*)a.take(9 * (size_t)m.fld * sizeof(float));
+        m.fgcv = (const double*)a.take(3 * (size_t)m.fld * D);
         s.ff = (double*)a.take((size_t)FACE_REC * (size_t)m.fld * gb);
         if (h->prm.face_mode >= 2) {   // colouring or atomics: per-cell face sums
             s.racc = (double*)a.take(10 * (size_t)ld * D);
             m.fcolor = (const int*)a.take((size_t)nface * I);
         }
     } else {
-        m.f_i = m.f_code = m.cface = nullptr;
+        m.f_i = m.f_code = m.cface = m.f_j = nullptr;
+        m.fgeo = nullptr;
+        m.fgcv = nullptr;
         s.ff = nullptr;
     }
     h->d_sync = (GridSync*)a.take(sizeof(GridSync));
@@ -667,6 +677,27 @@ __global__ void __launch_bounds__(128) k_offsets(DevMesh m) {
         if (!(b >= 0x1p-100 && b < 0x1p101)) out |= FK_LSQB_RANGE;
     }
     if (out) const_cast<unsigned*>(m.fk)[i] |= out;
+    if (m.dxnf)
+        for (int k = 0; k < 12; k++) {
+            const_cast<float*>(m.dxnf)[k * ld + i] = (float)dxn[k * ld + i];
+            const_cast<float*>(m.fxof)[k * ld + i] = (float)fxo[k * ld + i];
+        }
+}
+
+// Set-up, one thread per face: the face-ordered tables (after k_offsets).
+__global__ void __launch_bounds__(128) k_face_tables(DevMesh m) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= m.nface) return;
+    const long long ld = m.ld, fl = m.fld;
+    const int i = m.f_i[t], f = m.f_code[t] & 3;
+    float* g = const_cast<float*>(m.fgeo);
+    const_cast<int*>(m.f_j)[t] = m.nc[f * ld + i];
+    for (int d = 0; d < 3; d++) {
+        g[d * fl + t] = (float)m.sc[(3 * f + d) * ld + i];
+        g[(3 + d) * fl + t] = (float)m.fxo[(4 * d + f) * ld + i];
+        g[(6 + d) * fl + t] = (float)m.fxn[(4 * d + f) * ld + i];
+        const_cast<double*>(m.fgcv)[d * fl + t] = m.fcv[(4 * d + f) * ld + i];
+    }
 }
 }  // namespace
 
@@ -927,12 +958,6 @@ extern "C" int hp_create_batch(const hp_mesh* meshes, int32_t ncase, const hp_pa
     if (e == cudaSuccess) e = up(m.lsqb, L.lb.data(), NLSQ * ld * D);
     if (e == cudaSuccess) e = up(m.fk, L.fk.data(), ld * sizeof(unsigned));
     if (e == cudaSuccess) e = up(m.fxn, L.fch.data(), 12 * ld * D);
-    if (e == cudaSuccess) {
-        k_offsets<<<blocks_for(neles, 128), 128, 0, st>>>(m);
-        if (gb == D) h->var->setup(m, st);
-        else wall_fp64.setup(m, st);
-        e = cudaGetLastError();
-    }
     if (e == cudaSuccess && nghosts) e = up(m.g_par, L.gpar.data(), nghosts * (size_t)I);
     if (e == cudaSuccess && nghosts) e = up(m.g_id, L.gid.data(), nghosts * (size_t)I);
     if (e == cudaSuccess && nghosts) e = up(m.g_type, L.gtyp.data(), nghosts * (size_t)I);
@@ -941,6 +966,13 @@ extern "C" int hp_create_batch(const hp_mesh* meshes, int32_t ncase, const hp_pa
     if (e == cudaSuccess && nface) e = up(m.f_i, hf_i.data(), nface * (size_t)I);
     if (e == cudaSuccess && nface) e = up(m.f_code, hf_code.data(), nface * (size_t)I);
     if (e == cudaSuccess && nface) e = up(m.cface, hcface.data(), 4 * (size_t)ld * I);
+    if (e == cudaSuccess) {
+        k_offsets<<<blocks_for(neles, 128), 128, 0, st>>>(m);
+        if (nface) k_face_tables<<<blocks_for(nface, 128), 128, 0, st>>>(m);
+        if (gb == D) h->var->setup(m, st);
+        else wall_fp64.setup(m, st);
+        e = cudaGetLastError();
+    }
     m.face_mode = nface > 0 ? h->prm.face_mode : 0;
     m.ncolor = ncolor;
     for (int c = 0; c <= ncolor; c++) m.fcoff[c] = fcoff[c];

@@ -942,19 +942,18 @@ __device__ __forceinline__ void k_grad_body(DevMesh m, DevState<R> s, DevParams 
     int n[4];
 #pragma unroll
     for (int f = 0; f < 4; f++) n[f] = ldg(COL(m.nc, f) + i);
-    const double x0 = ldg(m.xc + i), y0 = ldg(m.yc + i), z0 = ldg(m.zc + i);
+    // centroid differences from the set-up tables (the same subtractions)
     R xa[4], ya[4], za[4];
 #pragma unroll
     for (int f = 0; f < 4; f++) {
-        if (FPR && HP_DXN_TABLE) {
-            // the centroid differences, formed at set-up (the same subtraction)
+        if constexpr (FPR) {
+            xa[f] = (R)ldg(COL(m.dxnf, 3 * f) + i);
+            ya[f] = (R)ldg(COL(m.dxnf, 3 * f + 1) + i);
+            za[f] = (R)ldg(COL(m.dxnf, 3 * f + 2) + i);
+        } else {
             xa[f] = (R)ldg(COL(m.dxn, 3 * f) + i);
             ya[f] = (R)ldg(COL(m.dxn, 3 * f + 1) + i);
             za[f] = (R)ldg(COL(m.dxn, 3 * f + 2) + i);
-        } else {
-            xa[f] = (R)(ldg(m.xc + n[f]) - x0);
-            ya[f] = (R)(ldg(m.yc + n[f]) - y0);
-            za[f] = (R)(ldg(m.zc + n[f]) - z0);
         }
     }
     // geometry-only terms (wt, a1..b3, dnr of src/sr_derivative.F90:163-176,
@@ -1023,9 +1022,15 @@ __device__ __forceinline__ void k_grad_body(DevMesh m, DevState<R> s, DevParams 
     R fx[4], fy[4], fz[4];
 #pragma unroll
     for (int f = 0; f < 4; f++) {
-        fx[f] = (R)ldg(COL(m.fxo, f) + i);
-        fy[f] = (R)ldg(COL(m.fxo, 4 + f) + i);
-        fz[f] = (R)ldg(COL(m.fxo, 8 + f) + i);
+        if constexpr (FPR) {
+            fx[f] = (R)ldg(COL(m.fxof, f) + i);
+            fy[f] = (R)ldg(COL(m.fxof, 4 + f) + i);
+            fz[f] = (R)ldg(COL(m.fxof, 8 + f) + i);
+        } else {
+            fx[f] = (R)ldg(COL(m.fxo, f) + i);
+            fy[f] = (R)ldg(COL(m.fxo, 4 + f) + i);
+            fz[f] = (R)ldg(COL(m.fxo, 8 + f) + i);
+        }
     }
     const int lv[4] = {8, 9, 11, 12};   // pg, pp, rog, rop rows of gv
     R phi = R(0);
@@ -1225,14 +1230,17 @@ enum { LIM_LD = 128, LIMC_N = 13, LIMC_LD = 32 };
 // Z selects the face flux: 0 HLLC-Batten (src/sr_hllcbatten.F90:338-529),
 // 1 HLLC-Zien (src/sr_hllczien.F90:348-487), 2 the Jameson central flux
 // (src/sr_jameson.F90:126-262).
-template <int F, int Z, class PT, bool NC = true>
+// LIST: the face is face t of the face list and its geometry comes from the
+// face-ordered FP32 tables: consecutive threads read consecutive words, where
+// the cell columns of four different f's gave a warp a quarter of each sector.
+template <int F, int Z, class PT, bool NC = true, bool LIST = false>
 __device__ __forceinline__ void face_eval(const DevMesh& m, const DevState<R>& s, const DevParams& P,
-                                          int i, int f, FaceOut& o, unsigned& bad, const PT* pr) {
-    const int neigh = ldg(COL(m.nc, f) + i);
+                                          int i, int f, FaceOut& o, unsigned& bad, const PT* pr, int t = 0) {
+#define FGEO(k) (R)ldg(m.fgeo + (size_t)(k) * m.fld + t)
+    const int neigh = LIST ? ldg(m.f_j + t) : ldg(COL(m.nc, f) + i);
     const unsigned kind = (ldg(m.fk + i) >> (4 * f)) & 0xFu;
-    // FP64: unit normal and area from the set-up table (the square root and
-    // the three divisions were 7% of the FP64 flux kernel's instructions);
-    // FP32: formed here, where its approximate divisions cost little
+    // FP64: unit normal and area from the set-up table; FP32: formed here,
+    // where its approximate divisions cost little
     R area, enx, eny, enz;
     if constexpr (sizeof(R) == 8) {
         enx = ldg(COL(m.nrm, 4 * f) + i);
@@ -1240,8 +1248,8 @@ __device__ __forceinline__ void face_eval(const DevMesh& m, const DevState<R>& s
         enz = ldg(COL(m.nrm, 4 * f + 2) + i);
         area = ldg(COL(m.nrm, 4 * f + 3) + i);
     } else {
-        const R scx = (R)ldg(COL(m.sc, 3 * f) + i), scy = (R)ldg(COL(m.sc, 3 * f + 1) + i),
-                scz = (R)ldg(COL(m.sc, 3 * f + 2) + i);
+        const R scx = LIST ? FGEO(0) : (R)ldg(COL(m.sc, 3 * f) + i), scy = LIST ? FGEO(1) : (R)ldg(COL(m.sc, 3 * f + 1) + i),
+                scz = LIST ? FGEO(2) : (R)ldg(COL(m.sc, 3 * f + 2) + i);
         area = sqrt(scx * scx + scy * scy + scz * scz);
         const R rarea = mrcp<F>(area, bad);
         enx = mdiv<F>(scx, area, rarea, bad);
@@ -1339,10 +1347,11 @@ __device__ __forceinline__ void face_eval(const DevMesh& m, const DevState<R>& s
         const R phimin = (R)mn2(PLD(s.phi + i), PLD(s.phi + neigh));
         // face centroid minus each side's centroid (set-up tables: the
         // neighbour's centroid would be three more gathers)
-        const R xf0 = (R)ldg(COL(m.fxo, f) + i), yf0 = (R)ldg(COL(m.fxo, 4 + f) + i),
-                zf0 = (R)ldg(COL(m.fxo, 8 + f) + i);
-        const R xfn = (R)ldg(COL(m.fxn, f) + i), yfn = (R)ldg(COL(m.fxn, 4 + f) + i),
-                zfn = (R)ldg(COL(m.fxn, 8 + f) + i);
+        const R xf0 = LIST ? FGEO(3) : (R)ldg(COL(m.fxo, f) + i), yf0 = LIST ? FGEO(4) : (R)ldg(COL(m.fxo, 4 + f) + i),
+                zf0 = LIST ? FGEO(5) : (R)ldg(COL(m.fxo, 8 + f) + i);
+        const R xfn = LIST ? FGEO(6) : (R)ldg(COL(m.fxn, f) + i), yfn = LIST ? FGEO(7) : (R)ldg(COL(m.fxn, 4 + f) + i),
+                zfn = LIST ? FGEO(8) : (R)ldg(COL(m.fxn, 8 + f) + i);
+#undef FGEO
         const R* g = s.gr;
 #define REC(v, X, Y, Z, G, c) \
     v = v + phimin * (X * PLD(COL(g, G) + c) + Y * PLD(COL(g, G + 1) + c) + Z * PLD(COL(g, G + 2) + c))
@@ -2430,7 +2439,7 @@ __device__ __forceinline__ void k_faceflux_body(DevMesh m, DevState<R> s, DevPar
     if (wall_face(m, i, f)) return;
     FaceOut o{};
     unsigned bad = 0;
-    face_eval<0, Z, R, NC>(m, s, P, i, f, o, bad, s.prr);
+    face_eval<0, Z, R, NC, true>(m, s, P, i, f, o, bad, s.prr, t);
     R rec[FACE_REC];
     if (o.wall) {
 #pragma unroll
@@ -2465,7 +2474,7 @@ __device__ __forceinline__ void k_facescatter_body(DevMesh m, DevState<R> s, Dev
     const int j = ldg(COL(m.nc, f) + i);
     FaceOut o{};
     unsigned bad = 0;
-    face_eval<0, Z>(m, s, P, i, f, o, bad, s.prr);
+    face_eval<0, Z, R, true, true>(m, s, P, i, f, o, bad, s.prr, fid);
     double e[10];
     if (o.wall) {
 #pragma unroll
@@ -2499,18 +2508,14 @@ __global__ void __launch_bounds__(128, HP_FLUX4_MINB) k_facescatter(DevMesh m, D
 // Face-centred viscous fluxes, src/sr_viscousgp.F90:488-1138 (AMUP constant).
 // One face f of cell i: face-centred LSQ over 5 (boundary) or 8 (interior)
 // cell centres, Newtonian stresses and heat flux; c[8] = the face's
-// contribution to visug..vistp.
+// contribution to visug..vistp.  neigh, sc, xf..zf: the cell on the face's
+// other side, its area vector and its centroid.
 template <int F, class PT>
 __device__ __forceinline__ void visc_face(const DevMesh& m, const DevState<R>& s, const DevParams& P,
-                                          int i, int f, const int nci[4], double c[8], unsigned& bad,
-                                          const PT* pr) {
+                                          int i, const int nci[4], int neigh, R scx, R scy, R scz, double xf,
+                                          double yf, double zf, double c[8], unsigned& bad, const PT* pr) {
     const int fcol[8] = {P_UG, P_VG, P_WG, P_TG, P_UP, P_VP, P_WP, P_TP};
     const R c23 = (R)P.c23;
-    const R scx = (R)ldg(COL(m.sc, 3 * f) + i), scy = (R)ldg(COL(m.sc, 3 * f + 1) + i),
-            scz = (R)ldg(COL(m.sc, 3 * f + 2) + i);
-    const double xf = ldg(COL(m.fcv, f) + i), yf = ldg(COL(m.fcv, 4 + f) + i),
-                 zf = ldg(COL(m.fcv, 8 + f) + i);
-    const int neigh = nci[f];
     R ff[8];
 #pragma unroll
     for (int v = 0; v < 8; v++) ff[v] = (R)((COL(pr, fcol[v])[i] + COL(pr, fcol[v])[neigh]) * 0.5);
@@ -2672,6 +2677,11 @@ __device__ __forceinline__ void visc_face_ph(const DevMesh& m, const DevState<R>
     c[3] = (double)(phif * (qxx * scx + qyy * scy + qzz * scz));
 }
 
+// area vector and centroid of face f of cell i from the cell columns
+#define VISC_GEO(i, f) \
+    (R)ldg(COL(m.sc, 3 * (f)) + (i)), (R)ldg(COL(m.sc, 3 * (f) + 1) + (i)), (R)ldg(COL(m.sc, 3 * (f) + 2) + (i)), \
+    ldg(COL(m.fcv, (f)) + (i)), ldg(COL(m.fcv, 4 + (f)) + (i)), ldg(COL(m.fcv, 8 + (f)) + (i))
+
 // one thread per cell (aliased meshes)
 __global__ void __launch_bounds__(128) k_visc(DevMesh m, DevState<R> s, DevParams P) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -2687,7 +2697,7 @@ __global__ void __launch_bounds__(128) k_visc(DevMesh m, DevState<R> s, DevParam
     for (int f = 0; f < 4; f++) {
         double c[8];
         unsigned bad_ = 0;
-        visc_face<0>(m, s, P, i, f, nci, c, bad_, s.pr);
+        visc_face<0>(m, s, P, i, nci, nci[f], VISC_GEO(i, f), c, bad_, s.pr);
 #pragma unroll
         for (int k = 0; k < 8; k++) acc[k] = acc[k] + c[k];
     }
@@ -2717,8 +2727,8 @@ __device__ __forceinline__ void k_visc4_body(DevMesh m, DevState<R> s, DevParams
     for (int pass = HP_FAST(4) ? 1 : 0; pass >= 0; pass--) {
         double c[8];
         unsigned bad = 0;
-        if (pass) visc_face<1>(m, s, P, i, q, nci, c, bad, s.prr);
-        else visc_face<0>(m, s, P, i, q, nci, c, bad, s.prr);
+        if (pass) visc_face<1>(m, s, P, i, nci, nci[q], VISC_GEO(i, q), c, bad, s.prr);
+        else visc_face<0>(m, s, P, i, nci, nci[q], VISC_GEO(i, q), c, bad, s.prr);
         double acc[8];
 #pragma unroll
         for (int k = 0; k < 8; k++) acc[k] = 0.0;
@@ -2794,7 +2804,10 @@ __device__ __forceinline__ void k_facevisc_body(DevMesh m, DevState<R> s, DevPar
     for (int k = 0; k < 4; k++) nci[k] = ldg(COL(m.nc, k) + i);
     double c[8];
     unsigned bad = 0;
-    visc_face<0>(m, s, P, i, f, nci, c, bad, s.prr);
+    const size_t fl = (size_t)m.fld;
+    visc_face<0>(m, s, P, i, nci, ldg(m.f_j + t), (R)ldg(m.fgeo + t), (R)ldg(m.fgeo + fl + t),
+                 (R)ldg(m.fgeo + 2 * fl + t), ldg(m.fgcv + t), ldg(m.fgcv + fl + t), ldg(m.fgcv + 2 * fl + t), c, bad,
+                 s.prr);
     R rec[FACE_REC];
 #pragma unroll
     for (int k = 0; k < 8; k++) rec[k] = (R)c[k];
@@ -3151,23 +3164,29 @@ static void enqueue_flux(const DevMesh& m, const DevState<R>& s, const DevParams
         k_flux<true, false, Z><<<gf, b, 0, st>>>(m, s, P, stage);
         MARK(KK_SERIAL);
         k_flux_carry<Z><<<1, 1, 0, st>>>(m, s, P);
-    } else if (sizeof(R) != sizeof(double) && m.nface > 0 && m.face_mode >= 2) {
-        cudaMemsetAsync(s.racc, 0, 10 * (size_t)m.ld * sizeof(double), st);
-        if (m.face_mode == 3) {
-            k_facescatter<Z, true><<<grid_for(m.nface, 128), 128, 0, st>>>(m, s, P, m.fcolor, m.nface);
-        } else {
-            for (int c = 0; c < m.ncolor; c++) {
-                const int n = m.fcoff[c + 1] - m.fcoff[c];
-                k_facescatter<Z, false><<<grid_for(n, 128), 128, 0, st>>>(m, s, P, m.fcolor + m.fcoff[c], n);
-            }
-        }
-        k_flux<false, false, Z, true><<<gf, 128, 0, st>>>(m, s, P, stage);
-    } else if (sizeof(R) != sizeof(double) && m.nface > 0) {
-        k_faceflux<Z><<<grid_for(m.nface, 128), 128, 0, st>>>(m, s, P);
-        k_flux<false, true, Z><<<gf, 128, 0, st>>>(m, s, P, stage);
-    } else {
-        k_flux4<Z, 0><<<g4, 128, 0, st>>>(m, s, P, stage);
+        return;
     }
+    if constexpr (sizeof(R) != sizeof(double)) {
+        if (m.nface > 0 && m.face_mode >= 2) {
+            cudaMemsetAsync(s.racc, 0, 10 * (size_t)m.ld * sizeof(double), st);
+            if (m.face_mode == 3) {
+                k_facescatter<Z, true><<<grid_for(m.nface, 128), 128, 0, st>>>(m, s, P, m.fcolor, m.nface);
+            } else {
+                for (int c = 0; c < m.ncolor; c++) {
+                    const int n = m.fcoff[c + 1] - m.fcoff[c];
+                    k_facescatter<Z, false><<<grid_for(n, 128), 128, 0, st>>>(m, s, P, m.fcolor + m.fcoff[c], n);
+                }
+            }
+            k_flux<false, false, Z, true><<<gf, 128, 0, st>>>(m, s, P, stage);
+            return;
+        }
+        if (m.nface > 0) {
+            k_faceflux<Z><<<grid_for(m.nface, 128), 128, 0, st>>>(m, s, P);
+            k_flux<false, true, Z><<<gf, 128, 0, st>>>(m, s, P, stage);
+            return;
+        }
+    }
+    k_flux4<Z, 0><<<g4, 128, 0, st>>>(m, s, P, stage);
 }
 
 // Threads per block of the one-thread-per-cell kernels where the caller leaves
@@ -3225,8 +3244,10 @@ static void enqueue_step(const DevMesh& m, const void* stp, const DevParams& P, 
         if (m.aliased) {
             k_visc<<<gf, b, 0, st>>>(m, s, P);
         } else if (sizeof(R) != sizeof(double) && HP_FACE_VISC && m.nface > 0) {
-            k_facevisc<<<grid_for(m.nface, 128), 128, 0, st>>>(m, s, P);
-            k_vis_gather<<<grid_for(m.neles, 256), 256, 0, st>>>(m, s);
+            if constexpr (sizeof(R) != sizeof(double)) {
+                k_facevisc<<<grid_for(m.nface, 128), 128, 0, st>>>(m, s, P);
+                k_vis_gather<<<grid_for(m.neles, 256), 256, 0, st>>>(m, s);
+            }
         } else if (HP_VISC_SPLIT) {
             k_visc8<0><<<grid_for(8ll * m.neles, 128), 128, 0, st>>>(m, s, P);
         } else {
@@ -3361,11 +3382,7 @@ __global__ void __launch_bounds__(128, HP_FUSED_MINB) k_step_fused(DevMesh m, De
         SYNC
     }
     if (!P.inviscid) {
-        if (sizeof(R) != sizeof(double) && HP_FACE_VISC && m.nface > 0) {
-            PHASE(m.nface, k_facevisc_body(m, s, P, vb))
-            SYNC
-            PHASE(m.neles, k_vis_gather_body<false>(m, s, vb))
-        } else if (HP_VISC_SPLIT) {
+        if (HP_VISC_SPLIT) {
             PHASE(8ll * m.neles, k_visc8_body<0>(m, s, P, vb))
         } else {
             PHASE(4ll * m.neles, k_visc4_body(m, s, P, vb))
@@ -3382,20 +3399,10 @@ __global__ void __launch_bounds__(128, HP_FUSED_MINB) k_step_fused(DevMesh m, De
             SYNC
         }
         if (P.myorder == 2) {
-            if (sizeof(R) != sizeof(double)) {
-                PHASE(m.neles, k_grad_body<true>(m, s, P, vb))
-            } else {
-                PHASE(4ll * m.neles, k_grad4_body<0>(m, s, P, vb))
-            }
+            PHASE(4ll * m.neles, k_grad4_body<0>(m, s, P, vb))
             SYNC
         }
-        if (sizeof(R) != sizeof(double) && m.nface > 0) {
-            PHASE(m.nface, (k_faceflux_body<Z, false>(m, s, P, vb)))
-            SYNC
-            PHASE(m.neles, (k_flux_body<false, true, Z, false, false>(m, s, P, stage, vb)))
-        } else {
-            PHASE(4ll * m.neles, (k_flux4_body<Z, 0, false>(m, s, P, stage, vb)))
-        }
+        PHASE(4ll * m.neles, (k_flux4_body<Z, 0, false>(m, s, P, stage, vb)))
         SYNC
     }
     PHASE(m.neles, { k_prim_body<PM_NEXT>(m, s, P, vb); __syncthreads(); })
