@@ -166,6 +166,9 @@ struct DevState {
                              // double, a float copy otherwise
     R* gr;                   // [33][ld]
     double* phi;             // [ld]
+    R* agrad;                // [3][ld] 1/r-weighted gradient of alpha_g (the
+                             // sources'), formed beside the others by the
+                             // FP32 gradient kernel; null where that does not run
     double *anu, *d2q;       // [2][ld], [10][ld]
     double *d24, *vis;       // [10][ld], [8][ld]
     double* egt;             // [2][ld] ghost egtotal/eptotal (aliased meshes)
@@ -192,6 +195,7 @@ template <class R>
 inline DevState<double> fp64_view(const DevState<R>& s) {
     DevState<double> v;
     v.cn = s.cn; v.cu = s.cu; v.cn1 = s.cn1; v.pr = s.pr; v.prr = s.pr; v.gr = s.gr64; v.phi = s.phi;
+    v.agrad = nullptr;
     v.anu = s.anu; v.d2q = s.d2q; v.d24 = s.d24; v.vis = s.vis; v.egt = s.egt;
     v.qpr = s.qpr; v.anuq = s.anuq; v.qdrag = s.qdrag; v.racc = s.racc; v.ff = nullptr;
     v.s = s.s; v.diag = s.diag; v.max_diag = s.max_diag; v.gr64 = s.gr64;
@@ -248,6 +252,9 @@ struct Variant {
     // 1 when the viscous fluxes are evaluated once per face on meshes with a
     // face list (k_facevisc + k_vis_gather instead of one kernel)
     int face_visc;
+    // 1 when the flux kernel of meshes with a face list recovers the next
+    // stage's primitives (see recover_in_flux in hp_kernels.cuh)
+    int flux_recovers;
     // fills the tables that the flux kernels read (m.nrm), once per handle
     void (*setup)(const DevMesh&, cudaStream_t);
     // fused step (one cooperative launch per step): the grid it runs with on

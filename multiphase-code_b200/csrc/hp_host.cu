@@ -228,7 +228,9 @@ static void plan_arena(hp_handle* h, Arena& a, int neles, int nghosts, long long
         s.gr64 = nullptr;
     }
     m.dxnf = m.fxof = nullptr;
+    s.agrad = nullptr;
     if (gb != D && !h->aliased) {
+        s.agrad = (double*)a.take(3 * (size_t)ld * gb);   // (read by the mixed variant alone)
         m.dxnf = (const float*)a.take(12 * (size_t)ld * sizeof(float));
         m.fxof = (const float*)a.take(12 * (size_t)ld * sizeof(float));
     }
@@ -1779,6 +1781,10 @@ extern "C" int hp_info(const hp_handle* h, int64_t* kernels_per_step, int64_t* d
         if (h->dm.nface > 0 && !h->prm.inviscid && h->var->face_visc) n += 1;   // k_vis_gather
         n += (int64_t)h->dp.nstage * per_stage + 1;
         if (h->aliased) n += 2;
+        // the flux kernel of the face-based variants recovers the next stage's
+        // primitives itself (see recover_in_flux)
+        if (grad && h->var->flux_recovers && h->dm.nface > 0 && !h->xfn && h->dm.nfringe == 0 && h->dm.nhalo == 0 && h->neq == 10)
+            n -= h->dp.nstage - 1;
         if (h->neq == 22) n += 2 + (int64_t)h->dp.nstage * (2 + (h->nghosts ? 1 : 0));   // k_qrs_*
         if (h->nwall > 0)   // FP64 wall layers: viscous once, gradients and fluxes per stage
             n += (h->prm.inviscid ? 0 : 1) + (int64_t)h->dp.nstage * (grad + 1);

@@ -286,6 +286,17 @@ __device__ __forceinline__ void blend_phases(const DevParams& P, S& phig, S& phi
     }
 }
 
+// a b + c, with one rounding in the variants built with contraction and two
+// in those without
+#ifndef HP_CONTRACT
+#define HP_CONTRACT 0
+#endif
+template <class T>
+__device__ __forceinline__ T mad(T a, T b, T c) {
+    if constexpr (HP_CONTRACT != 0) return fma(a, b, c);
+    else return a * b + c;
+}
+
 // qm: the dispersed masses cn(11), cn(15), cn(19) of the five-phase model
 // (src/sr_primitive.F90:56-80), or null for the two-phase model
 __device__ __forceinline__ void prim_full(double cd[10], PrimV& q, const DevParams& P,
@@ -336,7 +347,11 @@ __device__ __forceinline__ void prim_full(double cd[10], PrimV& q, const DevPara
     S eg2 = q.pg / ((gamag - S(1.0)) * q.rog);
     S ep2 = (q.pp + gamap * pinf) / ((gamap - S(1.0)) * q.rop);
     S egt = eg2 + S(0.5) * (q.ug * q.ug + q.vg * q.vg + q.wg * q.wg);
-    S ept = ep2 + S(0.5) * (q.up * q.up + q.vp * q.vp + q.wp * q.wp);
+    // the squares summed in order, contracted in the one way of the two that
+    // k_prim was compiled to: the flux kernel's copy of this function took
+    // the other, a last bit in 0.5% of a shock's cells
+    const S kep = mad(q.wp, q.wp, mad(q.vp, q.vp, q.up * q.up));
+    S ept = ep2 + S(0.5) * kep;
     cd[0] = q.phig * q.rog;
     cd[1] = q.phig * q.rog * q.ug;
     cd[2] = q.phig * q.rog * q.vg;
@@ -929,6 +944,41 @@ __device__ __forceinline__ bool wall_face(const DevMesh& m, int i, int f) {
     return j >= m.neles || ldg(m.wclass + j) != 0;
 }
 
+// FP32 fluxes with an FP64 state path (mixed): the gradient kernel forms the
+// sources' alpha_g gradient and the flux kernel recovers the next stage's
+// primitives.  The all-FP32 variant keeps its passes apart: its recovery
+// rounds to FP32 at every operation, and compiled into the flux kernel it
+// rounds otherwise (7e-6 in the state after 5 steps of a 15,552-cell shock).
+enum { FLUX_RECOVERS = sizeof(R) != sizeof(double) && sizeof(S) == sizeof(double) };
+
+// The sources' gradient of alpha_g (1/r weights, src/sr_source.F90:100-117)
+// from the centroid differences and the differences pa of alpha_g; the
+// variants without set-up tables.
+#if !HP_LSQ_TABLE
+__device__ __forceinline__ void alpha_gradient(const R xa[4], const R ya[4], const R za[4], const R pa[4], R& dpx,
+                                               R& dpy, R& dpz) {
+    R wt[4], rw[4];
+#define DW(x, f) div_rn((x), wt[f], rw[f])
+#pragma unroll
+    for (int f = 0; f < 4; f++) { wt[f] = sqrt(xa[f] * xa[f] + ya[f] * ya[f] + za[f] * za[f]); rw[f] = rcp(wt[f]); }
+    const R a1 = DW(xa[0] * xa[0], 0) + DW(xa[1] * xa[1], 1) + DW(xa[2] * xa[2], 2) + DW(xa[3] * xa[3], 3);
+    const R a2 = DW(ya[0] * ya[0], 0) + DW(ya[1] * ya[1], 1) + DW(ya[2] * ya[2], 2) + DW(ya[3] * ya[3], 3);
+    const R a3 = DW(za[0] * za[0], 0) + DW(za[1] * za[1], 1) + DW(za[2] * za[2], 2) + DW(za[3] * za[3], 3);
+    const R b1 = DW(xa[0] * ya[0], 0) + DW(xa[1] * ya[1], 1) + DW(xa[2] * ya[2], 2) + DW(xa[3] * ya[3], 3);
+    const R b2 = DW(xa[0] * za[0], 0) + DW(xa[1] * za[1], 1) + DW(xa[2] * za[2], 2) + DW(xa[3] * za[3], 3);
+    const R b3 = DW(ya[0] * za[0], 0) + DW(ya[1] * za[1], 1) + DW(ya[2] * za[2], 2) + DW(ya[3] * za[3], 3);
+    const R c1 = DW(pa[0] * xa[0], 0) + DW(pa[1] * xa[1], 1) + DW(pa[2] * xa[2], 2) + DW(pa[3] * xa[3], 3);
+    const R c2 = DW(pa[0] * ya[0], 0) + DW(pa[1] * ya[1], 1) + DW(pa[2] * ya[2], 2) + DW(pa[3] * ya[3], 3);
+    const R c3 = DW(pa[0] * za[0], 0) + DW(pa[1] * za[1], 1) + DW(pa[2] * za[2], 2) + DW(pa[3] * za[3], 3);
+#undef DW
+    const R dnr = det3(a1, b1, b2, b1, a2, b3, b2, b3, a3);
+    const R rdnr = rcp(dnr);
+    dpx = div_rn(det3(c1, c2, c3, b1, a2, b3, b2, b3, a3), dnr, rdnr);
+    dpy = div_rn(det3(a1, b1, b2, c1, c2, c3, b2, b3, a3), dnr, rdnr);
+    dpz = div_rn(det3(a1, b1, b2, b1, a2, b3, c1, c2, c3), dnr, rdnr);
+}
+#endif
+
 template <bool FPR>
 __device__ __forceinline__ void k_grad_body(DevMesh m, DevState<R> s, DevParams P, int bid) {
     using PT = typename std::conditional<FPR, R, double>::type;
@@ -993,6 +1043,18 @@ __device__ __forceinline__ void k_grad_body(DevMesh m, DevState<R> s, DevParams 
             const double qi = ldg(q + i);
             qa = (R)(ldg(q + n[0]) - qi); qb = (R)(ldg(q + n[1]) - qi);
             qc = (R)(ldg(q + n[2]) - qi); qd = (R)(ldg(q + n[3]) - qi);
+#if !HP_LSQ_TABLE
+            // the sources need the same differences: their gradient is formed
+            // here too, and the flux kernel gathers nothing but face records
+            if constexpr (FLUX_RECOVERS) {
+                const R pa[4] = {qa, qb, qc, qd};
+                R dpx, dpy, dpz;
+                alpha_gradient(xa, ya, za, pa, dpx, dpy, dpz);
+                COL(s.agrad, 0)[i] = dpx;
+                COL(s.agrad, 1)[i] = dpy;
+                COL(s.agrad, 2)[i] = dpz;
+            }
+#endif
         } else {
             const PT* q = COL(prb, pcol[v]);
             PT qi = ldg(q + i);
@@ -1616,17 +1678,47 @@ __global__ void k_flux_carry(DevMesh m, DevState<R> s, DevParams P) {
     for (int k = 0; k < 5; k++) s.s->fcarry[5 + k] = (double)tmp[k];
 }
 
+// Primitives of the state c of cell i, stored with the state they give back
+// (k_prim's recovery: the same call with the same two branches, so that the
+// variants built with contraction round it the same way).
+__device__ __forceinline__ void recover_store(const DevMesh& m, const DevState<R>& s, const DevParams& P, int i,
+                                              double c[10]) {
+    PrimV q;
+    double qm[3];
+    if (P.five_phase) {
+        qm[0] = COL(s.cn, 10)[i]; qm[1] = COL(s.cn, 14)[i]; qm[2] = COL(s.cn, 18)[i];
+    }
+    prim_full(c, q, P, P.five_phase ? qm : nullptr);
+#pragma unroll
+    for (int k = 0; k < 10; k++) COL(s.cn, k)[i] = c[k];
+    store_prims(m, s.pr, i, q);
+    if constexpr (sizeof(R) != sizeof(double)) store_prims(m, s.prr, i, q);
+}
+
 // Residual (4 faces + interphase sources, src/sr_source.F90:42-155) and the
 // RK stage update of src/sr_RK.F90 fused; iblank == 1 cells.
 // FACE: the four face fluxes are gathered from k_faceflux's output (face-
-// based variants) instead of evaluated here.
-template <bool ALIASED, bool FACE, int Z, bool ACC = false, bool NC = true>
+// based variants) instead of evaluated here (ACC: face modes 2 and 3, their
+// sums).  AG: the alpha_g gradient is k_grad's.  REC: the updated state is
+// recovered to primitives at once, as the next stage opens
+// (src/sr_primitiveplusbc.F90:36-172), for every cell of the mesh: with AG no
+// thread reads another cell's primitives, so writing them here is safe, and
+// the state makes one trip through memory instead of two.
+template <bool ALIASED, bool FACE, int Z, bool ACC = false, bool AG = false, bool REC = false>
 __device__ __forceinline__ void k_flux_body(DevMesh m, DevState<R> s, DevParams P, int stage, int bid) {
     int i = bid * blockDim.x + threadIdx.x;
     if (i >= m.neles) return;
-    if (ldg(m.iblank + i) != 1) return;
-    // cells of the FP64 wall layers: updated by the FP64 kernels
-    if (sizeof(R) != sizeof(double) && m.nwall > 0 && ldg(m.wclass + i)) return;
+    // cells of the FP64 wall layers are updated by the FP64 kernels
+    const bool upd = ldg(m.iblank + i) == 1 && !(sizeof(R) != sizeof(double) && m.nwall > 0 && ldg(m.wclass + i));
+    double cnew[10];
+    if (!upd) {
+        if constexpr (REC) {
+#pragma unroll
+            for (int k = 0; k < 10; k++) cnew[k] = COL(s.cn, k)[i];
+            recover_store(m, s, P, i, cnew);
+        }
+        return;
+    }
     double rhs[10];
 #pragma unroll
     for (int k = 0; k < 10; k++) rhs[k] = 0.0;
@@ -1643,7 +1735,7 @@ __device__ __forceinline__ void k_flux_body(DevMesh m, DevState<R> s, DevParams 
             const int fid = (code > 0 ? code : -code) - 1;
             const R sg = code > 0 ? R(1) : R(-1);
             R e[FACE_REC];
-            load_frec<NC>(s.ff + (size_t)FACE_REC * (size_t)fid, e);
+            load_frec(s.ff + (size_t)FACE_REC * (size_t)fid, e);
 #pragma unroll
             for (int k = 0; k < 10; k++) e[k] = sg * e[k];
             if (e[10] != R(0)) {
@@ -1720,44 +1812,40 @@ __device__ __forceinline__ void k_flux_body(DevMesh m, DevState<R> s, DevParams 
         const R uint_ = div_rn(phig * rog * ug + omg * rop * up, den, rden);
         const R vint = div_rn(phig * rog * vg + omg * rop * vp, den, rden);
         const R wint = div_rn(phig * rog * wg + omg * rop * wp, den, rden);
-        const double x0 = ldg(m.xc + i), y0 = ldg(m.yc + i), z0 = ldg(m.zc + i);
-        R xa[4], ya[4], za[4], pa[4], wt[4];
+        R dpx, dpy, dpz;
+        if constexpr (AG) {
+            dpx = COL(s.agrad, 0)[i];
+            dpy = COL(s.agrad, 1)[i];
+            dpz = COL(s.agrad, 2)[i];
+        } else {
+            const double x0 = ldg(m.xc + i), y0 = ldg(m.yc + i), z0 = ldg(m.zc + i);
+            R xa[4], ya[4], za[4], pa[4];
 #pragma unroll
-        for (int f = 0; f < 4; f++) {
-            int n = ldg(COL(m.nc, f) + i);
-            xa[f] = (R)(ldg(m.xc + n) - x0);
-            ya[f] = (R)(ldg(m.yc + n) - y0);
-            za[f] = (R)(ldg(m.zc + n) - z0);
-            pa[f] = (R)(COL(pr, P_PHIG)[n] - COL(pr, P_PHIG)[i]);
+            for (int f = 0; f < 4; f++) {
+                int n = ldg(COL(m.nc, f) + i);
+                xa[f] = (R)(ldg(m.xc + n) - x0);
+                ya[f] = (R)(ldg(m.yc + n) - y0);
+                za[f] = (R)(ldg(m.zc + n) - z0);
+                pa[f] = (R)(COL(pr, P_PHIG)[n] - COL(pr, P_PHIG)[i]);
+            }
+#if HP_LSQ_TABLE
+            R wt[4], rw[4];
+#pragma unroll
+            for (int f = 0; f < 4; f++) { wt[f] = (R)ldg(COL(m.lsqb, f) + i); rw[f] = rcp(wt[f]); }
+            const R a1 = (R)ldg(COL(m.lsqb, 4) + i), a2 = (R)ldg(COL(m.lsqb, 5) + i), a3 = (R)ldg(COL(m.lsqb, 6) + i);
+            const R b1 = (R)ldg(COL(m.lsqb, 7) + i), b2 = (R)ldg(COL(m.lsqb, 8) + i), b3 = (R)ldg(COL(m.lsqb, 9) + i);
+            R c1 = DW(pa[0] * xa[0], 0) + DW(pa[1] * xa[1], 1) + DW(pa[2] * xa[2], 2) + DW(pa[3] * xa[3], 3);
+            R c2 = DW(pa[0] * ya[0], 0) + DW(pa[1] * ya[1], 1) + DW(pa[2] * ya[2], 2) + DW(pa[3] * ya[3], 3);
+            R c3 = DW(pa[0] * za[0], 0) + DW(pa[1] * za[1], 1) + DW(pa[2] * za[2], 2) + DW(pa[3] * za[3], 3);
+            const R dnr = (R)ldg(COL(m.lsqb, 10) + i);
+            const R rdnr = rcp(dnr);
+            dpx = div_rn(det3(c1, c2, c3, b1, a2, b3, b2, b3, a3), dnr, rdnr);
+            dpy = div_rn(det3(a1, b1, b2, c1, c2, c3, b2, b3, a3), dnr, rdnr);
+            dpz = div_rn(det3(a1, b1, b2, b1, a2, b3, c1, c2, c3), dnr, rdnr);
+#else
+            alpha_gradient(xa, ya, za, pa, dpx, dpy, dpz);
+#endif
         }
-        R rw[4];
-#if HP_LSQ_TABLE
-#pragma unroll
-        for (int f = 0; f < 4; f++) { wt[f] = (R)ldg(COL(m.lsqb, f) + i); rw[f] = rcp(wt[f]); }
-        const R a1 = (R)ldg(COL(m.lsqb, 4) + i), a2 = (R)ldg(COL(m.lsqb, 5) + i), a3 = (R)ldg(COL(m.lsqb, 6) + i);
-        const R b1 = (R)ldg(COL(m.lsqb, 7) + i), b2 = (R)ldg(COL(m.lsqb, 8) + i), b3 = (R)ldg(COL(m.lsqb, 9) + i);
-#else
-#pragma unroll
-        for (int f = 0; f < 4; f++) { wt[f] = sqrt(xa[f] * xa[f] + ya[f] * ya[f] + za[f] * za[f]); rw[f] = rcp(wt[f]); }
-        const R a1 = DW(xa[0] * xa[0], 0) + DW(xa[1] * xa[1], 1) + DW(xa[2] * xa[2], 2) + DW(xa[3] * xa[3], 3);
-        const R a2 = DW(ya[0] * ya[0], 0) + DW(ya[1] * ya[1], 1) + DW(ya[2] * ya[2], 2) + DW(ya[3] * ya[3], 3);
-        const R a3 = DW(za[0] * za[0], 0) + DW(za[1] * za[1], 1) + DW(za[2] * za[2], 2) + DW(za[3] * za[3], 3);
-        const R b1 = DW(xa[0] * ya[0], 0) + DW(xa[1] * ya[1], 1) + DW(xa[2] * ya[2], 2) + DW(xa[3] * ya[3], 3);
-        const R b2 = DW(xa[0] * za[0], 0) + DW(xa[1] * za[1], 1) + DW(xa[2] * za[2], 2) + DW(xa[3] * za[3], 3);
-        const R b3 = DW(ya[0] * za[0], 0) + DW(ya[1] * za[1], 1) + DW(ya[2] * za[2], 2) + DW(ya[3] * za[3], 3);
-#endif
-        R c1 = DW(pa[0] * xa[0], 0) + DW(pa[1] * xa[1], 1) + DW(pa[2] * xa[2], 2) + DW(pa[3] * xa[3], 3);
-        R c2 = DW(pa[0] * ya[0], 0) + DW(pa[1] * ya[1], 1) + DW(pa[2] * ya[2], 2) + DW(pa[3] * ya[3], 3);
-        R c3 = DW(pa[0] * za[0], 0) + DW(pa[1] * za[1], 1) + DW(pa[2] * za[2], 2) + DW(pa[3] * za[3], 3);
-#if HP_LSQ_TABLE
-        const R dnr = (R)ldg(COL(m.lsqb, 10) + i);
-#else
-        const R dnr = det3(a1, b1, b2, b1, a2, b3, b2, b3, a3);
-#endif
-        const R rdnr = rcp(dnr);
-        R dpx = div_rn(det3(c1, c2, c3, b1, a2, b3, b2, b3, a3), dnr, rdnr);
-        R dpy = div_rn(det3(a1, b1, b2, c1, c2, c3, b2, b3, a3), dnr, rdnr);
-        R dpz = div_rn(det3(a1, b1, b2, b1, a2, b3, c1, c2, c3), dnr, rdnr);
         const R g = R(0);   // gravity (src/main.F90:341)
         R en = pint * (uint_ * dpx + vint * dpy + wint * dpz) + uint_ * fdgx + vint * fdgy + wint * fdgz + qsource;
         const double* vis = s.vis;
@@ -1785,30 +1873,33 @@ __device__ __forceinline__ void k_flux_body(DevMesh m, DevState<R> s, DevParams 
         const double r = rhs[j] - COL(s.d24, j)[i];
         const double cu = COL(s.cu, j)[i];
         double* cnp = COL(s.cn, j) + i;
+        double v;
         if (P.rk_scheme == 0) {
             if (stage == 1) {
-                double v = cu - (11.0 / 20.0) * dtbyvol * r;
-                *cnp = v;
+                v = cu - (11.0 / 20.0) * dtbyvol * r;
                 COL(s.cn1, j)[i] = v;
             } else {
                 double upd = *cnp - (11.0 / 20.0) * dtbyvol * r;
-                if (stage == 2) *cnp = (3.0 / 8.0) * cu + (5.0 / 8.0) * upd;
-                else if (stage == 3) *cnp = (4.0 / 9.0) * cu + (5.0 / 9.0) * upd;
-                else *cnp = (111.0 / 1331.0) * cu + (260.0 / 1331.0) * COL(s.cn1, j)[i] + (960.0 / 1331.0) * upd;
+                if (stage == 2) v = (3.0 / 8.0) * cu + (5.0 / 8.0) * upd;
+                else if (stage == 3) v = (4.0 / 9.0) * cu + (5.0 / 9.0) * upd;
+                else v = (111.0 / 1331.0) * cu + (260.0 / 1331.0) * COL(s.cn1, j)[i] + (960.0 / 1331.0) * upd;
             }
         } else {
-            if (stage == 1) *cnp = cu - dtbyvol * r;
+            if (stage == 1) v = cu - dtbyvol * r;
             else {
                 double upd = *cnp - dtbyvol * r;
-                if (stage == 2) *cnp = 0.75 * cu + 0.25 * upd;
-                else *cnp = (1.0 / 3.0) * cu + (2.0 / 3.0) * upd;
+                if (stage == 2) v = 0.75 * cu + 0.25 * upd;
+                else v = (1.0 / 3.0) * cu + (2.0 / 3.0) * upd;
             }
         }
+        if constexpr (REC) cnew[j] = v;
+        else *cnp = v;
     }
+    if constexpr (REC) recover_store(m, s, P, i, cnew);
 }
-template <bool ALIASED, bool FACE, int Z, bool ACC = false>
+template <bool ALIASED, bool FACE, int Z, bool ACC = false, bool AG = false, bool REC = false>
 __global__ void __launch_bounds__(128) k_flux(DevMesh m, DevState<R> s, DevParams P, int stage) {
-    k_flux_body<ALIASED, FACE, Z, ACC>(m, s, P, stage, blockIdx.x);
+    k_flux_body<ALIASED, FACE, Z, ACC, AG, REC>(m, s, P, stage, blockIdx.x);
 }
 
 
@@ -3154,19 +3245,45 @@ static void setup(const DevMesh& m, cudaStream_t st) {
 #define MARK(k) do { if (hook && hook->mark) hook->mark(hook->ctx, (k)); } while (0)
 #define EXCHANGE(p) do { if (hook && hook->exchange) hook->exchange(hook->xctx, (p)); } while (0)
 
+// The flux kernel of the face-based FP32 variants recovers the next stage's
+// primitives (k_flux with REC) where nothing else changes the state between
+// the stages: no overset fringe, partition halo or exchange, two phases; and
+// where the gradients run, whose kernel forms what the sources read of the
+// neighbours.
+static bool recover_in_flux(const DevMesh& m, const DevParams& P, const StepHook* hook) {
+    return FLUX_RECOVERS && m.nface > 0 && m.nfringe == 0 && m.nhalo == 0 && !P.five_phase &&
+           P.myorder == 2 && P.myflux != 3 && !(hook && hook->exchange);
+}
+
+// k_flux of the face-based variants (ACC: face modes 2 and 3).  rec: recover
+// the next stage's primitives.
+template <int Z, bool ACC>
+static void enqueue_face_update(const DevMesh& m, const DevState<R>& s, const DevParams& P, cudaStream_t st,
+                                int stage, bool rec) {
+    const unsigned g = grid_for(m.neles, 128);
+    if constexpr (FLUX_RECOVERS && Z != 2) {
+        if (P.myorder == 2) {
+            if (rec) k_flux<false, !ACC, Z, ACC, true, true><<<g, 128, 0, st>>>(m, s, P, stage);
+            else k_flux<false, !ACC, Z, ACC, true><<<g, 128, 0, st>>>(m, s, P, stage);
+            return;
+        }
+    }
+    k_flux<false, !ACC, Z, ACC><<<g, 128, 0, st>>>(m, s, P, stage);
+}
+
 // residual + RK update of one stage with Riemann solver Z (see face_eval)
 template <int Z>
 static void enqueue_flux(const DevMesh& m, const DevState<R>& s, const DevParams& P, cudaStream_t st, int stage,
                          const StepHook* hook) {
-    const int b = 128;
-    const unsigned gf = grid_for(m.neles, b), g4 = grid_for(4ll * m.neles, 128);
+    const unsigned g4 = grid_for(4ll * m.neles, 128);
     if (m.aliased) {
-        k_flux<true, false, Z><<<gf, b, 0, st>>>(m, s, P, stage);
+        k_flux<true, false, Z><<<grid_for(m.neles, 128), 128, 0, st>>>(m, s, P, stage);
         MARK(KK_SERIAL);
         k_flux_carry<Z><<<1, 1, 0, st>>>(m, s, P);
         return;
     }
     if constexpr (sizeof(R) != sizeof(double)) {
+        const bool rec = stage < P.nstage && recover_in_flux(m, P, hook);
         if (m.nface > 0 && m.face_mode >= 2) {
             cudaMemsetAsync(s.racc, 0, 10 * (size_t)m.ld * sizeof(double), st);
             if (m.face_mode == 3) {
@@ -3177,16 +3294,20 @@ static void enqueue_flux(const DevMesh& m, const DevState<R>& s, const DevParams
                     k_facescatter<Z, false><<<grid_for(n, 128), 128, 0, st>>>(m, s, P, m.fcolor + m.fcoff[c], n);
                 }
             }
-            k_flux<false, false, Z, true><<<gf, 128, 0, st>>>(m, s, P, stage);
-            return;
-        }
-        if (m.nface > 0) {
+        } else if (m.nface > 0) {
             k_faceflux<Z><<<grid_for(m.nface, 128), 128, 0, st>>>(m, s, P);
-            k_flux<false, true, Z><<<gf, 128, 0, st>>>(m, s, P, stage);
-            return;
+        } else {
+            k_flux4<Z, 0><<<g4, 128, 0, st>>>(m, s, P, stage);
         }
+        // FP64 wall layers: their fluxes, sources and RK update, before the
+        // kernel that may replace the primitives these read (the FP32 kernels
+        // leave those cells' update alone)
+        if (m.nwall > 0) wall_fp64.flux(m, fp64_view(s), P, st, stage);
+        if (m.nface > 0 && m.face_mode >= 2) enqueue_face_update<Z, true>(m, s, P, st, stage, rec);
+        else if (m.nface > 0) enqueue_face_update<Z, false>(m, s, P, st, stage, rec);
+    } else {
+        k_flux4<Z, 0><<<g4, 128, 0, st>>>(m, s, P, stage);
     }
-    k_flux4<Z, 0><<<g4, 128, 0, st>>>(m, s, P, stage);
 }
 
 // Threads per block of the one-thread-per-cell kernels where the caller leaves
@@ -3258,8 +3379,10 @@ static void enqueue_step(const DevMesh& m, const void* stp, const DevParams& P, 
     }
     for (int stage = 1; stage <= P.nstage; stage++) {
         // src/sr_hllcbatten.F90:29-33: primitiveplusbc, derivative, limiter
-        MARK(KK_PRIM_STAGE);
-        k_prim<PM_STAGE><<<ge, cb, 0, st>>>(m, s, P);
+        if (stage == 1 || !recover_in_flux(m, P, hook)) {
+            MARK(KK_PRIM_STAGE);
+            k_prim<PM_STAGE><<<ge, cb, 0, st>>>(m, s, P);
+        }
         if (m.nghosts > 0) {
             MARK(KK_BC);
             if (m.aliased) k_bc_serial<false><<<1, 1, 0, st>>>(m, s, P);
@@ -3287,9 +3410,6 @@ static void enqueue_step(const DevMesh& m, const void* stp, const DevParams& P, 
         if (P.myflux == 1) enqueue_flux<1>(m, s, P, st, stage, hook);
         else if (P.myflux == 3) enqueue_flux<2>(m, s, P, st, stage, hook);
         else enqueue_flux<0>(m, s, P, st, stage, hook);
-        // FP64 wall layers: their fluxes, sources and RK update (the FP32
-        // kernels above left those cells alone)
-        if (sizeof(R) != sizeof(double) && m.nwall > 0) wall_fp64.flux(m, fp64_view(s), P, st, stage);
         if (m.nfringe > 0) {
             MARK(KK_OVERSET);
             k_overset<<<grid_for(m.nfringe, 256), 256, 0, st>>>(m, s);

@@ -3,6 +3,8 @@
 // float-rounded values.  The precision-stress reference point: it shows what
 // the steps the mixed variant keeps in FP64 would lose.
 #define HP_NS v_fp32
+// built with multiply-add contraction
+#define HP_CONTRACT 1
 #define HP_R float
 #define HP_S float
 // geometry-only least-squares terms: recomputed in FP32
@@ -22,6 +24,7 @@
 #include "hp_kernels.cuh"
 
 namespace hp {
-const Variant variant_fp32 = {"fp32", sizeof(float), &v_fp32::enqueue_start, &v_fp32::enqueue_step, (HP_FACE_VISC && sizeof(HP_R) != sizeof(double)) ? 1 : 0, &v_fp32::setup,
+const Variant variant_fp32 = {"fp32", sizeof(float), &v_fp32::enqueue_start, &v_fp32::enqueue_step, (HP_FACE_VISC && sizeof(HP_R) != sizeof(double)) ? 1 : 0,
+    v_fp32::FLUX_RECOVERS, &v_fp32::setup,
     &v_fp32::fused_grid, &v_fp32::enqueue_fused};
 }

@@ -1,5 +1,7 @@
 // Precision variant "fp64": flux/gradient arithmetic in double.
 #define HP_NS v_fp64
+// built with multiply-add contraction
+#define HP_CONTRACT 1
 #define HP_R double
 // geometry-only least-squares terms: loaded from the set-up tables
 #define HP_LSQ_TABLE 1
@@ -34,7 +36,8 @@
 #include "hp_kernels.cuh"
 
 namespace hp {
-const Variant variant_fp64 = {"fp64", sizeof(double), &v_fp64::enqueue_start, &v_fp64::enqueue_step, (HP_FACE_VISC && sizeof(HP_R) != sizeof(double)) ? 1 : 0, &v_fp64::setup,
+const Variant variant_fp64 = {"fp64", sizeof(double), &v_fp64::enqueue_start, &v_fp64::enqueue_step, (HP_FACE_VISC && sizeof(HP_R) != sizeof(double)) ? 1 : 0,
+    v_fp64::FLUX_RECOVERS, &v_fp64::setup,
     &v_fp64::fused_grid, &v_fp64::enqueue_fused};
 
 // The FP64 (FMA) kernels over the wall-layer cell lists, for the steps of the

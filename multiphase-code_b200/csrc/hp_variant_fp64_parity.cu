@@ -36,6 +36,7 @@
 #include "hp_kernels.cuh"
 
 namespace hp {
-const Variant variant_fp64_parity = {"fp64_parity", sizeof(double), &v_fp64_parity::enqueue_start, &v_fp64_parity::enqueue_step, (HP_FACE_VISC && sizeof(HP_R) != sizeof(double)) ? 1 : 0, &v_fp64_parity::setup,
+const Variant variant_fp64_parity = {"fp64_parity", sizeof(double), &v_fp64_parity::enqueue_start, &v_fp64_parity::enqueue_step, (HP_FACE_VISC && sizeof(HP_R) != sizeof(double)) ? 1 : 0,
+    v_fp64_parity::FLUX_RECOVERS, &v_fp64_parity::setup,
     &v_fp64_parity::fused_grid, &v_fp64_parity::enqueue_fused};
 }
