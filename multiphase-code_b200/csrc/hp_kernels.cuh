@@ -2219,6 +2219,7 @@ __global__ void __launch_bounds__(128, HP_GRAD4_MINB) k_grad4(DevMesh m, DevStat
 // and cn; TAIL_LD cells (one 128-thread block) per column.  (Staging the 14
 // primitives and the 12 centroid differences as well measured 2% slower:
 // the face evaluation has just read the primitives.)
+enum { FLUX4_T = 128 };   // threads of the four-lane flux kernel's blocks
 enum { TAIL_DL = 0, TAIL_VOL = 1, TAIL_LSQB = 2, TAIL_VIS = 18, TAIL_D24 = 26, TAIL_CU = 36, TAIL_CN = 46,
        TAIL_N = 56, TAIL_LD = 32 };
 __device__ __forceinline__ const double* tail_col(const DevMesh& m, const DevState<R>& s, int k) {
@@ -2232,14 +2233,16 @@ __device__ __forceinline__ const double* tail_col(const DevMesh& m, const DevSta
 }
 
 // Residual + sources + RK update with four lanes per cell: lane q evaluates
-// face q; every lane re-assembles the residual in face order and computes
-// the sources; lane q writes variables q, q+4, q+8.  F selects the division
+// face q; the four faces' fluxes meet in shared memory (sres), and lane q sums
+// variables q, q+4, q+8 over the faces in order, adds their sources and
+// updates them.  (Every lane re-assembling all ten through shuffles took 80
+// of them and 40 additions: 983,040 cells, 802 us a launch against 703.)  F selects the division
 // form (see mdiv).  The fast form returns false, before any store, when a lane
 // of the warp flagged an operand (cn is read and written here, so the stores
 // must wait for that vote).
 template <int F, int Z, bool NC = true, bool PF = false>
 __device__ __forceinline__ bool flux4_body(const DevMesh& m, const DevState<R>& s, const DevParams& P, int stage,
-                                           int i, int q, bool active, const double* pf = nullptr) {
+                                           int i, int q, bool active, R* sres, const double* pf = nullptr) {
     unsigned bad = 0;
     const R* pr = s.prr;
     // PF: the cell's own values after the face evaluation come from the
@@ -2247,23 +2250,26 @@ __device__ __forceinline__ bool flux4_body(const DevMesh& m, const DevState<R>& 
     // k of the TAIL_* map)
 #define TL(k, expr) (PF ? (R)pf[(k) * TAIL_LD] : (R)(expr))
 #define TLS(k, expr) (PF ? (S)pf[(k) * TAIL_LD] : (S)(expr))
-    // this lane's face
-    R eff[10];
+    // this lane's face, into the warp's part of sres (column k: component k
+    // of the block's 128 faces)
+    const int tid = (int)(threadIdx.x & (FLUX4_T - 1));
     int flags;
     {
         FaceOut o;
         face_eval<F, Z, R, NC>(m, s, P, i, q, o, bad, s.prr);
         if (o.wall) {
 #pragma unroll
-            for (int k = 0; k < 10; k++) eff[k] = R(0);
-            eff[1] = o.w[0]; eff[2] = o.w[1]; eff[3] = o.w[2];
-            eff[6] = o.w[3]; eff[7] = o.w[4]; eff[8] = o.w[5];
+            for (int k = 0; k < 10; k++)
+                if (k == 0 || k == 4 || k == 5 || k == 9) sres[k * FLUX4_T + tid] = R(0);
+            sres[1 * FLUX4_T + tid] = o.w[0]; sres[2 * FLUX4_T + tid] = o.w[1]; sres[3 * FLUX4_T + tid] = o.w[2];
+            sres[6 * FLUX4_T + tid] = o.w[3]; sres[7 * FLUX4_T + tid] = o.w[4]; sres[8 * FLUX4_T + tid] = o.w[5];
         } else {
 #pragma unroll
-            for (int k = 0; k < 10; k++) eff[k] = o.F[k];
+            for (int k = 0; k < 10; k++) sres[k * FLUX4_T + tid] = o.F[k];
         }
         flags = (o.wall ? 1 : 0) | (o.takeg ? 2 : 0) | (o.takep ? 4 : 0);
     }
+    __syncwarp();
     if constexpr (PF) {
         cp_async_wait_all();
         __syncwarp();
@@ -2279,33 +2285,28 @@ __device__ __forceinline__ bool flux4_body(const DevMesh& m, const DevState<R>& 
 #endif
     // alpha_g differences from the FP64 primitives (see k_grad)
     const R pq = (R)(COL(s.pr, P_PHIG)[nq] - COL(s.pr, P_PHIG)[i]);
-    // residual in face order 1..4 (src/sr_hllcbatten.F90:534-552)
-    S rhs[10];
+    // residual of this lane's variables j = q, q + 4, q + 8 in face order 1..4
+    // (src/sr_hllcbatten.F90:534-552): a wall face adds its pressure terms, a
+    // face that took no wave branch (NaN states) the flux of the face before
+    S rhs[3];
+    {
+        int fl[4];
 #pragma unroll
-    for (int k = 0; k < 10; k++) rhs[k] = S(0.0);
-    R Fg[5] = {R(0), R(0), R(0), R(0), R(0)}, Fp[5] = {R(0), R(0), R(0), R(0), R(0)};
+        for (int f = 0; f < 4; f++) fl[f] = qshfl(flags, f);
 #pragma unroll
-    for (int f = 0; f < 4; f++) {
-        R e[10];
+        for (int r = 0; r < 3; r++) {
+            const int j = q + 4 * r;
+            rhs[r] = S(0.0);
+            // (no variables 10 and 11: lanes 2 and 3 repeat column 9 and drop
+            // it, so the warp stays together up to the shuffles below)
+            const R* e = sres + (j < 10 ? j : 9) * FLUX4_T + (tid & ~3);
+            const int take = j < 5 ? 2 : 4;
+            R cur = R(0);
 #pragma unroll
-        for (int k = 0; k < 10; k++) e[k] = qshfl(eff[k], f);
-        const int fl = qshfl(flags, f);
-        if (fl & 1) {
-            rhs[1] = rhs[1] + (S)e[1]; rhs[2] = rhs[2] + (S)e[2]; rhs[3] = rhs[3] + (S)e[3];
-            rhs[6] = rhs[6] + (S)e[6]; rhs[7] = rhs[7] + (S)e[7]; rhs[8] = rhs[8] + (S)e[8];
-        } else {
-            if (fl & 2) {
-#pragma unroll
-                for (int k = 0; k < 5; k++) Fg[k] = e[k];
-            }
-            if (fl & 4) {
-#pragma unroll
-                for (int k = 0; k < 5; k++) Fp[k] = e[5 + k];
-            }
-#pragma unroll
-            for (int k = 0; k < 5; k++) {
-                rhs[k] = rhs[k] + (S)Fg[k];
-                rhs[5 + k] = rhs[5 + k] + (S)Fp[k];
+            for (int f = 0; f < 4; f++) {
+                const R v = e[f];
+                if (fl[f] & take) cur = v;
+                rhs[r] = rhs[r] + (S)((fl[f] & 1) ? v : cur);
             }
         }
     }
@@ -2405,22 +2406,28 @@ __device__ __forceinline__ bool flux4_body(const DevMesh& m, const DevState<R>& 
 #define DW(x, f) div_rn((x), wt[f], rw[f])
         const R g = R(0);
         R en = pint * (uint_ * dpx + vint * dpy + wint * dpz) + uint_ * fdgx + vint * fdgy + wint * fdgz + qsource;
+        // the lane's variables: j = q gas momentum (q > 0), j = q + 4 gas energy
+        // (q = 0) and liquid momentum x, y (q = 2, 3), j = q + 8 liquid
+        // momentum z (q = 0) and liquid energy (q = 1)
         const double* vis = s.vis;
-        rhs[1] = rhs[1] - (S)((fdgx + pint * dpx + phig * rog * g) * voli) - TLS(TAIL_VIS + 0, COL(vis, 0)[i]);
-        rhs[2] = rhs[2] - (S)((fdgy + pint * dpy) * voli) - TLS(TAIL_VIS + 1, COL(vis, 1)[i]);
-        rhs[3] = rhs[3] - (S)((fdgz + pint * dpz) * voli) - TLS(TAIL_VIS + 2, COL(vis, 2)[i]);
-        rhs[4] = rhs[4] - (S)(en * voli) - TLS(TAIL_VIS + 3, COL(vis, 3)[i]);
-        rhs[6] = rhs[6] + (S)((fdgx + pint * dpx - phip * rop * g) * voli) - TLS(TAIL_VIS + 4, COL(vis, 4)[i]);
-        rhs[7] = rhs[7] + (S)((fdgy + pint * dpy) * voli) - TLS(TAIL_VIS + 5, COL(vis, 5)[i]);
-        rhs[8] = rhs[8] + (S)((fdgz + pint * dpz) * voli) - TLS(TAIL_VIS + 6, COL(vis, 6)[i]);
-        rhs[9] = rhs[9] + (S)(en * voli) - TLS(TAIL_VIS + 7, COL(vis, 7)[i]);
+        const R fq = q == 1 ? fdgx : (q == 2 ? fdgy : fdgz), pq3 = q == 1 ? dpx : (q == 2 ? dpy : dpz);
+        if (q > 0)
+            rhs[0] = rhs[0] - (S)((fq + pint * pq3 + phig * rog * g) * voli) - TLS(TAIL_VIS + q - 1, COL(vis, q - 1)[i]);
+        const R fl_ = q == 2 ? fdgx : (q == 3 ? fdgy : fdgz), pl_ = q == 2 ? dpx : (q == 3 ? dpy : dpz);
+        const R lm = fl_ + pint * pl_ - phip * rop * g;
+        const int v1 = q == 0 ? 3 : q + 2;
+        if (q != 1) rhs[1] = rhs[1] + (S)((q == 0 ? -en : lm) * voli) - TLS(TAIL_VIS + v1, COL(vis, v1)[i]);
+        if (q < 2) rhs[2] = rhs[2] + (S)((q == 0 ? lm : en) * voli) - TLS(TAIL_VIS + 6 + q, COL(vis, 6 + q)[i]);
     }
-    // five-phase: drag of q, r, s on the liquid (see k_flux)
-    if (P.five_phase) {
+    // five-phase: drag of q, r, s on the liquid momenta (see k_flux)
+    if (P.five_phase && (q == 0 || q > 1)) {
+        const int c = q == 0 ? 2 : q - 2;
 #pragma unroll
-        for (int d = 0; d < 3; d++)
-#pragma unroll
-            for (int c = 0; c < 3; c++) rhs[6 + c] = rhs[6 + c] + (S)COL(s.qdrag, 3 * d + c)[i];
+        for (int d = 0; d < 3; d++) {
+            const S x = (S)COL(s.qdrag, 3 * d + c)[i];
+            if (q == 0) rhs[2] = rhs[2] + x;
+            else rhs[1] = rhs[1] + x;
+        }
     }
     // only lanes that store count: a lane past the last cell has read
     // whatever follows the mesh in the columns (zero LSQ weights), and its
@@ -2436,7 +2443,7 @@ __device__ __forceinline__ bool flux4_body(const DevMesh& m, const DevState<R>& 
     for (int r = 0; r < 3; r++) {
         const int j = q + 4 * r;
         if (j >= 10) break;
-        const S rr = rhs[j] - TLS(TAIL_D24 + j, COL(s.d24, j)[i]);
+        const S rr = rhs[r] - TLS(TAIL_D24 + j, COL(s.d24, j)[i]);
         const S cu = TLS(TAIL_CU + j, COL(s.cu, j)[i]);
         double* cnp = COL(s.cn, j) + i;
         if (P.rk_scheme == 0) {
@@ -2478,6 +2485,7 @@ __device__ __forceinline__ void k_flux4_body(DevMesh m, DevState<R> s, DevParams
     const int i = LIST ? ldg(m.wcells + k) : k;
     bool active = valid && ldg(m.iblank + i) == 1;
     if (sizeof(R) != sizeof(double) && m.nwall > 0) active = active && !ldg(m.wclass + i);
+    __shared__ __align__(16) R sres[10 * FLUX4_T];
 #if HP_FLUX4_PREFETCH && HP_LSQ_TABLE && HP_DXN_TABLE
     if constexpr (NC && sizeof(R) == sizeof(double)) {
         // start the asynchronous copy of the values that the sources and the
@@ -2499,19 +2507,20 @@ __device__ __forceinline__ void k_flux4_body(DevMesh m, DevState<R> s, DevParams
         cp_async_commit();
         const double* pf = stail + ((threadIdx.x >> 2) & (TAIL_LD - 1));
         if constexpr (HP_FAST(2)) {
-            if (!flux4_body<1, Z, NC, true>(m, s, P, stage, i, q, active, pf))
-                flux4_body<0, Z, NC, true>(m, s, P, stage, i, q, active, pf);
+            if (!flux4_body<1, Z, NC, true>(m, s, P, stage, i, q, active, sres, pf))
+                flux4_body<0, Z, NC, true>(m, s, P, stage, i, q, active, sres, pf);
         } else {
-            flux4_body<0, Z, NC, true>(m, s, P, stage, i, q, active, pf);
+            flux4_body<0, Z, NC, true>(m, s, P, stage, i, q, active, sres, pf);
         }
         return;
     }
 #endif
     if constexpr (HP_FAST(2)) {
-        if (!flux4_body<1, Z, NC>(m, s, P, stage, i, q, active)) flux4_body<0, Z, NC>(m, s, P, stage, i, q, active);
+        if (!flux4_body<1, Z, NC>(m, s, P, stage, i, q, active, sres)) flux4_body<0, Z, NC>(m, s, P, stage, i, q, active, sres);
     } else {
-        flux4_body<0, Z, NC>(m, s, P, stage, i, q, active);
+        flux4_body<0, Z, NC>(m, s, P, stage, i, q, active, sres);
     }
+    __syncwarp();   // the fused step reuses sres for its next virtual block
 }
 template <int Z, int LIST>
 __global__ void __launch_bounds__(128, HP_FLUX4_MINB) k_flux4(DevMesh m, DevState<R> s, DevParams P, int stage) {
