@@ -2752,13 +2752,26 @@ __device__ __forceinline__ void visc_face_ph(const DevMesh& m, const DevState<R>
         }
     }
     const R dnr = det3(a11, a12, a13, a12, a22, a23, a13, a23, a33);
-    const R rdnr = mrcp<F>(dnr, bad);
+    // the twelve quotients share the determinant: its reciprocal is taken once
+    // (mquo), and a lane whose operands leave that form's range divides the
+    // three numerators at hand, so no second body is needed (983,040 cells,
+    // FP64: 584 -> 557 us; the sums of the normal matrix from a set-up table
+    // on top of that: 570 us, the kernel waits on its gathers)
+    unsigned out = 0;
+    const R rdnr = mrcpp<1>(dnr, out);
     R gr[4][3];
 #pragma unroll
     for (int v = 0; v < 4; v++) {
-        gr[v][0] = mdiv<F>(det3(b[v][0], b[v][1], b[v][2], a12, a22, a23, a13, a23, a33), dnr, rdnr, bad);
-        gr[v][1] = mdiv<F>(det3(a11, a12, a13, b[v][0], b[v][1], b[v][2], a13, a23, a33), dnr, rdnr, bad);
-        gr[v][2] = mdiv<F>(det3(a11, a12, a13, a12, a22, a23, b[v][0], b[v][1], b[v][2]), dnr, rdnr, bad);
+        const R d0 = det3(b[v][0], b[v][1], b[v][2], a12, a22, a23, a13, a23, a33);
+        const R d1 = det3(a11, a12, a13, b[v][0], b[v][1], b[v][2], a13, a23, a33);
+        const R d2 = det3(a11, a12, a13, a12, a22, a23, b[v][0], b[v][1], b[v][2]);
+        unsigned o = out;
+        mout<1>(d0, o); mout<1>(d1, o); mout<1>(d2, o);
+        if (sizeof(R) == 8 && o) {
+            gr[v][0] = d0 / dnr; gr[v][1] = d1 / dnr; gr[v][2] = d2 / dnr;
+        } else {
+            gr[v][0] = mquo<1>(d0, dnr, rdnr); gr[v][1] = mquo<1>(d1, dnr, rdnr); gr[v][2] = mquo<1>(d2, dnr, rdnr);
+        }
     }
     const R uf = ff[0], vf = ff[1], wf = ff[2];
     R delv = gr[0][0] + gr[1][1] + gr[2][2];
