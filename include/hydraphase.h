@@ -344,7 +344,7 @@ int hp_poll(hp_handle *h, int32_t *busy);
  * dt_dev[0].  Device pointers; the work is queued on `stream` (a
  * cudaStream_t, NULL for the default stream) and the call returns without
  * waiting.  The call allocates nothing: its only scratch, one partial minimum
- * per 256 cells, is a static device array sized for HP_NOALLOC_MAX_CELLS
+ * per 256 cells and 1024 block counters, is a static device array sized for HP_NOALLOC_MAX_CELLS
  * cells that each GPU using the library keeps until exit; larger ncells is
  * rejected with HP_E_ARG.  All calls share that array, so calls that overlap
  * on the GPU race.  The first call on each device looks up the array's device
