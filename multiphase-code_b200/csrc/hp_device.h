@@ -164,7 +164,7 @@ struct DevState {
     double* pr;              // [14][ld]
     R* prr;                  // [14][ld] primitives in R: pr itself when R is
                              // double, a float copy otherwise
-    R* gr;                   // [33][ld]
+    R* gr;                   // [ld / 32][33][32], see GRD in hp_kernels.cuh
     double* phi;             // [ld]
     R* agrad;                // [3][ld] 1/r-weighted gradient of alpha_g (the
                              // sources'), formed beside the others by the
@@ -184,7 +184,7 @@ struct DevState {
     DevScalars* s;
     double* diag;            // [max_steps][8]
     int max_diag;
-    double* gr64;            // [33][ld] FP64 gradients of the wall layers
+    double* gr64;            // as gr: FP64 gradients of the wall layers
                              // (FP32 variants with nwall > 0; else null)
 };
 
