@@ -21,6 +21,17 @@ enum { NEQ = 10, NPR = 14, NGR = 33, NLSQ = 16 };
 // tp,rog,rop of src/mod_GlobalVariables.F90:13)
 enum { P_UG = 0, P_VG, P_WG, P_TG, P_PG, P_PP, P_PHIG, P_PHIP, P_UP, P_VP,
        P_WP, P_TP, P_ROG, P_ROP };
+// Primitives are stored in tiles of 32 cells, a tile's 14 columns together:
+// column k of cell c stands at pr[PR_TILE * k + prim_off(c)].  Consecutive
+// cells share sectors as in plain columns, and the columns of a cell lie at
+// fixed distances from one address.
+enum { PR_TILE = 32 };
+#if defined(__CUDACC__)
+__host__ __device__
+#endif
+inline size_t prim_off(int c) {
+    return (size_t)((unsigned)c / PR_TILE) * (NPR * PR_TILE) + ((unsigned)c % PR_TILE);
+}
 // stored gradient columns (x,y,z per field), src/sr_derivative.F90:259-309
 enum { G_UG = 0, G_VG = 3, G_WG = 6, G_TG = 9, G_UP = 12, G_VP = 15,
        G_WP = 18, G_TP = 21, G_PG = 24, G_PP = 27, G_PHIG = 30 };
@@ -161,8 +172,8 @@ constexpr int FACE_REC = 12;
 template <class R>
 struct DevState {
     double *cn, *cu, *cn1;   // [10][ld]
-    double* pr;              // [14][ld]
-    R* prr;                  // [14][ld] primitives in R: pr itself when R is
+    double* pr;              // [ld / 32][14][32], see prim_off
+    R* prr;                  // as pr: primitives in R: pr itself when R is
                              // double, a float copy otherwise
     R* gr;                   // [ld / 32][33][32], see GRD in hp_kernels.cuh
     double* phi;             // [ld]

@@ -1095,27 +1095,42 @@ __global__ void k_gather_cols(const double* __restrict__ src, long long ld, int 
 // the ghost list in order, so repeated ghost ids keep the last value, as the
 // reference's sequential restart read does (src/main.F90:433-438).
 __global__ void k_scatter_ghost_prims(const double* __restrict__ src, int ng, Cols6 cols, const int* __restrict__ gid,
-                                      double* __restrict__ pr, long long ld, int ordered) {
+                                      double* __restrict__ pr, int ordered) {
     if (ordered) {
         int v = threadIdx.x;
         if (blockIdx.x != 0 || v >= 6) return;
-        for (int g = 0; g < ng; g++) pr[(size_t)cols.c[v] * ld + gid[g]] = src[(size_t)v * ng + g];
+        for (int g = 0; g < ng; g++) pr[cols.c[v] * PR_TILE + prim_off(gid[g])] = src[(size_t)v * ng + g];
         return;
     }
     long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= 6LL * ng) return;
     int v = (int)(t / ng), g = (int)(t - (long long)v * ng);
-    pr[(size_t)cols.c[v] * ld + gid[g]] = src[(size_t)v * ng + g];
+    pr[cols.c[v] * PR_TILE + prim_off(gid[g])] = src[(size_t)v * ng + g];
 }
-__global__ void k_gather_ghost_prims(const double* __restrict__ pr, long long ld, Cols6 cols, int ng,
+__global__ void k_gather_ghost_prims(const double* __restrict__ pr, Cols6 cols, int ng,
                                      const int* __restrict__ gid, double* __restrict__ dst) {
     long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= 6LL * ng) return;
     int v = (int)(t / ng), g = (int)(t - (long long)v * ng);
-    dst[(size_t)v * ng + g] = pr[(size_t)cols.c[v] * ld + gid[g]];
+    dst[(size_t)v * ng + g] = pr[cols.c[v] * PR_TILE + prim_off(gid[g])];
 }
 // p[k*ld + start + i] = v and dst[k*ld + start + i] = src[k*ld + start + i],
 // k < ncol, i < count (one case's element or ghost range)
+// primitives of cells [start, start + count) set to zero
+__global__ void k_zero_prims(double* pr, int start, int count) {
+    long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= (long long)count * NPR) return;
+    const int k = (int)(t / count), i = (int)(t - (long long)k * count);
+    pr[k * PR_TILE + prim_off(start + i)] = 0.0;
+}
+// primitive columns [col0, col0 + ncol) of n cells into plain columns
+__global__ void k_gather_prims(const double* __restrict__ pr, int col0, int n, int ncol, const int* __restrict__ idx,
+                               double* __restrict__ dst) {
+    long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= (long long)n * ncol) return;
+    const int k = (int)(t / n), i = (int)(t - (long long)k * n);
+    dst[(size_t)k * n + i] = pr[(col0 + k) * PR_TILE + prim_off(idx[i])];
+}
 __global__ void k_fill_cols(double* __restrict__ p, long long ld, int ncol, int start, int count, double v) {
     long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= (long long)count * ncol) return;
@@ -1149,17 +1164,17 @@ static int upload_state(hp_handle* h, int c, double time, const double* cu_elem,
     k_copy_cols<<<blocks_for((long long)nq * ne, 256), 256, 0, st>>>(h->ds.cn, h->ds.cu, ld, nq, cr.e0, ne);
     if (ng) k_copy_cols<<<blocks_for((long long)nq * ng, 256), 256, 0, st>>>(h->ds.cn, h->ds.cu, ld, nq, gs, ng);
     // primitives: zero, then the restart's ghost values (src/main.F90:433-438)
-    k_fill_cols<<<blocks_for((long long)NPR * ne, 256), 256, 0, st>>>(h->ds.pr, ld, NPR, cr.e0, ne, 0.0);
-    if (ng) k_fill_cols<<<blocks_for((long long)NPR * ng, 256), 256, 0, st>>>(h->ds.pr, ld, NPR, gs, ng, 0.0);
+    k_zero_prims<<<blocks_for((long long)NPR * ne, 256), 256, 0, st>>>(h->ds.pr, cr.e0, ne);
+    if (ng) k_zero_prims<<<blocks_for((long long)NPR * ng, 256), 256, 0, st>>>(h->ds.pr, gs, ng);
     CUDA_OK(h, cudaGetLastError());
     if (ghost_prims && ng) {
         CUDA_OK(h, cudaMemcpyAsync(h->d_gstage, ghost_prims, 6 * (size_t)ng * sizeof(double),
                                    cudaMemcpyHostToDevice, st));
         if (h->aliased)
-            k_scatter_ghost_prims<<<1, 32, 0, st>>>(h->d_gstage, ng, GHOST_COLS, h->d_gid + cr.g0, h->ds.pr, ld, 1);
+            k_scatter_ghost_prims<<<1, 32, 0, st>>>(h->d_gstage, ng, GHOST_COLS, h->d_gid + cr.g0, h->ds.pr, 1);
         else
             k_scatter_ghost_prims<<<blocks_for(6LL * ng, 256), 256, 0, st>>>(h->d_gstage, ng, GHOST_COLS,
-                                                                             h->d_gid + cr.g0, h->ds.pr, ld, 0);
+                                                                             h->d_gid + cr.g0, h->ds.pr, 0);
         CUDA_OK(h, cudaGetLastError());
     }
     DevScalars s0{};
@@ -1649,7 +1664,7 @@ extern "C" int hp_get_state_case(hp_handle* h, int32_t c, double* time, double* 
         CUDA_OK(h, cudaMemcpyAsync(cu_elem, h->ds.cn1, nq * (size_t)ne * sizeof(double), cudaMemcpyDeviceToHost, st));
     }
     if (ghost_prims && ng) {
-        k_gather_ghost_prims<<<blocks_for(6LL * ng, 256), 256, 0, st>>>(h->ds.pr, ld, GHOST_COLS, ng,
+        k_gather_ghost_prims<<<blocks_for(6LL * ng, 256), 256, 0, st>>>(h->ds.pr, GHOST_COLS, ng,
                                                                         h->d_gid + cr.g0, h->d_gstage);
         CUDA_OK(h, cudaGetLastError());
         CUDA_OK(h, cudaMemcpyAsync(ghost_prims, h->d_gstage, 6 * (size_t)ng * sizeof(double),
@@ -1707,7 +1722,7 @@ extern "C" int hp_output_async(hp_handle* h, int32_t c, const hp_mesh* mesh, con
     k_gather_cols<<<blocks_for(10LL * ne, 256), 256, 0, st>>>(h->ds.cu, ld, 0, ne, 10, h->d_perm + cr.e0, d + 1);
     CUDA_OK(h, cudaGetLastError());
     if (ng) {
-        k_gather_ghost_prims<<<blocks_for(6LL * ng, 256), 256, 0, st>>>(h->ds.pr, ld, GHOST_COLS, ng,
+        k_gather_ghost_prims<<<blocks_for(6LL * ng, 256), 256, 0, st>>>(h->ds.pr, GHOST_COLS, ng,
                                                                         h->d_gid + cr.g0, d + 1 + 10 * (size_t)ne);
         CUDA_OK(h, cudaGetLastError());
     }
@@ -1743,14 +1758,13 @@ extern "C" int hp_output_wait(hp_handle* h, int32_t ticket) {
 
 extern "C" int hp_get_prims(hp_handle* h, double* prims) {
     if (!h || !prims) return HP_E_ARG;
-    const long long ld = h->ld;
     const int ne = h->cases[0].ne;   // case 0 (the only one of a single-case handle)
     cudaStream_t st = h->stream;
     // cn1 stages at most 10 columns at a time
     for (int c0 = 0; c0 < NPR; c0 += 10) {
         const int nc = NPR - c0 < 10 ? NPR - c0 : 10;
-        k_gather_cols<<<blocks_for((long long)nc * ne, 256), 256, 0, st>>>(h->ds.pr, ld, c0, ne, nc, h->d_perm + h->cases[0].e0,
-                                                                          h->ds.cn1);
+        k_gather_prims<<<blocks_for((long long)nc * ne, 256), 256, 0, st>>>(h->ds.pr, c0, ne, nc,
+                                                                            h->d_perm + h->cases[0].e0, h->ds.cn1);
         CUDA_OK(h, cudaGetLastError());
         CUDA_OK(h, cudaMemcpyAsync(prims + (size_t)c0 * ne, h->ds.cn1, (size_t)nc * ne * sizeof(double),
                                    cudaMemcpyDeviceToHost, st));

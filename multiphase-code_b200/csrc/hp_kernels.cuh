@@ -240,6 +240,11 @@ __device__ __forceinline__ T qshfl(T v, int q) {
 }
 
 #define COL(ptr, k) ((ptr) + (size_t)(k) * (size_t)m.ld)
+// Primitive column k, indexed by prim_off(c).  983,040 cells against plain
+// columns: FP32 viscous terms 218 -> 180 us, FP32 gradients 326 -> 314 us
+// (three launches), FP64 viscous terms 560 -> 551 us, k_flux4 2007 -> 1998 us.
+#define PCOL(ptr, k) ((ptr) + (k) * PR_TILE)
+#define po(c) prim_off(c)
 // Gradient column k of cell c: tiles of 32 cells, a tile's 33 columns
 // together.  Neighbouring cells still share sectors, as in plain columns, but
 // the columns of a cell lie at fixed distances from one address (a face reads
@@ -372,11 +377,11 @@ __device__ __forceinline__ void prim_full(double cd[10], PrimV& q, const DevPara
 
 template <class T>
 __device__ __forceinline__ void store_prims(const DevMesh& m, T* pr, int i, const PrimV& q) {
-    COL(pr, P_UG)[i] = (T)q.ug; COL(pr, P_VG)[i] = (T)q.vg; COL(pr, P_WG)[i] = (T)q.wg;
-    COL(pr, P_TG)[i] = (T)q.tg; COL(pr, P_PG)[i] = (T)q.pg; COL(pr, P_PP)[i] = (T)q.pp;
-    COL(pr, P_PHIG)[i] = (T)q.phig; COL(pr, P_PHIP)[i] = (T)q.phip;
-    COL(pr, P_UP)[i] = (T)q.up; COL(pr, P_VP)[i] = (T)q.vp; COL(pr, P_WP)[i] = (T)q.wp;
-    COL(pr, P_TP)[i] = (T)q.tp; COL(pr, P_ROG)[i] = (T)q.rog; COL(pr, P_ROP)[i] = (T)q.rop;
+    PCOL(pr, P_UG)[po(i)] = (T)q.ug; PCOL(pr, P_VG)[po(i)] = (T)q.vg; PCOL(pr, P_WG)[po(i)] = (T)q.wg;
+    PCOL(pr, P_TG)[po(i)] = (T)q.tg; PCOL(pr, P_PG)[po(i)] = (T)q.pg; PCOL(pr, P_PP)[po(i)] = (T)q.pp;
+    PCOL(pr, P_PHIG)[po(i)] = (T)q.phig; PCOL(pr, P_PHIP)[po(i)] = (T)q.phip;
+    PCOL(pr, P_UP)[po(i)] = (T)q.up; PCOL(pr, P_VP)[po(i)] = (T)q.vp; PCOL(pr, P_WP)[po(i)] = (T)q.wp;
+    PCOL(pr, P_TP)[po(i)] = (T)q.tp; PCOL(pr, P_ROG)[po(i)] = (T)q.rog; PCOL(pr, P_ROP)[po(i)] = (T)q.rop;
 }
 
 // Block-wide min / max of 64-bit keys, then one atomic per block.
@@ -559,8 +564,11 @@ __device__ __forceinline__ void step_end_case(const DevState<R>& s, int c) {
 // residuals are complete then), in place of a launch of its own, whose
 // fixed cost a small mesh pays on every step.  The counter of finished blocks
 // is case 0's, and that block leaves it at zero.
+// (768 caps the registers at 80, three blocks of 256 threads per SM; at 82
+// two fit and the closing pass takes 116 instead of 93 us for 983,040 cells.
+// Blocks have at most 512 threads.)
 template <int MODE>
-__global__ void __launch_bounds__(512) k_prim(DevMesh m, DevState<R> s, DevParams P) {
+__global__ void __launch_bounds__(768) k_prim(DevMesh m, DevState<R> s, DevParams P) {
     k_prim_body<MODE>(m, s, P, blockIdx.x);
     if constexpr (MODE == PM_NEXT) {
         __shared__ int last;
@@ -685,12 +693,12 @@ __device__ __forceinline__ void bc_one(const DevMesh& m, double* pr, double* egt
     double c[NPR];
 #pragma unroll
     for (int k = 0; k < NPR; k++) {
-        c[k] = COL(pr, k)[np];
-        g[k] = COL(pr, k)[ng];
+        c[k] = PCOL(pr, k)[po(np)];
+        g[k] = PCOL(pr, k)[po(ng)];
     }
     if (!ghost_prims<VISC>(P, nt, c, g, m.dd[np], dt, total)) return;
 #pragma unroll
-    for (int k = 0; k < NPR; k++) COL(pr, k)[ng] = g[k];
+    for (int k = 0; k < NPR; k++) PCOL(pr, k)[po(ng)] = g[k];
     if (!VISC && egt != nullptr) {
         const double gamag = P.gamag, gamap = P.gamap, pinf = P.pinf;
         double eg, ep;
@@ -711,10 +719,10 @@ __device__ __forceinline__ void bc_one(const DevMesh& m, double* pr, double* egt
 __device__ __forceinline__ void ghost_cn_one(const DevMesh& m, double* pr, double* cn,
                                              const double* egtp, int gidx) {
     const int ng = m.g_id[gidx];
-    double ug = COL(pr, P_UG)[ng], vg = COL(pr, P_VG)[ng], wg = COL(pr, P_WG)[ng];
-    double up = COL(pr, P_UP)[ng], vp = COL(pr, P_VP)[ng], wp = COL(pr, P_WP)[ng];
-    double phig = COL(pr, P_PHIG)[ng], phip = COL(pr, P_PHIP)[ng];
-    double rog = COL(pr, P_ROG)[ng], rop = COL(pr, P_ROP)[ng];
+    double ug = PCOL(pr, P_UG)[po(ng)], vg = PCOL(pr, P_VG)[po(ng)], wg = PCOL(pr, P_WG)[po(ng)];
+    double up = PCOL(pr, P_UP)[po(ng)], vp = PCOL(pr, P_VP)[po(ng)], wp = PCOL(pr, P_WP)[po(ng)];
+    double phig = PCOL(pr, P_PHIG)[po(ng)], phip = PCOL(pr, P_PHIP)[po(ng)];
+    double rog = PCOL(pr, P_ROG)[po(ng)], rop = PCOL(pr, P_ROP)[po(ng)];
     double egt = egtp[ng], ept = egtp[m.ld + ng];
     COL(cn, 0)[ng] = phig * rog; COL(cn, 1)[ng] = phig * rog * ug;
     COL(cn, 2)[ng] = phig * rog * vg; COL(cn, 3)[ng] = phig * rog * wg;
@@ -735,7 +743,7 @@ __device__ __forceinline__ void k_bc_body(DevMesh m, DevState<R> s, DevParams P,
     if constexpr (sizeof(R) != sizeof(double)) {
         const int ng = m.g_id[g];
 #pragma unroll
-        for (int k = 0; k < NPR; k++) COL(s.prr, k)[ng] = (R)v[k];
+        for (int k = 0; k < NPR; k++) PCOL(s.prr, k)[po(ng)] = (R)v[k];
     }
 }
 template <bool VISC>
@@ -765,8 +773,8 @@ __global__ void k_smooth_copy_serial(DevMesh m, DevState<R> s, int which) {
     for (int g = 0; g < m.nghosts; g++) {
         int ng = m.g_id[g], np = m.g_par[g];
         if (which == 0) {
-            COL(s.pr, P_PG)[ng] = COL(s.pr, P_PG)[np];
-            COL(s.pr, P_PP)[ng] = COL(s.pr, P_PP)[np];
+            PCOL(s.pr, P_PG)[po(ng)] = PCOL(s.pr, P_PG)[po(np)];
+            PCOL(s.pr, P_PP)[po(ng)] = PCOL(s.pr, P_PP)[po(np)];
             for (int k = 0; k < 10; k++) COL(s.cn, k)[ng] = COL(s.cn, k)[np];
         } else {
             for (int k = 0; k < 10; k++) COL(s.d2q, k)[ng] = COL(s.d2q, k)[np];
@@ -804,7 +812,7 @@ enum { JST_CELLS = 64 };
 __device__ __forceinline__ void smooth1_set(const DevMesh& m, const DevState<R>& s, int i, int set) {
     const int a = ldg(COL(m.snb, 0) + i), b = ldg(COL(m.snb, 1) + i);
     const int c = ldg(COL(m.snb, 2) + i), d = ldg(COL(m.snb, 3) + i);
-    const double* pq = COL(s.pr, set == 0 ? P_PG : P_PP);
+    const double* pq = PCOL(s.pr, set == 0 ? P_PG : P_PP);
     const S e6 = (S)(double)1.0e-6f;
     // switch sums of the set's first and last variable (1 and 5, or 6 and
     // 10) and the Laplacian of its five variables
@@ -819,7 +827,7 @@ __device__ __forceinline__ void smooth1_set(const DevMesh& m, const DevState<R>&
         }
         lap[k] = v1 - v0 + v2 - v0 + v3 - v0 + v4 - v0;
     }
-    const S qi = (S)pq[i], qa = (S)pq[a], qb = (S)pq[b], qc = (S)pq[c], qd = (S)pq[d];
+    const S qi = (S)pq[po(i)], qa = (S)pq[po(a)], qb = (S)pq[po(b)], qc = (S)pq[po(c)], qd = (S)pq[po(d)];
     const S anun = fabs(qa - qi) + fabs(qb - qi) + fabs(qc - qi) + fabs(qd - qi);
     const S anud = fabs(qa + qi) + fabs(qb + qi) + fabs(qc + qi) + fabs(qd + qi);
     S anu;
@@ -1045,10 +1053,10 @@ __device__ __forceinline__ void k_grad_body(DevMesh m, DevState<R> s, DevParams 
             // the FP32 copies differ by whole ulps (6e-8), as much as a trace
             // alpha_p = 1 - alpha_g itself, whose reconstruction uses this
             // gradient
-            const double* q = COL(s.pr, P_PHIG);
-            const double qi = ldg(q + i);
-            qa = (R)(ldg(q + n[0]) - qi); qb = (R)(ldg(q + n[1]) - qi);
-            qc = (R)(ldg(q + n[2]) - qi); qd = (R)(ldg(q + n[3]) - qi);
+            const double* q = PCOL(s.pr, P_PHIG);
+            const double qi = ldg(q + po(i));
+            qa = (R)(ldg(q + po(n[0])) - qi); qb = (R)(ldg(q + po(n[1])) - qi);
+            qc = (R)(ldg(q + po(n[2])) - qi); qd = (R)(ldg(q + po(n[3])) - qi);
 #if !HP_LSQ_TABLE
             // the sources need the same differences: their gradient is formed
             // here too, and the flux kernel gathers nothing but face records
@@ -1062,10 +1070,10 @@ __device__ __forceinline__ void k_grad_body(DevMesh m, DevState<R> s, DevParams 
             }
 #endif
         } else {
-            const PT* q = COL(prb, pcol[v]);
-            PT qi = ldg(q + i);
-            qa = (R)(ldg(q + n[0]) - qi); qb = (R)(ldg(q + n[1]) - qi);
-            qc = (R)(ldg(q + n[2]) - qi); qd = (R)(ldg(q + n[3]) - qi);
+            const PT* q = PCOL(prb, pcol[v]);
+            PT qi = ldg(q + po(i));
+            qa = (R)(ldg(q + po(n[0])) - qi); qb = (R)(ldg(q + po(n[1])) - qi);
+            qc = (R)(ldg(q + po(n[2])) - qi); qd = (R)(ldg(q + po(n[3])) - qi);
         }
         R c1 = DW(qa * xa[0], 0) + DW(qb * xa[1], 1) + DW(qc * xa[2], 2) + DW(qd * xa[3], 3);
         R c2;
@@ -1104,8 +1112,9 @@ __device__ __forceinline__ void k_grad_body(DevMesh m, DevState<R> s, DevParams 
     R phi = R(0);
 #pragma unroll
     for (int t = 0; t < 4; t++) {
-        const PT* q = COL(prb, pcol[lv[t]]);
-        PT qi = ldg(q + i), q0 = ldg(q + n[0]), q1 = ldg(q + n[1]), q2 = ldg(q + n[2]), q3 = ldg(q + n[3]);
+        const PT* q = PCOL(prb, pcol[lv[t]]);
+        PT qi = ldg(q + po(i)), q0 = ldg(q + po(n[0])), q1 = ldg(q + po(n[1])), q2 = ldg(q + po(n[2])),
+           q3 = ldg(q + po(n[3]));
         PT vmax = mx2(mx2(mx2(mx2(qi, q0), q1), q2), q3);
         PT vmin = mn2(mn2(mn2(mn2(qi, q0), q1), q2), q3);
         R dmax = (R)(vmax - qi), dmin = (R)(vmin - qi);
@@ -1324,14 +1333,14 @@ __device__ __forceinline__ void face_eval(const DevMesh& m, const DevState<R>& s
         eny = mdiv<F>(scy, area, rarea, bad);
         enz = mdiv<F>(scz, area, rarea, bad);
     }
-    R ugL = (R)PLD(COL(pr, P_UG) + i), vgL = (R)PLD(COL(pr, P_VG) + i), wgL = (R)PLD(COL(pr, P_WG) + i);
-    R tgL = (R)PLD(COL(pr, P_TG) + i), phigL = (R)PLD(COL(pr, P_PHIG) + i);
-    R upL = (R)PLD(COL(pr, P_UP) + i), vpL = (R)PLD(COL(pr, P_VP) + i), wpL = (R)PLD(COL(pr, P_WP) + i);
-    R tpL = (R)PLD(COL(pr, P_TP) + i), pgL = (R)PLD(COL(pr, P_PG) + i), ppL = (R)PLD(COL(pr, P_PP) + i);
-    R ugR = (R)PLD(COL(pr, P_UG) + neigh), vgR = (R)PLD(COL(pr, P_VG) + neigh), wgR = (R)PLD(COL(pr, P_WG) + neigh);
-    R tgR = (R)PLD(COL(pr, P_TG) + neigh), phigR = (R)PLD(COL(pr, P_PHIG) + neigh);
-    R upR = (R)PLD(COL(pr, P_UP) + neigh), vpR = (R)PLD(COL(pr, P_VP) + neigh), wpR = (R)PLD(COL(pr, P_WP) + neigh);
-    R tpR = (R)PLD(COL(pr, P_TP) + neigh), pgR = (R)PLD(COL(pr, P_PG) + neigh), ppR = (R)PLD(COL(pr, P_PP) + neigh);
+    R ugL = (R)PLD(PCOL(pr, P_UG) + po(i)), vgL = (R)PLD(PCOL(pr, P_VG) + po(i)), wgL = (R)PLD(PCOL(pr, P_WG) + po(i));
+    R tgL = (R)PLD(PCOL(pr, P_TG) + po(i)), phigL = (R)PLD(PCOL(pr, P_PHIG) + po(i));
+    R upL = (R)PLD(PCOL(pr, P_UP) + po(i)), vpL = (R)PLD(PCOL(pr, P_VP) + po(i)), wpL = (R)PLD(PCOL(pr, P_WP) + po(i));
+    R tpL = (R)PLD(PCOL(pr, P_TP) + po(i)), pgL = (R)PLD(PCOL(pr, P_PG) + po(i)), ppL = (R)PLD(PCOL(pr, P_PP) + po(i));
+    R ugR = (R)PLD(PCOL(pr, P_UG) + po(neigh)), vgR = (R)PLD(PCOL(pr, P_VG) + po(neigh)), wgR = (R)PLD(PCOL(pr, P_WG) + po(neigh));
+    R tgR = (R)PLD(PCOL(pr, P_TG) + po(neigh)), phigR = (R)PLD(PCOL(pr, P_PHIG) + po(neigh));
+    R upR = (R)PLD(PCOL(pr, P_UP) + po(neigh)), vpR = (R)PLD(PCOL(pr, P_VP) + po(neigh)), wpR = (R)PLD(PCOL(pr, P_WP) + po(neigh));
+    R tpR = (R)PLD(PCOL(pr, P_TP) + po(neigh)), pgR = (R)PLD(PCOL(pr, P_PG) + po(neigh)), ppR = (R)PLD(PCOL(pr, P_PP) + po(neigh));
     // alpha_p.  The reference forms it as 1 - alpha_g after reconstruction
     // (src/sr_hllcbatten.F90:226-227), which the FP64 variants keep.  In FP32
     // that difference loses everything where the water is a trace: with
@@ -1344,11 +1353,11 @@ __device__ __forceinline__ void face_eval(const DevMesh& m, const DevState<R>& s
     R phipL = R(0), phipR = R(0);
     if constexpr (sizeof(R) == 4) {
         if (P.five_phase) {
-            phipL = (R)(1.0 - PLD(COL(s.pr, P_PHIG) + i));
-            phipR = (R)(1.0 - PLD(COL(s.pr, P_PHIG) + neigh));
+            phipL = (R)(1.0 - PLD(PCOL(s.pr, P_PHIG) + po(i)));
+            phipR = (R)(1.0 - PLD(PCOL(s.pr, P_PHIG) + po(neigh)));
         } else {
-            phipL = (R)PLD(COL(pr, P_PHIP) + i);
-            phipR = (R)PLD(COL(pr, P_PHIP) + neigh);
+            phipL = (R)PLD(PCOL(pr, P_PHIP) + po(i));
+            phipR = (R)PLD(PCOL(pr, P_PHIP) + po(neigh));
         }
     }
     if constexpr (Z == 2) {
@@ -1373,8 +1382,8 @@ __device__ __forceinline__ void face_eval(const DevMesh& m, const DevState<R>& s
         }
         const R rrg = (R)P.rrg, gamag = (R)P.gamag, gamap = (R)P.gamap, pinf = (R)P.pinf, cpp = (R)P.cpp;
         const R rgm1 = (R)P.r_gm1, rgamap = (R)P.r_gamap;
-        const R rogL = (R)PLD(COL(pr, P_ROG) + i), ropL = (R)PLD(COL(pr, P_ROP) + i);
-        const R rogR = (R)PLD(COL(pr, P_ROG) + neigh), ropR = (R)PLD(COL(pr, P_ROP) + neigh);
+        const R rogL = (R)PLD(PCOL(pr, P_ROG) + po(i)), ropL = (R)PLD(PCOL(pr, P_ROP) + po(i));
+        const R rogR = (R)PLD(PCOL(pr, P_ROG) + po(neigh)), ropR = (R)PLD(PCOL(pr, P_ROP) + po(neigh));
         const R rrogL = mrcp<F>(rogL, bad), rrogR = mrcp<F>(rogR, bad);
         const R rropL = mrcp<F>(ropL, bad), rropR = mrcp<F>(ropR, bad);
         // :194-212 (the sound speeds formed there enter no flux)
@@ -1787,11 +1796,11 @@ __device__ __forceinline__ void k_flux_body(DevMesh m, DevState<R> s, DevParams 
     // interphase sources with the 1/r-weighted LSQ gradient of alpha_g
     {
         const double* pr = s.pr;
-        const R tg = (R)COL(pr, P_TG)[i], phig = (R)COL(pr, P_PHIG)[i], rog = (R)COL(pr, P_ROG)[i];
-        const R rop = (R)COL(pr, P_ROP)[i], phip = (R)COL(pr, P_PHIP)[i];
-        const R ug = (R)COL(pr, P_UG)[i], vg = (R)COL(pr, P_VG)[i], wg = (R)COL(pr, P_WG)[i];
-        const R up = (R)COL(pr, P_UP)[i], vp = (R)COL(pr, P_VP)[i], wp = (R)COL(pr, P_WP)[i];
-        const R tp = (R)COL(pr, P_TP)[i], pg = (R)COL(pr, P_PG)[i];
+        const R tg = (R)PCOL(pr, P_TG)[po(i)], phig = (R)PCOL(pr, P_PHIG)[po(i)], rog = (R)PCOL(pr, P_ROG)[po(i)];
+        const R rop = (R)PCOL(pr, P_ROP)[po(i)], phip = (R)PCOL(pr, P_PHIP)[po(i)];
+        const R ug = (R)PCOL(pr, P_UG)[po(i)], vg = (R)PCOL(pr, P_VG)[po(i)], wg = (R)PCOL(pr, P_WG)[po(i)];
+        const R up = (R)PCOL(pr, P_UP)[po(i)], vp = (R)PCOL(pr, P_VP)[po(i)], wp = (R)PCOL(pr, P_WP)[po(i)];
+        const R tp = (R)PCOL(pr, P_TP)[po(i)], pg = (R)PCOL(pr, P_PG)[po(i)];
         const R dl = (R)ldg(m.dl + i), voli = (R)ldg(m.vol + i);
         const R amug = (R)P.as * sqrt(tg) / (R(1) + (R)P.ts / tg);
         const R du = ug - up, dv = vg - vp, dw = wg - wp;
@@ -1802,7 +1811,7 @@ __device__ __forceinline__ void k_flux_body(DevMesh m, DevState<R> s, DevParams 
         // forms in FP64)
         R drag, omg;
         if constexpr (sizeof(R) == 4) {
-            omg = P.five_phase ? (R)(1.0 - COL(s.pr, P_PHIG)[i]) : phip;
+            omg = P.five_phase ? (R)(1.0 - PCOL(s.pr, P_PHIG)[po(i)]) : phip;
             drag = -(R(0.44) * phig * omg) * rog * sqrt(du * du + dv * dv + dw * dw) * dl;
         } else {
             omg = R(1) - phig;
@@ -1832,7 +1841,7 @@ __device__ __forceinline__ void k_flux_body(DevMesh m, DevState<R> s, DevParams 
                 xa[f] = (R)(ldg(m.xc + n) - x0);
                 ya[f] = (R)(ldg(m.yc + n) - y0);
                 za[f] = (R)(ldg(m.zc + n) - z0);
-                pa[f] = (R)(COL(pr, P_PHIG)[n] - COL(pr, P_PHIG)[i]);
+                pa[f] = (R)(PCOL(pr, P_PHIG)[po(n)] - PCOL(pr, P_PHIG)[po(i)]);
             }
 #if HP_LSQ_TABLE
             R wt[4], rw[4];
@@ -1932,10 +1941,10 @@ __device__ __forceinline__ unsigned grad4_limiter(const DevMesh& m, const DevSta
         __syncwarp();
     }
     const R epssq = lc ? (R)lc[12 * LIMC_LD] : (R)ldg(m.eps2 + i);
-    const R* qq = COL(s.prr, lcol);
-    R qi = lp ? (R)lp[0] : qq[i];
-    R q0 = lp ? (R)lp[LIM_LD] : qq[n[0]], q1 = lp ? (R)lp[2 * LIM_LD] : qq[n[1]];
-    R q2 = lp ? (R)lp[3 * LIM_LD] : qq[n[2]], q3 = lp ? (R)lp[4 * LIM_LD] : qq[n[3]];
+    const R* qq = PCOL(s.prr, lcol);
+    R qi = lp ? (R)lp[0] : qq[po(i)];
+    R q0 = lp ? (R)lp[LIM_LD] : qq[po(n[0])], q1 = lp ? (R)lp[2 * LIM_LD] : qq[po(n[1])];
+    R q2 = lp ? (R)lp[3 * LIM_LD] : qq[po(n[2])], q3 = lp ? (R)lp[4 * LIM_LD] : qq[po(n[3])];
     R vmax = mx2(mx2(mx2(mx2(qi, q0), q1), q2), q3);
     R vmin = mn2(mn2(mn2(mn2(qi, q0), q1), q2), q3);
     R dmax = (R)(vmax - qi), dmin = (R)(vmin - qi);
@@ -2116,9 +2125,10 @@ __device__ __forceinline__ unsigned grad4_body(const DevMesh& m, const DevState<
     for (int r = 0; r < 4; r++) {
         const int v = q + 4 * r;
         if (v >= 13) break;
-        const R* qq = COL(s.prr, pcol[v]);
-        R qi = qq[i];
-        R qa = (R)(qq[n[0]] - qi), qb = (R)(qq[n[1]] - qi), qc = (R)(qq[n[2]] - qi), qd = (R)(qq[n[3]] - qi);
+        const R* qq = PCOL(s.prr, pcol[v]);
+        R qi = qq[po(i)];
+        R qa = (R)(qq[po(n[0])] - qi), qb = (R)(qq[po(n[1])] - qi), qc = (R)(qq[po(n[2])] - qi),
+          qd = (R)(qq[po(n[3])] - qi);
         R c1 = DW(qa * xa[0], 0) + DW(qb * xa[1], 1) + DW(qc * xa[2], 2) + DW(qd * xa[3], 3);
         R c2;
         if (v == 7)   // cTp2 lacks the /wt4 (src/sr_derivative.F90:225)
@@ -2176,21 +2186,21 @@ __device__ __forceinline__ void k_grad4_body(DevMesh m, DevState<R> s, DevParams
         for (int r = 0; r < 4; r++) {
             const int v = q + 4 * r;
             if (v < 13) {
-                const double* qv = reinterpret_cast<const double*>(COL(s.prr, pcol[v]));
+                const double* qv = reinterpret_cast<const double*>(PCOL(s.prr, pcol[v]));
                 double* g = sgat + 5 * r * LIM_LD + tid;
-                cp_async8(g, qv + i);
+                cp_async8(g, qv + po(i));
 #pragma unroll
-                for (int f = 0; f < 4; f++) cp_async8(g + (1 + f) * LIM_LD, qv + nn[f]);
+                for (int f = 0; f < 4; f++) cp_async8(g + (1 + f) * LIM_LD, qv + po(nn[f]));
             }
             cp_async_commit();
         }
         // group 5: the limiter field at the cell and its neighbours, face
         // centroid columns q, 4 + q, 8 + q and (lane 0) epsilon^2
         const int lcol = q == 0 ? P_PG : q == 1 ? P_PP : q == 2 ? P_ROG : P_ROP;
-        const double* ql = reinterpret_cast<const double*>(COL(s.prr, lcol));
-        cp_async8(slim + tid, ql + i);
+        const double* ql = reinterpret_cast<const double*>(PCOL(s.prr, lcol));
+        cp_async8(slim + tid, ql + po(i));
 #pragma unroll
-        for (int f = 0; f < 4; f++) cp_async8(slim + (1 + f) * LIM_LD + tid, ql + nn[f]);
+        for (int f = 0; f < 4; f++) cp_async8(slim + (1 + f) * LIM_LD + tid, ql + po(nn[f]));
 #pragma unroll
         for (int d = 0; d < 3; d++) cp_async8(slimc + (4 * d + q) * LIMC_LD + cl, COL(m.fxo, 4 * d + q) + i);
         if (q == 0) cp_async8(slimc + 12 * LIMC_LD + cl, m.eps2 + i);
@@ -2290,7 +2300,7 @@ __device__ __forceinline__ bool flux4_body(const DevMesh& m, const DevState<R>& 
     const R xq = (R)(ldg(m.xc + nq) - x0), yq = (R)(ldg(m.yc + nq) - y0), zq = (R)(ldg(m.zc + nq) - z0);
 #endif
     // alpha_g differences from the FP64 primitives (see k_grad)
-    const R pq = (R)(COL(s.pr, P_PHIG)[nq] - COL(s.pr, P_PHIG)[i]);
+    const R pq = (R)(PCOL(s.pr, P_PHIG)[po(nq)] - PCOL(s.pr, P_PHIG)[po(i)]);
     // residual of this lane's variables j = q, q + 4, q + 8 in face order 1..4
     // (src/sr_hllcbatten.F90:534-552): a wall face adds its pressure terms, a
     // face that took no wave branch (NaN states) the flux of the face before
@@ -2323,12 +2333,12 @@ __device__ __forceinline__ bool flux4_body(const DevMesh& m, const DevState<R>& 
     }
     // interphase sources (src/sr_source.F90:46-155)
     {
-        const R tg = (R)COL(pr, P_TG)[i], phig = (R)COL(pr, P_PHIG)[i],
-                rog = (R)COL(pr, P_ROG)[i];
-        const R rop = (R)COL(pr, P_ROP)[i], phip = (R)COL(pr, P_PHIP)[i];
-        const R ug = (R)COL(pr, P_UG)[i], vg = (R)COL(pr, P_VG)[i], wg = (R)COL(pr, P_WG)[i];
-        const R up = (R)COL(pr, P_UP)[i], vp = (R)COL(pr, P_VP)[i], wp = (R)COL(pr, P_WP)[i];
-        const R tp = (R)COL(pr, P_TP)[i], pg = (R)COL(pr, P_PG)[i];
+        const R tg = (R)PCOL(pr, P_TG)[po(i)], phig = (R)PCOL(pr, P_PHIG)[po(i)],
+                rog = (R)PCOL(pr, P_ROG)[po(i)];
+        const R rop = (R)PCOL(pr, P_ROP)[po(i)], phip = (R)PCOL(pr, P_PHIP)[po(i)];
+        const R ug = (R)PCOL(pr, P_UG)[po(i)], vg = (R)PCOL(pr, P_VG)[po(i)], wg = (R)PCOL(pr, P_WG)[po(i)];
+        const R up = (R)PCOL(pr, P_UP)[po(i)], vp = (R)PCOL(pr, P_VP)[po(i)], wp = (R)PCOL(pr, P_WP)[po(i)];
+        const R tp = (R)PCOL(pr, P_TP)[po(i)], pg = (R)PCOL(pr, P_PG)[po(i)];
         const R dl = TL(TAIL_DL, ldg(m.dl + i)), voli = TL(TAIL_VOL, ldg(m.vol + i));
         const R amug = (R)P.as * sqrt(tg) / (R(1) + (R)P.ts / tg);
         const R du = ug - up, dv = vg - vp, dw = wg - wp;
@@ -2339,7 +2349,7 @@ __device__ __forceinline__ bool flux4_body(const DevMesh& m, const DevState<R>& 
         // forms in FP64)
         R drag, omg;
         if constexpr (sizeof(R) == 4) {
-            omg = P.five_phase ? (R)(1.0 - COL(s.pr, P_PHIG)[i]) : phip;
+            omg = P.five_phase ? (R)(1.0 - PCOL(s.pr, P_PHIG)[po(i)]) : phip;
             drag = -(R(0.44) * phig * omg) * rog * sqrt(du * du + dv * dv + dw * dw) * dl;
         } else {
             omg = R(1) - phig;
@@ -2624,9 +2634,9 @@ __device__ __forceinline__ void visc_face(const DevMesh& m, const DevState<R>& s
     const R c23 = (R)P.c23;
     R ff[8];
 #pragma unroll
-    for (int v = 0; v < 8; v++) ff[v] = (R)((COL(pr, fcol[v])[i] + COL(pr, fcol[v])[neigh]) * 0.5);
-    const R phigf = (R)((COL(pr, P_PHIG)[i] + COL(pr, P_PHIG)[neigh]) * 0.5);
-    const R phipf = (R)((COL(pr, P_PHIP)[i] + COL(pr, P_PHIP)[neigh]) * 0.5);
+    for (int v = 0; v < 8; v++) ff[v] = (R)((PCOL(pr, fcol[v])[po(i)] + PCOL(pr, fcol[v])[po(neigh)]) * 0.5);
+    const R phigf = (R)((PCOL(pr, P_PHIG)[po(i)] + PCOL(pr, P_PHIG)[po(neigh)]) * 0.5);
+    const R phipf = (R)((PCOL(pr, P_PHIP)[po(i)] + PCOL(pr, P_PHIP)[po(neigh)]) * 0.5);
     const R tgf = ff[3];
     const R amug = (R)P.as * sqrt(tgf) / (R(1) + (R)P.ts / tgf);
     const R akg = mdiv<F>(amug * (R)P.cpg, (R)P.prg, (R)P.r_prg, bad);
@@ -2659,11 +2669,11 @@ __device__ __forceinline__ void visc_face(const DevMesh& m, const DevState<R>& s
     R gr[8][3];
 #pragma unroll
     for (int v = 0; v < 8; v++) {
-        const PT* q = COL(pr, fcol[v]);
-        R d0 = (R)q[mm[0]] - ff[v];
+        const PT* q = PCOL(pr, fcol[v]);
+        R d0 = (R)q[po(mm[0])] - ff[v];
         R b1 = d0 * dx[0], b2 = d0 * dy[0], b3 = d0 * dz[0];
         for (int k = 1; k < nm; k++) {
-            R dk = (R)q[mm[k]] - ff[v];
+            R dk = (R)q[po(mm[k])] - ff[v];
             b1 = b1 + dk * dx[k]; b2 = b2 + dk * dy[k]; b3 = b3 + dk * dz[k];
         }
         gr[v][0] = mdiv<F>(det3(b1, b2, b3, a12, a22, a23, a13, a23, a33), dnr, rdnr, bad);
@@ -2723,8 +2733,8 @@ __device__ __forceinline__ void visc_face_ph(const DevMesh& m, const DevState<R>
     const int neigh = nci[f];
     R ff[4];
 #pragma unroll
-    for (int v = 0; v < 4; v++) ff[v] = (R)((COL(pr, c0 + v)[i] + COL(pr, c0 + v)[neigh]) * 0.5);
-    const R phif = (R)((COL(pr, P_PHIG + ph)[i] + COL(pr, P_PHIG + ph)[neigh]) * 0.5);
+    for (int v = 0; v < 4; v++) ff[v] = (R)((PCOL(pr, c0 + v)[po(i)] + PCOL(pr, c0 + v)[po(neigh)]) * 0.5);
+    const R phif = (R)((PCOL(pr, P_PHIG + ph)[po(i)] + PCOL(pr, P_PHIG + ph)[po(neigh)]) * 0.5);
     R amu, ak;
     if (ph == 0) {
         const R tgf = ff[3];
@@ -2749,7 +2759,7 @@ __device__ __forceinline__ void visc_face_ph(const DevMesh& m, const DevState<R>
         }
 #pragma unroll
         for (int v = 0; v < 4; v++) {
-            const R d = (R)COL(pr, c0 + v)[mk] - ff[v];
+            const R d = (R)PCOL(pr, c0 + v)[po(mk)] - ff[v];
             if (k == 0) {
                 b[v][0] = d * dx; b[v][1] = d * dy; b[v][2] = d * dz;
             } else {
@@ -3014,8 +3024,8 @@ __global__ void __launch_bounds__(256) k_qrs_diss1(DevMesh m, DevState<R> s) {
     const int a = ldg(COL(m.snb, 0) + i), b = ldg(COL(m.snb, 1) + i);
     const int c = ldg(COL(m.snb, 2) + i), d = ldg(COL(m.snb, 3) + i);
     const double e16 = (double)1.0e-16f;      // a REAL(4) literal in the reference
-    const double* pp = COL(s.pr, P_PP);
-    const double ppi = pp[i], ppa = pp[a], ppb = pp[b], ppc = pp[c], ppd = pp[d];
+    const double* pp = PCOL(s.pr, P_PP);
+    const double ppi = pp[po(i)], ppa = pp[po(a)], ppb = pp[po(b)], ppc = pp[po(c)], ppd = pp[po(d)];
     double anun = fabs(ppa - ppi) + fabs(ppb - ppi) + fabs(ppc - ppi) + fabs(ppd - ppi);
     double anud = fabs(ppa + ppi) + fabs(ppb + ppi) + fabs(ppc + ppi) + fabs(ppd + ppi);
     double anupp = anun / anud;
@@ -3094,7 +3104,7 @@ __global__ void __launch_bounds__(256) k_qrs_prim(DevMesh m, DevState<R> s, DevP
     double phd[3], u[3], v[3], w[3];
 #pragma unroll
     for (int d = 0; d < 3; d++) phd[d] = mn2(mx2(COL(s.cn, 10 + 4 * d)[i] / P.rhod[d], emin), 1.0 - emin);
-    const double phitotal = COL(s.pr, P_PHIG)[i] + COL(s.pr, P_PHIP)[i] + phd[0] + phd[1] + phd[2];
+    const double phitotal = PCOL(s.pr, P_PHIG)[po(i)] + PCOL(s.pr, P_PHIP)[po(i)] + phd[0] + phd[1] + phd[2];
 #pragma unroll
     for (int d = 0; d < 3; d++) phd[d] = phd[d] / phitotal;
 #pragma unroll
@@ -3137,7 +3147,7 @@ __global__ void __launch_bounds__(256) k_qrs_bc(DevMesh m, DevState<R> s, DevPar
         double* w = COL(s.qpr, 4 * d + 3);
         if (nt == 2) {
             ph[ng] = P.emin;
-            u[ng] = COL(s.pr, P_UP)[ng]; v[ng] = COL(s.pr, P_VP)[ng]; w[ng] = COL(s.pr, P_WP)[ng];
+            u[ng] = PCOL(s.pr, P_UP)[po(ng)]; v[ng] = PCOL(s.pr, P_VP)[po(ng)]; w[ng] = PCOL(s.pr, P_WP)[po(ng)];
         } else if (nt == 3) {
             ph[ng] = ph[np]; u[ng] = u[np]; v[ng] = v[np]; w[ng] = w[np];
         } else if (nt == 5) {
@@ -3195,7 +3205,7 @@ __global__ void __launch_bounds__(128) k_qrs_flux(DevMesh m, DevState<R> s, DevP
     }
     // drag (Schiller-Naumann-type coefficient of the reference)
     const double voli = ldg(m.vol + i);
-    const double up = COL(s.pr, P_UP)[i], vp = COL(s.pr, P_VP)[i], wp = COL(s.pr, P_WP)[i];
+    const double up = PCOL(s.pr, P_UP)[po(i)], vp = PCOL(s.pr, P_VP)[po(i)], wp = PCOL(s.pr, P_WP)[po(i)];
     const double amup = 0.001, gravity = 0.0;
 #pragma unroll
     for (int d = 0; d < 3; d++) {
