@@ -2,7 +2,8 @@
 // per-variant kernel entry table.  Shared by the host code (hp_host.cu) and
 // every precision variant (hp_variant_*.cu).
 //
-// Layout in HBM: structure of arrays, one column per variable, leading
+// Layout in HBM: structure of arrays, one column per variable (primitives and
+// gradients: tiles of 32 cells, see prim_off), leading
 // dimension `ld` (= ntot rounded up to 64 cells) so each column starts on a
 // 512-byte boundary.  Cell ids are 0-based internally: elements [0, neles),
 // boundary ghosts [neles, neles + nghosts) -- the reference's 1-based ids
