@@ -344,10 +344,12 @@ int hp_poll(hp_handle *h, int32_t *busy);
  * dt_dev[0].  Device pointers; the work is queued on `stream` (a
  * cudaStream_t, NULL for the default stream) and the call returns without
  * waiting.  The call allocates nothing: its only scratch, one partial minimum
- * per 256 cells and 1024 block counters, is a static device array sized for HP_NOALLOC_MAX_CELLS
- * cells that each GPU using the library keeps until exit; larger ncells is
- * rejected with HP_E_ARG.  All calls share that array, so calls that overlap
- * on the GPU race.  The first call on each device looks up the array's device
+ * per 256 cells and 1024 block counters, is a static device array sized for
+ * HP_NOALLOC_MAX_CELLS cells that each GPU using the library keeps until exit;
+ * larger ncells is rejected with HP_E_ARG.  All calls share that array, so
+ * calls that overlap on the GPU race: their results are undefined (dt_dev may
+ * stay as it was), later calls are not affected.  A call into a capturing
+ * stream records two launches, any other is one.  The first call on each device looks up the array's device
  * address; make it before any stream capture.  The lookup is repeated when
  * the device's context changes (after cudaDeviceReset, or a runtime that
  * shuts the device down and opens it again), so the call stays valid across

@@ -28,22 +28,23 @@
 #include <mutex>
 
 #include "../../include/hydraphase.h"
+#include "hp_dt_count.h"
 
 namespace {
 
 constexpr int kBlock = 256;
 constexpr int kMaxBlocks = HP_NOALLOC_MAX_CELLS / kBlock;
+static_assert(kMaxBlocks < (1 << hp::DT_COUNT_BITS), "a call's blocks must fit its range of a counter");
 constexpr int kCounters = 1024;
 
 // One partial minimum (bit pattern of a non-negative double) per block, then
-// the counters of finished blocks.  The partial minima are shared by every
-// call on the device; each call writes the slots it reads, so nothing has to
-// be cleared between calls.  Calls that overlap on the GPU (different
-// streams, or threads issuing concurrently) race on them.  A counter belongs
-// to one call (they are handed out in turn; a captured call keeps its own)
-// and is left at zero, so a race on the minima does not outlive its calls.
+// the counters of finished blocks.  Both are shared by every call on the
+// device, and each call is right whatever an earlier one left in them: it
+// writes the minima that it reads, and counts in its own range of a counter
+// (hp_dt_count.h).  Calls that overlap on the GPU (different streams, or threads
+// issuing concurrently) race on the minima.
 static __device__ __align__(256) unsigned long long g_dt_partial[kMaxBlocks + kCounters];
-std::atomic<unsigned> g_call{0};
+std::atomic<unsigned long long> g_call{0};
 
 std::mutex g_mu;
 constexpr int kMaxDevices = 64;
@@ -103,16 +104,44 @@ cudaError_t scratch_on_device(int dev, unsigned long long** out) {
 using namespace hp;
 using namespace hp::v_noalloc;
 
-// One launch: each block stores its partial minimum, and the block that
-// finishes last reduces them all.  (A second, one-block launch for that
-// reduction cost the caller as much again: 48,000 cells, calls back to back,
-// 10.2 -> 8.6 us a call.)
-__global__ void __launch_bounds__(kBlock) k_dt(const double* cn, long long ld, const double* dl, int n, DevParams P,
-                                               unsigned long long* part, unsigned long long* done, double* dt_out) {
+// minimum of the block's keys, for thread 0
+__device__ __forceinline__ unsigned long long block_min(unsigned long long v) {
     __shared__ unsigned long long red[kBlock / 32];
-    __shared__ int last;
+    v = warp_min_u64(v);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+#pragma unroll
+        for (int w = 1; w < kBlock / 32; w++) v = red[w] < v ? red[w] : v;
+    }
+    return v;
+}
+
+// dt from the partial minima, by one block.  The reference's running minimum
+// starts at 1.0E8 (src/main.F90:521); four loads in flight a thread.
+__device__ __forceinline__ void dt_from_partials(const unsigned long long* part, int nb, double cfl, double* dt_out) {
+    unsigned long long v = (unsigned long long)__double_as_longlong(1.0e8);
+    for (int b = threadIdx.x; b < nb; b += 4 * kBlock) {
+        unsigned long long w[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) w[u] = b + u * kBlock < nb ? __ldcg(part + b + u * kBlock) : v;
+#pragma unroll
+        for (int u = 0; u < 4; u++) v = w[u] < v ? w[u] : v;
+    }
+    v = block_min(v);
+    if (threadIdx.x == 0) dt_out[0] = __longlong_as_double((long long)v) * cfl;
+}
+
+// Each block stores its partial minimum.  ONE: the block that finishes last
+// (see hp_dt_count.h) reduces them all, in the same launch; a second,
+// one-block launch for that cost the caller as much again (48,000 cells,
+// calls back to back, 10.2 -> 8.6 us a call).
+template <bool ONE>
+__global__ void __launch_bounds__(kBlock) k_dt(const double* cn, long long ld, const double* dl, int n, DevParams P,
+                                               unsigned long long* part, unsigned long long* done,
+                                               unsigned long long call, double* dt_out) {
+    if (ONE && threadIdx.x == 0) dt_count_open(done, call);
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     unsigned long long key = ~0ull;
     if (i < n) {
         double c[10];
@@ -123,39 +152,24 @@ __global__ void __launch_bounds__(kBlock) k_dt(const double* cn, long long ld, c
         prim_full(c, q, P);
         key = dt_key(P, q, dli);
     }
-    key = warp_min_u64(key);
-    if (lane == 0) red[wid] = key;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-#pragma unroll
-        for (int w = 1; w < kBlock / 32; w++) key = red[w] < key ? red[w] : key;
-        __stcg(part + blockIdx.x, key);
-        __threadfence();
-        last = atomicAdd(done, 1ull) == gridDim.x - 1;
-        __threadfence();
+    key = block_min(key);
+    if constexpr (ONE) {
+        __shared__ int last;
+        if (threadIdx.x == 0) {
+            __stcg(part + blockIdx.x, key);
+            __threadfence();
+            last = dt_count_arrive(done, call, gridDim.x);
+            __threadfence();
+        }
+        __syncthreads();
+        if (last) dt_from_partials(part, (int)gridDim.x, P.cfl, dt_out);
+    } else {
+        if (threadIdx.x == 0) __stcg(part + blockIdx.x, key);
     }
-    __syncthreads();
-    if (!last) return;
-    // the reference's running minimum starts at 1.0E8 (src/main.F90:521);
-    // four loads in flight a thread
-    unsigned long long v = (unsigned long long)__double_as_longlong(1.0e8);
-    const int nb = (int)gridDim.x;
-    for (int b = threadIdx.x; b < nb; b += 4 * kBlock) {
-        unsigned long long w[4];
-#pragma unroll
-        for (int u = 0; u < 4; u++) w[u] = b + u * kBlock < nb ? __ldcg(part + b + u * kBlock) : v;
-#pragma unroll
-        for (int u = 0; u < 4; u++) v = w[u] < v ? w[u] : v;
-    }
-    v = warp_min_u64(v);
-    if (lane == 0) red[wid] = v;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-#pragma unroll
-        for (int w = 1; w < kBlock / 32; w++) v = red[w] < v ? red[w] : v;
-        dt_out[0] = __longlong_as_double((long long)v) * P.cfl;
-        *done = 0ull;
-    }
+}
+__global__ void __launch_bounds__(kBlock) k_dt_final(const unsigned long long* part, int nb, double cfl,
+                                                     double* dt_out) {
+    dt_from_partials(part, nb, cfl, dt_out);
 }
 
 }  // namespace
@@ -182,8 +196,20 @@ extern "C" int hp_dt_noalloc(const double* cn_dev, int64_t ld, const double* dl_
     P.r_emm = 1.0 / (P.emax - P.emin);
     const int nblocks = (ncells + kBlock - 1) / kBlock;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    k_dt<<<nblocks, kBlock, 0, st>>>(cn_dev, ld, dl_dev, ncells, P, part,
-                                     part + kMaxBlocks + g_call.fetch_add(1) % kCounters, dt_dev);
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) {
+        cudaGetLastError();   // a legacy-stream call beside a capture: refused, as its launch would be
+        return HP_E_CUDA;
+    }
+    if (cap == cudaStreamCaptureStatusNone) {
+        const unsigned long long call = g_call.fetch_add(1) + 1;
+        k_dt<true><<<nblocks, kBlock, 0, st>>>(cn_dev, ld, dl_dev, ncells, P, part,
+                                               part + kMaxBlocks + call % kCounters, call, dt_dev);
+    } else {
+        // a captured launch is replayed with the same call number: no counter
+        k_dt<false><<<nblocks, kBlock, 0, st>>>(cn_dev, ld, dl_dev, ncells, P, part, nullptr, 0, dt_dev);
+        k_dt_final<<<1, kBlock, 0, st>>>(part, nblocks, P.cfl, dt_dev);
+    }
     // nothing was pending on entry, so an error now is this call's launch
     return cudaGetLastError() == cudaSuccess ? HP_OK : HP_E_CUDA;
 }
