@@ -237,8 +237,10 @@ __global__ void k_hole_cut(DMesh M, const int* block, hp_ov::HoleView H, int32_t
     iblank[e - 1] = ib;
 }
 
-// Device buffers of one build, freed on every exit.
-// The temporary device memory of one call and the stream of its work.  The
+// The temporary device memory of one call and the stream of its work.  Every
+// exit, by an error too, frees the memory and waits for the stream: what was
+// queued reads and writes arrays of the caller, and host arrays of the call
+// that are declared before this object.  The
 // buffers come from the device's stream-ordered pool, which may keep up to
 // POOL_KEEP bytes between calls (more where a handle of this library already
 // keeps its arenas there): twenty cudaMalloc and cudaFree per table, each of
@@ -264,7 +266,9 @@ struct Buffers {
     }
     ~Buffers() {
         for (void* q : p) cudaFreeAsync(q, st);
-        if (st) cudaStreamDestroy(st);
+        if (!st) return;
+        cudaStreamSynchronize(st);
+        cudaStreamDestroy(st);
     }
     template <class T>
     cudaError_t get(T** out, size_t n) {
@@ -303,7 +307,6 @@ extern "C" int hp_overset_build_gpu(const hp_mesh* mesh, const int32_t* block, i
     for (int f = 0; f < nf; f++) out->fringe[f] = P.fr[f];
     if (nf == 0) return HP_OK;
     {
-        Buffers buf;
         cudaStream_t st = nullptr;
         double *x = nullptr, *y = nullptr, *z = nullptr, *w = nullptr;
         int32_t *elem = nullptr, *dn = nullptr;
@@ -313,6 +316,7 @@ extern "C" int hp_overset_build_gpu(const hp_mesh* mesh, const int32_t* block, i
         std::vector<int> hdonor(nf), hmiss;
         Bins bins[2];
         DMesh M;
+        Buffers buf;
         OV_CUDA(buf.open());
         st = buf.st;
         OV_CUDA(buf.get(&x, nodes));
@@ -405,13 +409,13 @@ extern "C" int hp_overset_hole_cut_gpu(const hp_mesh* mesh, const int32_t* block
     if (rc != HP_OK) return rc;
     const int neles = mesh->neles, nodes = mesh->nodes;
     {
-        Buffers buf;
         cudaStream_t st = nullptr;
         double *x = nullptr, *y = nullptr, *z = nullptr, *tri = nullptr;
         int32_t *elem = nullptr, *ib = nullptr;
         int *blk = nullptr, *s3 = nullptr, *i3 = nullptr, *s2 = nullptr, *i2 = nullptr, *cnt = nullptr;
         int hcount = 0;
         hp_ov::HoleView V = HP.v;
+        Buffers buf;
         OV_CUDA(buf.open());
         st = buf.st;
         OV_CUDA(buf.get(&x, nodes));
