@@ -219,8 +219,10 @@ int hp_overset_build(const hp_mesh *mesh, const int32_t *block, int32_t layers, 
                      int32_t *iblank_out, hp_overset *out);
 /* The same tables, bit for bit, with the donor search, the nearest-centroid
  * fallback and the weights on the current CUDA device (the host marks the
- * fringe and sizes the search grids).  Allocates temporary device memory;
- * HP_E_CUDA if a device call fails. */
+ * fringe and sizes the search grids).  Temporary device memory comes
+ * from the device's default memory pool and goes back to it before the call
+ * returns; nothing that the call queued is unfinished then, whatever its
+ * status.  HP_E_CUDA if a device call fails. */
 int hp_overset_build_gpu(const hp_mesh *mesh, const int32_t *block, int32_t layers, int32_t outer_type,
                          int32_t *iblank_out, hp_overset *out);
 /* Hole cut, the step before hp_overset_build (new work: the reference takes

@@ -240,30 +240,22 @@ __global__ void k_hole_cut(DMesh M, const int* block, hp_ov::HoleView H, int32_t
 // The temporary device memory of one call and the stream of its work.  Every
 // exit, by an error too, frees the memory and waits for the stream: what was
 // queued reads and writes arrays of the caller, and host arrays of the call
-// that are declared before this object.  The
-// buffers come from the device's stream-ordered pool, which may keep up to
-// POOL_KEEP bytes between calls (more where a handle of this library already
-// keeps its arenas there): twenty cudaMalloc and cudaFree per table, each of
-// which synchronises the device, took 8 ms of a 246,000-cell mesh's hole cut
-// and tables at best and up to a second at worst (25 -> 14 ms a pass with
-// the pool).
-constexpr uint64_t POOL_KEEP = 256ull << 20;
+// that are declared before this object.
+//
+// One block of memory holds all buffers whose sizes are known at the start
+// (take() is called for each of them twice, to add up and to place), from the
+// device's stream-ordered pool.  The pool's settings stay the process's own:
+// where nothing has told it to keep memory (a handle of this library does),
+// the wait at the exit gives the block back.  Hole cut and tables of a
+// 246,000-cell mesh, a pass: 19.5 ms with a cudaMalloc and a cudaFree for
+// each of twenty buffers, 14.8 with the block, 15.4 with cudaMalloc for it,
+// 13.5 where the pool keeps it.
 struct Buffers {
     std::vector<void*> p;
     cudaStream_t st = nullptr;
-    cudaError_t open() {
-        int dev = 0;
-        cudaMemPool_t pool = nullptr;
-        uint64_t keep = 0;
-        cudaError_t e = cudaGetDevice(&dev);
-        if (e == cudaSuccess) e = cudaDeviceGetDefaultMemPool(&pool, dev);
-        if (e == cudaSuccess) e = cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
-        if (e == cudaSuccess && keep < POOL_KEEP) {
-            keep = POOL_KEEP;
-            e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
-        }
-        return e == cudaSuccess ? cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) : e;
-    }
+    char* base = nullptr;
+    size_t used = 0;
+    cudaError_t open() { return cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking); }
     ~Buffers() {
         for (void* q : p) cudaFreeAsync(q, st);
         if (!st) return;
@@ -271,11 +263,17 @@ struct Buffers {
         cudaStreamDestroy(st);
     }
     template <class T>
-    cudaError_t get(T** out, size_t n) {
+    void take(T** out, size_t n) {
+        *out = base ? reinterpret_cast<T*>(base + used) : nullptr;
+        used += (n * sizeof(T) + 255) / 256 * 256;
+    }
+    // memory for what has been taken so far; the takes are then repeated
+    cudaError_t alloc() {
         void* q = nullptr;
-        cudaError_t e = cudaMallocAsync(&q, (n ? n : 1) * sizeof(T), st);
+        cudaError_t e = cudaMallocAsync(&q, used ? used : 1, st);
         if (e == cudaSuccess) p.push_back(q);
-        *out = (T*)q;
+        base = static_cast<char*>(q);
+        used = 0;
         return e;
     }
 };
@@ -313,23 +311,42 @@ extern "C" int hp_overset_build_gpu(const hp_mesh* mesh, const int32_t* block, i
         int *blk = nullptr, *ib = nullptr, *fr = nullptr, *donor = nullptr, *miss = nullptr;
         int* field[2] = {nullptr, nullptr};
         int *start[2] = {nullptr, nullptr}, *items[2] = {nullptr, nullptr};
+        int *cnt[2] = {nullptr, nullptr}, *fill[2] = {nullptr, nullptr}, total[2] = {0, 0};
+        char* tmp[2] = {nullptr, nullptr};
+        size_t ncell[2] = {0, 0}, tmp_bytes[2] = {0, 0};
         std::vector<int> hdonor(nf), hmiss;
         Bins bins[2];
         DMesh M;
         Buffers buf;
         OV_CUDA(buf.open());
         st = buf.st;
-        OV_CUDA(buf.get(&x, nodes));
-        OV_CUDA(buf.get(&y, nodes));
-        OV_CUDA(buf.get(&z, nodes));
-        OV_CUDA(buf.get(&elem, 9 * (size_t)neles));
-        OV_CUDA(buf.get(&blk, neles));
-        OV_CUDA(buf.get(&ib, neles));
-        OV_CUDA(buf.get(&fr, nf));
-        OV_CUDA(buf.get(&donor, nf));
-        OV_CUDA(buf.get(&miss, nf));
-        OV_CUDA(buf.get(&dn, 4 * (size_t)nf));
-        OV_CUDA(buf.get(&w, 4 * (size_t)nf));
+        for (int b = 0; b < 2; b++) {
+            ncell[b] = (size_t)P.grid[b].n[0] * P.grid[b].n[1] * P.grid[b].n[2];
+            if (!P.field[b].empty())
+                OV_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tmp_bytes[b], cnt[b], start[b], (int)(ncell[b] + 1), st));
+        }
+        for (int pass = 0; pass < 2; pass++) {
+            if (pass) OV_CUDA(buf.alloc());
+            buf.take(&x, nodes);
+            buf.take(&y, nodes);
+            buf.take(&z, nodes);
+            buf.take(&elem, 9 * (size_t)neles);
+            buf.take(&blk, neles);
+            buf.take(&ib, neles);
+            buf.take(&fr, nf);
+            buf.take(&donor, nf);
+            buf.take(&miss, nf);
+            buf.take(&dn, 4 * (size_t)nf);
+            buf.take(&w, 4 * (size_t)nf);
+            for (int b = 0; b < 2; b++) {
+                if (P.field[b].empty()) continue;
+                buf.take(&field[b], P.field[b].size());
+                buf.take(&cnt[b], ncell[b] + 1);
+                buf.take(&start[b], ncell[b] + 1);
+                buf.take(&fill[b], ncell[b]);
+                buf.take(&tmp[b], tmp_bytes[b]);
+            }
+        }
         OV_CUDA(cudaMemcpyAsync(x, mesh->x, nodes * sizeof(double), cudaMemcpyHostToDevice, st));
         OV_CUDA(cudaMemcpyAsync(y, mesh->y, nodes * sizeof(double), cudaMemcpyHostToDevice, st));
         OV_CUDA(cudaMemcpyAsync(z, mesh->z, nodes * sizeof(double), cudaMemcpyHostToDevice, st));
@@ -338,6 +355,8 @@ extern "C" int hp_overset_build_gpu(const hp_mesh* mesh, const int32_t* block, i
         OV_CUDA(cudaMemcpyAsync(ib, iblank_out, neles * sizeof(int), cudaMemcpyHostToDevice, st));
         OV_CUDA(cudaMemcpyAsync(fr, P.fr.data(), nf * sizeof(int), cudaMemcpyHostToDevice, st));
         M = DMesh{x, y, z, elem, neles};
+        // bins of both blocks: counts and their scans, then, with the totals
+        // on the host, the items
         for (int b = 0; b < 2; b++) {
             const int n = (int)P.field[b].size();
             bins[b].g = P.grid[b];
@@ -345,28 +364,25 @@ extern "C" int hp_overset_build_gpu(const hp_mesh* mesh, const int32_t* block, i
             bins[b].start = nullptr;
             bins[b].items = nullptr;
             if (n == 0) continue;
-            const hp_ov::GridParams& g = P.grid[b];
-            const size_t ncell = (size_t)g.n[0] * g.n[1] * g.n[2];
-            int *cnt = nullptr, *fill = nullptr;
-            OV_CUDA(buf.get(&field[b], n));
             OV_CUDA(cudaMemcpyAsync(field[b], P.field[b].data(), n * sizeof(int), cudaMemcpyHostToDevice, st));
-            OV_CUDA(buf.get(&cnt, ncell + 1));
-            OV_CUDA(buf.get(&start[b], ncell + 1));
-            OV_CUDA(buf.get(&fill, ncell));
-            OV_CUDA(cudaMemsetAsync(cnt, 0, (ncell + 1) * sizeof(int), st));
-            OV_CUDA(cudaMemsetAsync(fill, 0, ncell * sizeof(int), st));
-            k_bin_count<<<blocks_for(n, 256), 256, 0, st>>>(M, g, field[b], n, cnt);
+            OV_CUDA(cudaMemsetAsync(cnt[b], 0, (ncell[b] + 1) * sizeof(int), st));
+            OV_CUDA(cudaMemsetAsync(fill[b], 0, ncell[b] * sizeof(int), st));
+            k_bin_count<<<blocks_for(n, 256), 256, 0, st>>>(M, P.grid[b], field[b], n, cnt[b]);
             OV_CUDA(cudaGetLastError());
-            size_t tmp_bytes = 0;
-            void* tmp = nullptr;
-            OV_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tmp_bytes, cnt, start[b], (int)(ncell + 1), st));
-            OV_CUDA(buf.get((char**)&tmp, tmp_bytes));
-            OV_CUDA(cub::DeviceScan::ExclusiveSum(tmp, tmp_bytes, cnt, start[b], (int)(ncell + 1), st));
-            int total = 0;
-            OV_CUDA(cudaMemcpyAsync(&total, start[b] + ncell, sizeof(int), cudaMemcpyDeviceToHost, st));
-            OV_CUDA(cudaStreamSynchronize(st));
-            OV_CUDA(buf.get(&items[b], (size_t)total));
-            k_bin_fill<<<blocks_for(n, 256), 256, 0, st>>>(M, g, field[b], n, start[b], fill, items[b]);
+            OV_CUDA(cub::DeviceScan::ExclusiveSum(tmp[b], tmp_bytes[b], cnt[b], start[b], (int)(ncell[b] + 1), st));
+            OV_CUDA(cudaMemcpyAsync(&total[b], start[b] + ncell[b], sizeof(int), cudaMemcpyDeviceToHost, st));
+        }
+        OV_CUDA(cudaStreamSynchronize(st));
+        buf.base = nullptr;
+        buf.used = 0;
+        for (int pass = 0; pass < 2; pass++) {
+            if (pass) OV_CUDA(buf.alloc());
+            for (int b = 0; b < 2; b++) buf.take(&items[b], (size_t)total[b]);
+        }
+        for (int b = 0; b < 2; b++) {
+            const int n = bins[b].nfield;
+            if (n == 0) continue;
+            k_bin_fill<<<blocks_for(n, 256), 256, 0, st>>>(M, P.grid[b], field[b], n, start[b], fill[b], items[b]);
             OV_CUDA(cudaGetLastError());
             bins[b].start = start[b];
             bins[b].items = items[b];
@@ -418,18 +434,21 @@ extern "C" int hp_overset_hole_cut_gpu(const hp_mesh* mesh, const int32_t* block
         Buffers buf;
         OV_CUDA(buf.open());
         st = buf.st;
-        OV_CUDA(buf.get(&x, nodes));
-        OV_CUDA(buf.get(&y, nodes));
-        OV_CUDA(buf.get(&z, nodes));
-        OV_CUDA(buf.get(&elem, 9 * (size_t)neles));
-        OV_CUDA(buf.get(&blk, neles));
-        OV_CUDA(buf.get(&ib, neles));
-        OV_CUDA(buf.get(&cnt, 1));
-        OV_CUDA(buf.get(&tri, HP.tri.size()));
-        OV_CUDA(buf.get(&s3, HP.start3.size()));
-        OV_CUDA(buf.get(&i3, HP.items3.size()));
-        OV_CUDA(buf.get(&s2, HP.start2.size()));
-        OV_CUDA(buf.get(&i2, HP.items2.size()));
+        for (int pass = 0; pass < 2; pass++) {
+            if (pass) OV_CUDA(buf.alloc());
+            buf.take(&x, nodes);
+            buf.take(&y, nodes);
+            buf.take(&z, nodes);
+            buf.take(&elem, 9 * (size_t)neles);
+            buf.take(&blk, neles);
+            buf.take(&ib, neles);
+            buf.take(&cnt, 1);
+            buf.take(&tri, HP.tri.size());
+            buf.take(&s3, HP.start3.size());
+            buf.take(&i3, HP.items3.size());
+            buf.take(&s2, HP.start2.size());
+            buf.take(&i2, HP.items2.size());
+        }
         OV_CUDA(cudaMemcpyAsync(x, mesh->x, nodes * sizeof(double), cudaMemcpyHostToDevice, st));
         OV_CUDA(cudaMemcpyAsync(y, mesh->y, nodes * sizeof(double), cudaMemcpyHostToDevice, st));
         OV_CUDA(cudaMemcpyAsync(z, mesh->z, nodes * sizeof(double), cudaMemcpyHostToDevice, st));
