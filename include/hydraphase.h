@@ -318,7 +318,8 @@ int hp_output_wait(hp_handle *h, int32_t ticket);
 /* --- serving many cases ---------------------------------------------------- */
 /* No counterpart in the reference, which runs one case per process.  Device
  * bytes hp_create would allocate for this mesh and precision (admission
- * against an HBM budget before creating). */
+ * against an HBM budget before creating).  elem and ghost may be null: an
+ * upper bound from the sizes alone. */
 int hp_estimate_bytes(const hp_mesh *mesh, const hp_params *params, int64_t *bytes);
 /* Host threads of the set-up loops (geometry, least-squares tables, cell
  * order) that hp_create runs on the calling thread; 0 = one per core.  A

@@ -16,7 +16,7 @@
 
 namespace hp {
 
-enum { NEQ = 10, NPR = 14, NGR = 33, NLSQ = 16 };
+enum { NEQ = 10, NPR = 14, NGR = 33, NLSQ = 16, NLSQB = 12 };
 
 // primitive columns (the reference's ug,vg,wg,tg,pg,pp,phig,phip,up,vp,wp,
 // tp,rog,rop of src/mod_GlobalVariables.F90:13)
@@ -40,10 +40,11 @@ enum { G_UG = 0, G_VG = 3, G_WG = 6, G_TG = 9, G_UP = 12, G_VP = 15,
 // face kind bits per cell, 4 bits per face: bit 0 = wall (ghost type 5),
 // bit 1 = MUSCL-reconstruct across the face (interior or partition ghost).
 enum { FK_WALL = 1, FK_RECON = 2 };
-// cell bits of the same word, set by the host where a least-squares weight,
-// determinant or centroid difference of the cell lies outside the range in
-// which the kernels' shared-reciprocal division is exact (LSQA, LSQB tables)
-enum { FK_LSQA_RANGE = 1 << 16, FK_LSQB_RANGE = 1 << 17 };
+// cell bits of the same word, set at set-up where a least-squares weight,
+// determinant or centroid difference of the cell (LSQA, LSQB tables), or the
+// area or area vector of a face, lies outside the range in which the kernels'
+// shared-reciprocal division is exact
+enum { FK_LSQA_RANGE = 1 << 16, FK_LSQB_RANGE = 1 << 17, FK_AREA_RANGE = 1 << 18 };
 
 struct DevParams {
     double gamag, gamap, pinf, cpp, cpg, prg, rrg, prp;
@@ -79,24 +80,27 @@ struct DevMesh {
     // once at set-up with the host's pow, as the reference evaluates it
     const double* eps2;     // [ld]
     const double* sc;       // [12][ld] face area vectors sc1x..sc4z
-    // face centroids (0.3333 factor: HLLC, VK) minus the cell's centroid and
-    // minus the centroid of the face's neighbour: x of faces 1-4, then y, z
-    const double *fxo, *fxn;   // [12][ld]
-    // unit normal (x, y, z) and area of face 1, then 2, 3, 4; formed on the
-    // device by the variant that reads them (Variant::setup), null when the
-    // handle runs no FP64 flux kernel
+    const double* fch;      // [12][ld] face centroids, 0.3333 factor (HLLC, VK): x of faces 1-4, then y, z
+    const double* fxo;      // [12][ld] the same minus the cell's centroid (FP64 gradients, else null)
+    // face areas or, for the Jameson flux, unit normal (x, y, z) and area of
+    // face 1, then 2, 3, 4; formed on the device by the variant that reads them
+    // (Variant::setup), null when the handle runs no FP64 flux kernel
+    const double* area;     // [4][ld]
     const double* nrm;      // [16][ld]
-    const double* fcv;      // [12][ld] face centroids, /3 (viscous)
+    const double* fcv;      // [12][ld] face centroids, /3 (viscous; null in inviscid handles)
     // geometry-only least-squares terms, evaluated once at set-up with the
     // reference's expressions: [0..3] weights, [4..9] a1 a2 a3 b1 b2 b3,
-    // [10] the determinant, [11..14] and [15] the correctly rounded
-    // reciprocals of the weights and of the determinant; LSQA for the 1/r^2
-    // cell gradients (src/sr_derivative.F90:163-176,255), LSQB for the 1/r
-    // gradient of alpha_g in the sources (src/sr_source.F90:100-117)
+    // [10] the determinant; LSQA for the 1/r^2 cell gradients
+    // (src/sr_derivative.F90:163-176,255), then the correctly rounded
+    // reciprocals of the weights ([11..14]) and of the determinant ([15]);
+    // LSQB for the 1/r gradient of alpha_g in the sources
+    // (src/sr_source.F90:100-117), then that of the determinant ([11])
     const double* dxn;      // [12][ld] centroid of neighbour f minus the
-                            // cell's (x, y, z of face 1, then 2, 3, 4)
+                            // cell's (x, y, z of face 1, then 2, 3, 4; FP64
+                            // gradients, else null)
+    // (null where nothing reads them: no FP64 kernels, no gradients)
     const double* lsqa;     // [NLSQ][ld]
-    const double* lsqb;     // [NLSQ][ld]
+    const double* lsqb;     // [NLSQB][ld]
     const int *g_par, *g_id, *g_type;   // [nghosts] ghost list (reference order)
     // overset fringe (nfringe = 0: none): cells, 4 donor cells each and
     // barycentric weights, [4][nfringe] column-major
@@ -181,9 +185,13 @@ struct DevState {
     R* agrad;                // [3][ld] 1/r-weighted gradient of alpha_g (the
                              // sources'), formed beside the others by the
                              // FP32 gradient kernel; null where that does not run
+    // switches and Laplacian of the smoothing passes, dead once d24 stands:
+    // they share the memory of vis (written by the viscous pass after them;
+    // inviscid handles, whose vis is zero, keep two columns for anu) and of
+    // cn1 (written by the first stage)
     double *anu, *d2q;       // [2][ld], [10][ld]
     double *d24, *vis;       // [10][ld], [8][ld]
-    double* egt;             // [2][ld] ghost egtotal/eptotal (aliased meshes)
+    double* egt;             // [2][ld] ghost egtotal/eptotal (aliased meshes, else null)
     // five-phase model only (null otherwise): cn, cu, cn1, d2q and d24 then
     // hold 22 columns
     double* qpr;             // [12][ld] phi, u, v, w of q, r, s
@@ -267,7 +275,7 @@ struct Variant {
     // 1 when the flux kernel of meshes with a face list recovers the next
     // stage's primitives (see recover_in_flux in hp_kernels.cuh)
     int flux_recovers;
-    // fills the tables that the flux kernels read (m.nrm), once per handle
+    // fills the tables that the flux kernels read (m.area, m.nrm), once per handle
     void (*setup)(const DevMesh&, cudaStream_t);
     // fused step (one cooperative launch per step): the grid it runs with on
     // this device (blocks of 128 threads), and the launch of one step

@@ -186,13 +186,19 @@ static void plan_arena(hp_handle* h, Arena& a, int neles, int nghosts, long long
     m.xc = (double*)a.take(ld * D); m.yc = (double*)a.take(ld * D); m.zc = (double*)a.take(ld * D);
     m.vol = (double*)a.take(ld * D); m.dl = (double*)a.take(ld * D); m.dd = (double*)a.take(ld * D);
     m.eps2 = (double*)a.take(ld * D);
-    m.sc = (double*)a.take(12 * ld * D); m.fxo = (double*)a.take(12 * ld * D);
-    m.fxn = (double*)a.take(12 * ld * D);
-    m.nrm = gb == D || h->nwall > 0 ? (double*)a.take(16 * ld * D) : nullptr;
-    m.fcv = (double*)a.take(12 * ld * D);
-    m.dxn = (double*)a.take(12 * ld * D);
-    m.lsqa = (double*)a.take(NLSQ * ld * D);
-    m.lsqb = (double*)a.take(NLSQ * ld * D);
+    // geometry tables of the FP64 gradients and fluxes (the wall layers' too);
+    // first order and the Jameson flux (myflux 3) have no gradients
+    const bool fp64 = gb == D || h->nwall > 0, grad = h->prm.myorder == 2 && h->prm.myflux != 3;
+    auto table = [&](bool read, int ncol) { return read ? (double*)a.take(ncol * (size_t)ld * D) : nullptr; };
+    m.sc = table(true, 12);
+    m.fch = table(true, 12);
+    m.fxo = table(fp64 && grad, 12);
+    m.dxn = table(fp64 && grad, 12);
+    m.nrm = table(fp64 && h->prm.myflux == 3, 16);
+    m.area = table(fp64 && h->prm.myflux != 3, 4);
+    m.fcv = table(!h->prm.inviscid, 12);
+    m.lsqa = table(fp64 && grad, NLSQ);
+    m.lsqb = table(fp64, NLSQB);
     m.g_par = (int*)a.take((nghosts + 1) * (size_t)I); m.g_id = (int*)a.take((nghosts + 1) * (size_t)I);
     m.g_type = (int*)a.take((nghosts + 1) * (size_t)I);
     DevState<double>& s = h->ds;
@@ -203,15 +209,16 @@ static void plan_arena(hp_handle* h, Arena& a, int neles, int nghosts, long long
     // for the FP32-arithmetic variants, the FP64 columns themselves otherwise
     s.prr = gb == D ? s.pr : (double*)a.take(NPR * ld * gb);
     s.gr = (double*)a.take(NGR * ld * gb); s.phi = (double*)a.take(ld * D);
-    s.anu = (double*)a.take(2 * ld * D); s.d2q = (double*)a.take(nq * ld * D);
     s.d24 = (double*)a.take(nq * ld * D); s.vis = (double*)a.take(8 * ld * D);
+    s.d2q = s.cn1;
+    s.anu = h->prm.inviscid ? (double*)a.take(2 * ld * D) : s.vis;
     if (h->neq == 22) {
         s.qpr = (double*)a.take(12 * ld * D); s.anuq = (double*)a.take(3 * ld * D);
         s.qdrag = (double*)a.take(9 * ld * D);
     } else {
         s.qpr = s.anuq = s.qdrag = nullptr;
     }
-    s.egt = (double*)a.take(2 * ld * D);
+    s.egt = h->aliased ? (double*)a.take(2 * ld * D) : nullptr;
     s.s = (DevScalars*)a.take(ncase * sizeof(DevScalars));
     s.diag = (double*)a.take((size_t)ncase * h->max_diag * 8 * D);
     s.max_diag = h->max_diag;
@@ -229,8 +236,8 @@ static void plan_arena(hp_handle* h, Arena& a, int neles, int nghosts, long long
     }
     m.dxnf = m.fxof = nullptr;
     s.agrad = nullptr;
-    if (gb != D && !h->aliased) {
-        s.agrad = (double*)a.take(3 * (size_t)ld * gb);   // (read by the mixed variant alone)
+    if (gb != D && !h->aliased && grad) {
+        if (h->prm.precision == HP_PREC_MIXED) s.agrad = (double*)a.take(3 * (size_t)ld * gb);
         m.dxnf = (const float*)a.take(12 * (size_t)ld * sizeof(float));
         m.fxof = (const float*)a.take(12 * (size_t)ld * sizeof(float));
     }
@@ -244,7 +251,7 @@ static void plan_arena(hp_handle* h, Arena& a, int neles, int nghosts, long long
         m.cface = (const int*)a.take(4 * (size_t)ld * I);
         m.f_j = (const int*)a.take((size_t)nface * I);
         m.fgeo = (const float*)a.take(9 * (size_t)m.fld * sizeof(float));
-        m.fgcv = (const double*)a.take(3 * (size_t)m.fld * D);
+        m.fgcv = h->prm.inviscid ? nullptr : (const double*)a.take(3 * (size_t)m.fld * D);
         s.ff = (double*)a.take((size_t)FACE_REC * (size_t)m.fld * gb);
         if (h->prm.face_mode >= 2) {   // colouring or atomics: per-cell face sums
             s.racc = (double*)a.take(10 * (size_t)ld * D);
@@ -275,7 +282,7 @@ struct Layout {
         gpar.assign(ng, 0); gid.assign(ng, 0); gtyp.assign(ng, 0); perm.assign(ne, 0); ghost_id.assign(ng, 0);
         for (auto* v : {&x, &y, &z, &vol, &dl, &dd, &eps2}) v->assign(ld, 0.0);
         for (auto* v : {&sc, &fch, &fcv}) v->assign(12 * ld, 0.0);
-        la.assign(NLSQ * ld, 0.0); lb.assign(NLSQ * ld, 0.0);
+        la.assign(NLSQ * ld, 0.0); lb.assign(NLSQB * ld, 0.0);
     }
 };
 
@@ -333,6 +340,30 @@ static void wall_layers(const Layout& L, int neles, int nghosts, long long ld, i
         }
         if (inner) cls[t] = 2;
     }
+}
+
+// Ghost slots that are elements, repeated, or ghost parents, or that elements
+// refer to but no ghost has.  (hp_estimate_* ask before the ids are validated:
+// ids out of range count as aliased.)
+static bool ghosts_aliased(const hp_mesh* mesh) {
+    const int neles = mesh->neles, ntot = neles + mesh->nghosts;
+    std::vector<char> seen((size_t)ntot + 1, 0);
+    for (int g = 0; g < mesh->nghosts; g++) {
+        const int id = mesh->ghost[4 * (size_t)g + 1];
+        if (id <= neles || id > ntot || seen[id]) return true;
+        seen[id] = 1;
+    }
+    for (int g = 0; g < mesh->nghosts; g++) {
+        const int par = mesh->ghost[4 * (size_t)g];
+        if (par < 1 || par > neles) return true;
+    }
+    // neighbours in the ghost range must be ghost slots that exist
+    for (long long e = 0; e < neles; e++)
+        for (int k = 4; k < 8; k++) {
+            const int j = mesh->elem[9 * e + k];
+            if (j < 1 || j > ntot || (j > neles && !seen[j])) return true;
+        }
+    return false;
 }
 
 // One case of a handle: validates its connectivity, computes its geometry
@@ -463,7 +494,7 @@ static int fill_case(const hp_mesh* mesh, const hp_params* params, Layout& L, Ca
         }
     }
     // --- static least-squares terms of the gradient and source operators ---
-    std::vector<double> lsqa(NLSQ * (size_t)(neles + 1), 0.0), lsqb(NLSQ * (size_t)(neles + 1), 0.0);
+    std::vector<double> lsqa(NLSQ * (size_t)(neles + 1), 0.0), lsqb(NLSQB * (size_t)(neles + 1), 0.0);
     auto LA = [&](int k, int i) -> double& { return lsqa[(size_t)k * (neles + 1) + i]; };
     auto LB = [&](int k, int i) -> double& { return lsqb[(size_t)k * (neles + 1) + i]; };
 #pragma omp parallel for schedule(static)
@@ -501,25 +532,9 @@ static int fill_case(const hp_mesh* mesh, const hp_params* params, Layout& L, Ca
         for (int f = 0; f < 4; f++) LB(f, i) = wb[f];
         LB(4, i) = a1; LB(5, i) = a2; LB(6, i) = a3; LB(7, i) = b1; LB(8, i) = b2; LB(9, i) = b3;
         LB(10, i) = det3(a1, b1, b2, b1, a2, b3, b2, b3, a3);
-        for (int f = 0; f < 4; f++) LB(11 + f, i) = 1.0 / wb[f];
-        LB(15, i) = 1.0 / LB(10, i);
+        LB(11, i) = 1.0 / LB(10, i);
     }
-    // --- aliasing: ghost slots that are elements, repeated, or ghost parents ---
-    {
-        std::vector<char> seen(ntot + 1, 0);
-        int al = 0;
-        for (int g = 0; g < nghosts && !al; g++) {
-            if (gid[g] <= neles || seen[gid[g]]) al = 1;
-            seen[gid[g]] = 1;
-        }
-        for (int g = 0; g < nghosts && !al; g++)
-            if (gpar[g] > neles || seen[gpar[g]]) al = 1;
-        // neighbours in the ghost range must be ghost slots that exist
-        for (int e = 1; e <= neles && !al; e++)
-            for (int k = 0; k < 4; k++)
-                if (nc[k][e] > neles && !seen[nc[k][e]]) { al = 1; break; }
-        cr.aliased = al;
-    }
+    cr.aliased = ghosts_aliased(mesh) ? 1 : 0;
     // --- internal order: space-filling curve over element centroids ---
     std::vector<int> perm(neles + 1);   // 1-based reference id -> 0-based internal
     std::iota(perm.begin(), perm.end(), -1);
@@ -632,7 +647,8 @@ static int fill_case(const hp_mesh* mesh, const hp_params* params, Layout& L, Ca
             for (int k = 0; k < 12; k++) {
                 hsc[k * ld + t] = SC(k, i); hfch[k * ld + t] = FCH(k, i); hfcv[k * ld + t] = FCV(k, i);
             }
-            for (int k = 0; k < NLSQ; k++) { hla[k * ld + t] = LA(k, i); hlb[k * ld + t] = LB(k, i); }
+            for (int k = 0; k < NLSQ; k++) hla[k * ld + t] = LA(k, i);
+            for (int k = 0; k < NLSQB; k++) hlb[k * ld + t] = LB(k, i);
         } else {
             for (int k = 0; k < 4; k++) { hnc[k * ld + t] = map(nc[k][i]); hsnb[k * ld + t] = map(nc[k][i]); }
         }
@@ -648,42 +664,50 @@ namespace {
 inline unsigned blocks_for(long long n, int b) { return (unsigned)((n + b - 1) / b); }
 
 // Set-up, one thread per cell: the neighbour centroid differences of the
-// gradient and source LSQ (m.dxn), the face centroids (in m.fxn on entry)
-// minus the centroids of both sides (m.fxo, m.fxn), the subtractions that the
-// step's kernels would do on gathered centroids; and the range bits of m.fk:
-// weights and determinants in [2^-100, 2^101), centroid differences zero or
-// in [2^-100, 2^100).
+// gradient LSQ (m.dxn), the face centroids minus the cell's own (m.fxo), and
+// float copies of both, the subtractions that the step's kernels would do; and
+// the range bits of m.fk: weights, determinants and face areas in [2^-100,
+// 2^101), centroid differences zero or in [2^-100, 2^100), components of area
+// vectors zero or at least 2^-800.
 __global__ void __launch_bounds__(128) k_offsets(DevMesh m) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= m.neles) return;
     const long long ld = m.ld;
-    double *dxn = const_cast<double*>(m.dxn), *fxo = const_cast<double*>(m.fxo), *fxn = const_cast<double*>(m.fxn);
     const double* x[3] = {m.xc, m.yc, m.zc};
     unsigned out = 0;
     for (int f = 0; f < 4; f++) {
         const int j = m.nc[f * ld + i];
         for (int d = 0; d < 3; d++) {
-            const double xi = x[d][i], xj = x[d][j], fc = fxn[(4 * d + f) * ld + i];
-            const double dx = xj - xi;
-            dxn[(3 * f + d) * ld + i] = dx;
-            fxo[(4 * d + f) * ld + i] = fc - xi;
-            fxn[(4 * d + f) * ld + i] = fc - xj;
+            const double dx = x[d][j] - x[d][i], fo = m.fch[(4 * d + f) * ld + i] - x[d][i];
+            if (m.dxn) {
+                const_cast<double*>(m.dxn)[(3 * f + d) * ld + i] = dx;
+                const_cast<double*>(m.fxo)[(4 * d + f) * ld + i] = fo;
+            }
+            if (m.dxnf) {
+                const_cast<float*>(m.dxnf)[(3 * f + d) * ld + i] = (float)dx;
+                const_cast<float*>(m.fxof)[(4 * d + f) * ld + i] = (float)fo;
+            }
             const double a = fabs(dx);
-            if (a != 0.0 && !(a >= 0x1p-100 && a < 0x1p100)) out = FK_LSQA_RANGE | FK_LSQB_RANGE;
+            if (a != 0.0 && !(a >= 0x1p-100 && a < 0x1p100)) out |= FK_LSQA_RANGE | FK_LSQB_RANGE;
         }
+    }
+    for (int f = 0; f < 4; f++) {
+        double a2 = 0.0;
+        for (int d = 0; d < 3; d++) {
+            const double a = fabs(m.sc[(3 * f + d) * ld + i]);
+            a2 += a * a;
+            if (a != 0.0 && !(a >= 0x1p-800)) out |= FK_AREA_RANGE;
+        }
+        const double area = sqrt(a2);
+        if (!(area >= 0x1p-100 && area < 0x1p101)) out |= FK_AREA_RANGE;
     }
     for (int t = 0; t < 5; t++) {
         const int k = t < 4 ? t : 10;
-        const double a = m.lsqa[k * ld + i], b = m.lsqb[k * ld + i];
+        const double a = m.lsqa ? m.lsqa[k * ld + i] : 1.0, b = m.lsqb ? m.lsqb[k * ld + i] : 1.0;
         if (!(a >= 0x1p-100 && a < 0x1p101)) out |= FK_LSQA_RANGE;
         if (!(b >= 0x1p-100 && b < 0x1p101)) out |= FK_LSQB_RANGE;
     }
     if (out) const_cast<unsigned*>(m.fk)[i] |= out;
-    if (m.dxnf)
-        for (int k = 0; k < 12; k++) {
-            const_cast<float*>(m.dxnf)[k * ld + i] = (float)dxn[k * ld + i];
-            const_cast<float*>(m.fxof)[k * ld + i] = (float)fxo[k * ld + i];
-        }
 }
 
 // Set-up, one thread per face: the face-ordered tables (after k_offsets).
@@ -693,12 +717,15 @@ __global__ void __launch_bounds__(128) k_face_tables(DevMesh m) {
     const long long ld = m.ld, fl = m.fld;
     const int i = m.f_i[t], f = m.f_code[t] & 3;
     float* g = const_cast<float*>(m.fgeo);
-    const_cast<int*>(m.f_j)[t] = m.nc[f * ld + i];
+    const int j = m.nc[f * ld + i];
+    const_cast<int*>(m.f_j)[t] = j;
+    const double* x[3] = {m.xc, m.yc, m.zc};
     for (int d = 0; d < 3; d++) {
+        const double fc = m.fch[(4 * d + f) * ld + i];
         g[d * fl + t] = (float)m.sc[(3 * f + d) * ld + i];
-        g[(3 + d) * fl + t] = (float)m.fxo[(4 * d + f) * ld + i];
-        g[(6 + d) * fl + t] = (float)m.fxn[(4 * d + f) * ld + i];
-        const_cast<double*>(m.fgcv)[d * fl + t] = m.fcv[(4 * d + f) * ld + i];
+        g[(3 + d) * fl + t] = (float)(fc - x[d][i]);
+        g[(6 + d) * fl + t] = (float)(fc - x[d][j]);
+        if (m.fgcv) const_cast<double*>(m.fgcv)[d * fl + t] = m.fcv[(4 * d + f) * ld + i];
     }
 }
 }  // namespace
@@ -955,11 +982,11 @@ extern "C" int hp_create_batch(const hp_mesh* meshes, int32_t ncase, const hp_pa
     if (e == cudaSuccess) e = up(m.eps2, L.eps2.data(), ld * D);
     if (e == cudaSuccess) e = up(m.dd, L.dd.data(), ld * D);
     if (e == cudaSuccess) e = up(m.sc, L.sc.data(), 12 * ld * D);
-    if (e == cudaSuccess) e = up(m.fcv, L.fcv.data(), 12 * ld * D);
-    if (e == cudaSuccess) e = up(m.lsqa, L.la.data(), NLSQ * ld * D);
-    if (e == cudaSuccess) e = up(m.lsqb, L.lb.data(), NLSQ * ld * D);
+    if (e == cudaSuccess && m.fcv) e = up(m.fcv, L.fcv.data(), 12 * ld * D);
+    if (e == cudaSuccess && m.lsqa) e = up(m.lsqa, L.la.data(), NLSQ * ld * D);
+    if (e == cudaSuccess && m.lsqb) e = up(m.lsqb, L.lb.data(), NLSQB * ld * D);
     if (e == cudaSuccess) e = up(m.fk, L.fk.data(), ld * sizeof(unsigned));
-    if (e == cudaSuccess) e = up(m.fxn, L.fch.data(), 12 * ld * D);
+    if (e == cudaSuccess) e = up(m.fch, L.fch.data(), 12 * ld * D);
     if (e == cudaSuccess && nghosts) e = up(m.g_par, L.gpar.data(), nghosts * (size_t)I);
     if (e == cudaSuccess && nghosts) e = up(m.g_id, L.gid.data(), nghosts * (size_t)I);
     if (e == cudaSuccess && nghosts) e = up(m.g_type, L.gtyp.data(), nghosts * (size_t)I);
@@ -1580,44 +1607,37 @@ extern "C" int hp_dtmin_ptr(hp_handle* h, uint64_t** bits) {
 }
 
 extern "C" int hp_estimate_bytes(const hp_mesh* mesh, const hp_params* params, int64_t* bytes) {
-    if (!mesh || !params || !bytes || mesh->neles <= 0 || mesh->nghosts < 0) return HP_E_ARG;
-    hp_handle probe_h;
-    const long long ld = ((long long)mesh->neles + mesh->nghosts + 63) / 64 * 64;
-    const size_t gb = (params->precision == HP_PREC_MIXED || params->precision == HP_PREC_FP32) ? sizeof(float)
-                                                                                                : sizeof(double);
-    Arena probe;
-    const int nface = gb == sizeof(double) || params->face_mode == 1 ? 0
-                                                                      : (int)((4LL * mesh->neles + mesh->nghosts) / 2);
-    probe_h.neq = params->five_phase ? 22 : 10;
-    probe_h.prm.face_mode = params->face_mode;
-    if (gb != sizeof(double) && params->wall_fp64_layers > 0)   // bound: every cell in the layers
-        probe_h.nwall = probe_h.ngwall = mesh->neles;
-    plan_arena(&probe_h, probe, mesh->neles, mesh->nghosts, ld, gb, 1, nface);
-    *bytes = (int64_t)(probe.used + 256);
-    return HP_OK;
+    return hp_estimate_batch_bytes(mesh, 1, params, bytes);
 }
 
 extern "C" int hp_estimate_batch_bytes(const hp_mesh* meshes, int32_t ncase, const hp_params* params,
                                        int64_t* bytes) {
     if (!meshes || !params || !bytes || ncase < 1) return HP_E_ARG;
     long long ne = 0, ng = 0;
+    bool sizes_only = false;
+    hp_handle probe_h;
+    probe_h.prm = *params;
     for (int c = 0; c < ncase; c++) {
         if (meshes[c].neles <= 0 || meshes[c].nghosts < 0) return HP_E_ARG;
         ne += meshes[c].neles;
         ng += meshes[c].nghosts;
+        if (!meshes[c].elem || (meshes[c].nghosts > 0 && !meshes[c].ghost)) sizes_only = true;
+        else if (ghosts_aliased(meshes + c)) probe_h.aliased = 1;
     }
-    hp_handle probe_h;
     const long long ld = (ne + ng + 63) / 64 * 64;
     const size_t gb = (params->precision == HP_PREC_MIXED || params->precision == HP_PREC_FP32) ? sizeof(float)
                                                                                                 : sizeof(double);
-    Arena probe;
-    const int nface = gb == sizeof(double) || params->face_mode == 1 ? 0 : (int)((4 * ne + ng) / 2);
     probe_h.neq = params->five_phase ? 22 : 10;
-    probe_h.prm.face_mode = params->face_mode;
     if (gb != sizeof(double) && params->wall_fp64_layers > 0)   // bound: every cell in the layers
         probe_h.nwall = probe_h.ngwall = (int)ne;
-    plan_arena(&probe_h, probe, (int)ne, (int)ng, ld, gb, ncase, nface);
-    *bytes = (int64_t)(probe.used + 256);
+    *bytes = 0;
+    for (int pass = 0; pass < (sizes_only ? 2 : 1); pass++) {   // sizes alone: the larger of both kinds of ghosts
+        if (pass) probe_h.aliased = !probe_h.aliased;
+        const bool faces = gb != sizeof(double) && params->face_mode != 1 && !probe_h.aliased;
+        Arena probe;
+        plan_arena(&probe_h, probe, (int)ne, (int)ng, ld, gb, ncase, faces ? (int)((4 * ne + ng) / 2) : 0);
+        *bytes = std::max(*bytes, (int64_t)(probe.used + 256));
+    }
     return HP_OK;
 }
 

@@ -82,11 +82,6 @@ template <class T> __device__ __forceinline__ T ldg(const T* p) { return __ldg(p
 #endif
 // viscous fluxes of the cell-centric variants with eight lanes per cell (one
 // phase each, k_visc8) instead of four (k_visc4)
-// FP64 four-lane kernels: neighbour centroid differences from the set-up
-// table m.dxn instead of gathered centroids
-#ifndef HP_DXN_TABLE
-#define HP_DXN_TABLE 1
-#endif
 #ifndef HP_VISC_SPLIT
 #define HP_VISC_SPLIT 1
 #endif
@@ -1006,7 +1001,7 @@ __device__ __forceinline__ void k_grad_body(DevMesh m, DevState<R> s, DevParams 
     int n[4];
 #pragma unroll
     for (int f = 0; f < 4; f++) n[f] = ldg(COL(m.nc, f) + i);
-    // centroid differences from the set-up tables (the same subtractions)
+    // FPR: centroid differences from the set-up table (the same subtractions)
     R xa[4], ya[4], za[4];
 #pragma unroll
     for (int f = 0; f < 4; f++) {
@@ -1015,9 +1010,9 @@ __device__ __forceinline__ void k_grad_body(DevMesh m, DevState<R> s, DevParams 
             ya[f] = (R)ldg(COL(m.dxnf, 3 * f + 1) + i);
             za[f] = (R)ldg(COL(m.dxnf, 3 * f + 2) + i);
         } else {
-            xa[f] = (R)ldg(COL(m.dxn, 3 * f) + i);
-            ya[f] = (R)ldg(COL(m.dxn, 3 * f + 1) + i);
-            za[f] = (R)ldg(COL(m.dxn, 3 * f + 2) + i);
+            xa[f] = (R)(ldg(m.xc + n[f]) - ldg(m.xc + i));
+            ya[f] = (R)(ldg(m.yc + n[f]) - ldg(m.yc + i));
+            za[f] = (R)(ldg(m.zc + n[f]) - ldg(m.zc + i));
         }
     }
     // geometry-only terms (wt, a1..b3, dnr of src/sr_derivative.F90:163-176,
@@ -1103,9 +1098,9 @@ __device__ __forceinline__ void k_grad_body(DevMesh m, DevState<R> s, DevParams 
             fy[f] = (R)ldg(COL(m.fxof, 4 + f) + i);
             fz[f] = (R)ldg(COL(m.fxof, 8 + f) + i);
         } else {
-            fx[f] = (R)ldg(COL(m.fxo, f) + i);
-            fy[f] = (R)ldg(COL(m.fxo, 4 + f) + i);
-            fz[f] = (R)ldg(COL(m.fxo, 8 + f) + i);
+            fx[f] = (R)(ldg(COL(m.fch, f) + i) - ldg(m.xc + i));
+            fy[f] = (R)(ldg(COL(m.fch, 4 + f) + i) - ldg(m.yc + i));
+            fz[f] = (R)(ldg(COL(m.fch, 8 + f) + i) - ldg(m.zc + i));
         }
     }
     const int lv[4] = {8, 9, 11, 12};   // pg, pp, rog, rop rows of gv
@@ -1316,14 +1311,27 @@ __device__ __forceinline__ void face_eval(const DevMesh& m, const DevState<R>& s
 #define FGEO(k) (R)ldg(m.fgeo + (size_t)(k) * m.fld + t)
     const int neigh = LIST ? ldg(m.f_j + t) : ldg(COL(m.nc, f) + i);
     const unsigned kind = (ldg(m.fk + i) >> (4 * f)) & 0xFu;
-    // FP64: unit normal and area from the set-up table; FP32: formed here,
-    // where its approximate divisions cost little
+    // area and unit normal
     R area, enx, eny, enz;
-    if constexpr (sizeof(R) == 8) {
+    if constexpr (sizeof(R) == 8 && Z == 2) {
+        // the Jameson flux has little else to do, and its handles have no
+        // gradient tables (formed here: 1694 -> 1719 us, 983,040 cells, four
+        // launches)
         enx = ldg(COL(m.nrm, 4 * f) + i);
         eny = ldg(COL(m.nrm, 4 * f + 1) + i);
         enz = ldg(COL(m.nrm, 4 * f + 2) + i);
         area = ldg(COL(m.nrm, 4 * f + 3) + i);
+    } else if constexpr (sizeof(R) == 8) {
+        // the area from a set-up table, and one reciprocal for the three
+        // quotients (ranges tested at set-up).  The normals as a table too, 96
+        // B a cell, would take 23 us off three launches of 1976 (983,040
+        // cells).
+        const R scx = ldg(COL(m.sc, 3 * f) + i), scy = ldg(COL(m.sc, 3 * f + 1) + i), scz = ldg(COL(m.sc, 3 * f + 2) + i);
+        area = ldg(COL(m.area, f) + i);
+        const R rarea = F == 0 ? R(0) : R(1) / area;
+        enx = mquo<F>(scx, area, rarea);
+        eny = mquo<F>(scy, area, rarea);
+        enz = mquo<F>(scz, area, rarea);
     } else {
         const R scx = LIST ? FGEO(0) : (R)ldg(COL(m.sc, 3 * f) + i), scy = LIST ? FGEO(1) : (R)ldg(COL(m.sc, 3 * f + 1) + i),
                 scz = LIST ? FGEO(2) : (R)ldg(COL(m.sc, 3 * f + 2) + i);
@@ -1422,12 +1430,18 @@ __device__ __forceinline__ void face_eval(const DevMesh& m, const DevState<R>& s
     }
     if (P.myorder == 2 && (kind & FK_RECON)) {
         const R phimin = (R)mn2(PLD(s.phi + i), PLD(s.phi + neigh));
-        // face centroid minus each side's centroid (set-up tables: the
-        // neighbour's centroid would be three more gathers)
-        const R xf0 = LIST ? FGEO(3) : (R)ldg(COL(m.fxo, f) + i), yf0 = LIST ? FGEO(4) : (R)ldg(COL(m.fxo, 4 + f) + i),
-                zf0 = LIST ? FGEO(5) : (R)ldg(COL(m.fxo, 8 + f) + i);
-        const R xfn = LIST ? FGEO(6) : (R)ldg(COL(m.fxn, f) + i), yfn = LIST ? FGEO(7) : (R)ldg(COL(m.fxn, 4 + f) + i),
-                zfn = LIST ? FGEO(8) : (R)ldg(COL(m.fxn, 8 + f) + i);
+        // face centroid minus each side's centroid.  (Tables of both
+        // differences in place of the gathered centroids: 983,040 cells, FP64,
+        // three launches, 1995 us against 1974.)
+        R xf0, yf0, zf0, xfn, yfn, zfn;
+        if constexpr (LIST) {
+            xf0 = FGEO(3); yf0 = FGEO(4); zf0 = FGEO(5);
+            xfn = FGEO(6); yfn = FGEO(7); zfn = FGEO(8);
+        } else {
+            const double xf = ldg(COL(m.fch, f) + i), yf = ldg(COL(m.fch, 4 + f) + i), zf = ldg(COL(m.fch, 8 + f) + i);
+            xf0 = (R)(xf - ldg(m.xc + i)); yf0 = (R)(yf - ldg(m.yc + i)); zf0 = (R)(zf - ldg(m.zc + i));
+            xfn = (R)(xf - ldg(m.xc + neigh)); yfn = (R)(yf - ldg(m.yc + neigh)); zfn = (R)(zf - ldg(m.zc + neigh));
+        }
 #undef FGEO
         const R* g = s.gr;
 #define REC(v, X, Y, Z, G, c) \
@@ -1980,7 +1994,7 @@ __device__ __forceinline__ unsigned grad4_limiter(const DevMesh& m, const DevSta
 #ifndef HP_GRAD4_STAGE
 #define HP_GRAD4_STAGE 0
 #endif
-#define GRAD4_STAGED (HP_GRAD4_STAGE && HP_DXN_TABLE && HP_LSQ_TABLE)
+#define GRAD4_STAGED (HP_GRAD4_STAGE && HP_LSQ_TABLE)
 enum { GEO_N = 28, GEO_LD = 32 };
 struct Grad4Stage {
     const double* geo;    // geo[k * GEO_LD], k < 12 centroid differences, 12 + j LSQA column j
@@ -2069,22 +2083,13 @@ __device__ __forceinline__ unsigned grad4_body(const DevMesh& m, const DevState<
     }
 #endif
     (void)st;
-#if !HP_DXN_TABLE
     const double x0 = ldg(m.xc + i), y0 = ldg(m.yc + i), z0 = ldg(m.zc + i);
-#endif
     R xa[4], ya[4], za[4];
 #pragma unroll
     for (int f = 0; f < 4; f++) {
-#if HP_DXN_TABLE
-        // the centroid differences, formed at set-up (the same subtraction)
-        xa[f] = (R)ldg(COL(m.dxn, 3 * f) + i);
-        ya[f] = (R)ldg(COL(m.dxn, 3 * f + 1) + i);
-        za[f] = (R)ldg(COL(m.dxn, 3 * f + 2) + i);
-#else
         xa[f] = (R)(ldg(m.xc + n[f]) - x0);
         ya[f] = (R)(ldg(m.yc + n[f]) - y0);
         za[f] = (R)(ldg(m.zc + n[f]) - z0);
-#endif
     }
     // geometry-only terms (wt, a1..b3, dnr of src/sr_derivative.F90:163-176,
     // 255), evaluated once at set-up with the same expressions
@@ -2231,13 +2236,13 @@ __global__ void __launch_bounds__(128, HP_GRAD4_MINB) k_grad4(DevMesh m, DevStat
     k_grad4_body<LIST>(m, s, P, blockIdx.x);
 }
 
-// Columns of the tail prefetch: dl, vol, the 16 LSQB terms, vis, d24, cu
+// Columns of the tail prefetch: dl, vol, the 12 LSQB terms, vis, d24, cu
 // and cn; TAIL_LD cells (one 128-thread block) per column.  (Staging the 14
 // primitives and the 12 centroid differences as well measured 2% slower:
 // the face evaluation has just read the primitives.)
 enum { FLUX4_T = 128 };   // threads of the four-lane flux kernel's blocks
-enum { TAIL_DL = 0, TAIL_VOL = 1, TAIL_LSQB = 2, TAIL_VIS = 18, TAIL_D24 = 26, TAIL_CU = 36, TAIL_CN = 46,
-       TAIL_N = 56, TAIL_LD = 32 };
+enum { TAIL_DL = 0, TAIL_VOL = 1, TAIL_LSQB = 2, TAIL_VIS = TAIL_LSQB + NLSQB, TAIL_D24 = TAIL_VIS + 8,
+       TAIL_CU = TAIL_D24 + 10, TAIL_CN = TAIL_CU + 10, TAIL_N = TAIL_CN + 10, TAIL_LD = 32 };
 __device__ __forceinline__ const double* tail_col(const DevMesh& m, const DevState<R>& s, int k) {
     if (k == TAIL_DL) return m.dl;
     if (k == TAIL_VOL) return m.vol;
@@ -2293,12 +2298,7 @@ __device__ __forceinline__ bool flux4_body(const DevMesh& m, const DevState<R>& 
     // neighbour data for the alpha_g gradient of the sources
     const int nq = ldg(COL(m.nc, q) + i);
     const double x0 = ldg(m.xc + i), y0 = ldg(m.yc + i), z0 = ldg(m.zc + i);
-#if HP_DXN_TABLE
-    const R xq = (R)ldg(COL(m.dxn, 3 * q) + i), yq = (R)ldg(COL(m.dxn, 3 * q + 1) + i),
-            zq = (R)ldg(COL(m.dxn, 3 * q + 2) + i);
-#else
     const R xq = (R)(ldg(m.xc + nq) - x0), yq = (R)(ldg(m.yc + nq) - y0), zq = (R)(ldg(m.zc + nq) - z0);
-#endif
     // alpha_g differences from the FP64 primitives (see k_grad)
     const R pq = (R)(PCOL(s.pr, P_PHIG)[po(nq)] - PCOL(s.pr, P_PHIG)[po(i)]);
     // residual of this lane's variables j = q, q + 4, q + 8 in face order 1..4
@@ -2325,11 +2325,6 @@ __device__ __forceinline__ bool flux4_body(const DevMesh& m, const DevState<R>& 
                 rhs[r] = rhs[r] + (S)((fl[f] & 1) ? v : cur);
             }
         }
-    }
-    R xa[4], ya[4], za[4], pa[4];
-#pragma unroll
-    for (int f = 0; f < 4; f++) {
-        xa[f] = qshfl(xq, f); ya[f] = qshfl(yq, f); za[f] = qshfl(zq, f); pa[f] = qshfl(pq, f);
     }
     // interphase sources (src/sr_source.F90:46-155)
     {
@@ -2370,21 +2365,27 @@ __device__ __forceinline__ bool flux4_body(const DevMesh& m, const DevState<R>& 
         const R uint_ = qshfl(vq_int, 0), vint = qshfl(vq_int, 1), wint = qshfl(vq_int, 2);
         // geometry-only terms (src/sr_source.F90:100-117), evaluated (and
         // their ranges tested) at set-up
-        R wt[4], rw[4];
 #undef DW
 #if HP_LSQ_TABLE
-#define DW(x, f) mquo<F>((x), wt[f], rw[f])
 #define LB(k) TL(TAIL_LSQB + (k), ldg(COL(m.lsqb, k) + i))
-        if (F != 0) bad |= ldg(m.fk + i) & FK_LSQB_RANGE;
-#pragma unroll
-        for (int f = 0; f < 4; f++) {
-            mout<F, -800, 700>(pa[f], bad);
-            wt[f] = LB(f);
-            rw[f] = LB(11 + f);
-        }
+        if (F != 0) bad |= ldg(m.fk + i) & (FK_LSQB_RANGE | FK_AREA_RANGE);
+        // face q's three quotients, by one reciprocal of its weight; every lane
+        // then sums them over the faces
+        mout<F, -800, 700>(pq, bad);
+        const R wq = LB(q), rwq = F == 0 ? R(0) : R(1) / wq;
+        const R tx = mquo<F>(pq * xq, wq, rwq), ty = mquo<F>(pq * yq, wq, rwq), tz = mquo<F>(pq * zq, wq, rwq);
+        const R c1 = qshfl(tx, 0) + qshfl(tx, 1) + qshfl(tx, 2) + qshfl(tx, 3);
+        const R c2 = qshfl(ty, 0) + qshfl(ty, 1) + qshfl(ty, 2) + qshfl(ty, 3);
+        const R c3 = qshfl(tz, 0) + qshfl(tz, 1) + qshfl(tz, 2) + qshfl(tz, 3);
         const R a1 = LB(4), a2 = LB(5), a3 = LB(6);
         const R b1 = LB(7), b2 = LB(8), b3 = LB(9);
+        const R dnr = LB(10);
 #else
+        R xa[4], ya[4], za[4], pa[4], wt[4], rw[4];
+#pragma unroll
+        for (int f = 0; f < 4; f++) {
+            xa[f] = qshfl(xq, f); ya[f] = qshfl(yq, f); za[f] = qshfl(zq, f); pa[f] = qshfl(pq, f);
+        }
 #define DW(x, f) mdiv<F>((x), wt[f], rw[f], bad)
 #pragma unroll
         for (int f = 0; f < 4; f++) { wt[f] = sqrt(xa[f] * xa[f] + ya[f] * ya[f] + za[f] * za[f]); rw[f] = mrcp<F>(wt[f], bad); }
@@ -2394,24 +2395,20 @@ __device__ __forceinline__ bool flux4_body(const DevMesh& m, const DevState<R>& 
         const R b1 = DW(xa[0] * ya[0], 0) + DW(xa[1] * ya[1], 1) + DW(xa[2] * ya[2], 2) + DW(xa[3] * ya[3], 3);
         const R b2 = DW(xa[0] * za[0], 0) + DW(xa[1] * za[1], 1) + DW(xa[2] * za[2], 2) + DW(xa[3] * za[3], 3);
         const R b3 = DW(ya[0] * za[0], 0) + DW(ya[1] * za[1], 1) + DW(ya[2] * za[2], 2) + DW(ya[3] * za[3], 3);
-#endif
-#if HP_LSQ_TABLE
-        const R dnr = LB(10);
-#else
         const R dnr = det3(a1, b1, b2, b1, a2, b3, b2, b3, a3);
-#endif
         R dir[4];
 #pragma unroll
         for (int f = 0; f < 4; f++) dir[f] = q == 0 ? xa[f] : (q == 1 ? ya[f] : za[f]);
         const R cq = DW(pa[0] * dir[0], 0) + DW(pa[1] * dir[1], 1) + DW(pa[2] * dir[2], 2) + DW(pa[3] * dir[3], 3);
         const R c1 = qshfl(cq, 0), c2 = qshfl(cq, 1), c3 = qshfl(cq, 2);
+#endif
         // Cramer: lane 0 replaces the first column by c, lane 1 the second,
         // lane 2 the third
         const R A11 = q == 0 ? c1 : a1, A21 = q == 0 ? c2 : b1, A31 = q == 0 ? c3 : b2;
         const R A12 = q == 1 ? c1 : b1, A22 = q == 1 ? c2 : a2, A32 = q == 1 ? c3 : b3;
         const R A13 = q >= 2 ? c1 : b2, A23 = q >= 2 ? c2 : b3, A33 = q >= 2 ? c3 : a3;
 #if HP_LSQ_TABLE
-        const R rdnr = LB(15);
+        const R rdnr = LB(11);
 #undef LB
         const R dq = star_quo<F>(det3(A11, A21, A31, A12, A22, A32, A13, A23, A33), dnr, rdnr, bad);
 #else
@@ -2502,7 +2499,7 @@ __device__ __forceinline__ void k_flux4_body(DevMesh m, DevState<R> s, DevParams
     bool active = valid && ldg(m.iblank + i) == 1;
     if (sizeof(R) != sizeof(double) && m.nwall > 0) active = active && !ldg(m.wclass + i);
     __shared__ __align__(16) R sres[10 * FLUX4_T];
-#if HP_FLUX4_PREFETCH && HP_LSQ_TABLE && HP_DXN_TABLE
+#if HP_FLUX4_PREFETCH && HP_LSQ_TABLE
     if constexpr (NC && sizeof(R) == sizeof(double)) {
         // start the asynchronous copy of the values that the sources and the
         // RK update read (TAIL_*) while the faces are evaluated: for all
@@ -3253,22 +3250,26 @@ __global__ void __launch_bounds__(128) k_qrs_flux(DevMesh m, DevState<R> s, DevP
     }
 }
 
-// Set-up: unit normals and areas of the cells' faces (m.nrm), by the
-// expressions that the flux kernel would otherwise evaluate per face and
-// stage, compiled with the same flags.
-__global__ void __launch_bounds__(128) k_face_normals(DevMesh m) {
+// Set-up: areas of the cells' faces (m.area) or areas and unit normals (m.nrm,
+// Jameson flux), by the expressions that the flux kernel would otherwise
+// evaluate per face and stage, compiled with the same flags.
+__global__ void __launch_bounds__(128) k_face_areas(DevMesh m) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= m.neles) return;
-    double* out = const_cast<double*>(m.nrm);
 #pragma unroll
     for (int f = 0; f < 4; f++) {
         const double scx = ldg(COL(m.sc, 3 * f) + i), scy = ldg(COL(m.sc, 3 * f + 1) + i),
                      scz = ldg(COL(m.sc, 3 * f + 2) + i);
         const double area = sqrt(scx * scx + scy * scy + scz * scz);
-        COL(out, 4 * f)[i] = scx / area;
-        COL(out, 4 * f + 1)[i] = scy / area;
-        COL(out, 4 * f + 2)[i] = scz / area;
-        COL(out, 4 * f + 3)[i] = area;
+        if (m.nrm) {
+            double* out = const_cast<double*>(m.nrm);
+            COL(out, 4 * f)[i] = scx / area;
+            COL(out, 4 * f + 1)[i] = scy / area;
+            COL(out, 4 * f + 2)[i] = scz / area;
+            COL(out, 4 * f + 3)[i] = area;
+        } else {
+            COL(const_cast<double*>(m.area), f)[i] = area;
+        }
     }
 }
 
@@ -3277,7 +3278,7 @@ static inline unsigned grid_for(long long n, int block) {
 }
 
 static void setup(const DevMesh& m, cudaStream_t st) {
-    if (m.nrm) k_face_normals<<<grid_for(m.neles, 128), 128, 0, st>>>(m);
+    if (m.area || m.nrm) k_face_areas<<<grid_for(m.neles, 128), 128, 0, st>>>(m);
 }
 
 #define MARK(k) do { if (hook && hook->mark) hook->mark(hook->ctx, (k)); } while (0)

@@ -148,8 +148,8 @@ def write_tecplot(path: str, mesh: MeshArrays, fields: np.ndarray):
 
 def estimate_batch_bytes(meshes, params: HpParams) -> int:
     """Device bytes a Batch of these meshes would hold."""
-    arr = (HpMesh * len(meshes))(*[HpMesh(m.nodes, m.neles, m.nghosts, 0, None, None, None, None, None)
-                                   for m in meshes])
+    keep = []
+    arr = (HpMesh * len(meshes))(*[_hp_mesh(m, keep) for m in meshes])
     b = ctypes.c_int64()
     _check(lib().hp_estimate_batch_bytes(arr, len(meshes), ctypes.byref(params), ctypes.byref(b)))
     return int(b.value)
@@ -157,7 +157,8 @@ def estimate_batch_bytes(meshes, params: HpParams) -> int:
 
 def estimate_bytes(mesh: MeshArrays, params: HpParams) -> int:
     """Device bytes a Case of this mesh and precision would hold."""
-    hm = HpMesh(mesh.nodes, mesh.neles, mesh.nghosts, 0, None, None, None, None, None)
+    keep = []
+    hm = _hp_mesh(mesh, keep)
     b = ctypes.c_int64()
     _check(lib().hp_estimate_bytes(ctypes.byref(hm), ctypes.byref(params), ctypes.byref(b)))
     return int(b.value)
