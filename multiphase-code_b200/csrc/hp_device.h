@@ -79,15 +79,23 @@ struct DevMesh {
     // limiter epsilon^2 = (K dl)^3 per cell (src/sr_VK.F90:34), evaluated
     // once at set-up with the host's pow, as the reference evaluates it
     const double* eps2;     // [ld]
-    const double* sc;       // [12][ld] face area vectors sc1x..sc4z
-    const double* fch;      // [12][ld] face centroids, 0.3333 factor (HLLC, VK): x of faces 1-4, then y, z
-    const double* fxo;      // [12][ld] the same minus the cell's centroid (FP64 gradients, else null)
+    // Geometry tables, of leading dimension ldt.  FP64 handles, and FP32 ones
+    // without a face list, have a row for every cell.  Where only the FP64
+    // kernels of the wall layers read them, a row for each cell of gcells in
+    // list order (trows = 1): gcells starts with wcells, so row k is that of
+    // wcells[k] too, and with wprefix that of cell k.  Else no rows (null).
+    long long ldt;
+    int trows, trows_n;     // rows by list position; number of rows
+    const double* sc;       // [12][ldt] face area vectors sc1x..sc4z
+    const double* scq;      // [12][ld] the same for every cell (five-phase model, else null)
+    const double* fch;      // [12][ldt] face centroids, 0.3333 factor (HLLC, VK): x of faces 1-4, then y, z
+    const double* fxo;      // [12][ldt] the same minus the cell's centroid (FP64 gradients, else null)
     // face areas or, for the Jameson flux, unit normal (x, y, z) and area of
     // face 1, then 2, 3, 4; formed on the device by the variant that reads them
     // (Variant::setup), null when the handle runs no FP64 flux kernel
-    const double* area;     // [4][ld]
-    const double* nrm;      // [16][ld]
-    const double* fcv;      // [12][ld] face centroids, /3 (viscous; null in inviscid handles)
+    const double* area;     // [4][ldt]
+    const double* nrm;      // [16][ldt]
+    const double* fcv;      // [12][ldt] face centroids, /3 (viscous; null in inviscid handles)
     // geometry-only least-squares terms, evaluated once at set-up with the
     // reference's expressions: [0..3] weights, [4..9] a1 a2 a3 b1 b2 b3,
     // [10] the determinant; LSQA for the 1/r^2 cell gradients
@@ -95,18 +103,20 @@ struct DevMesh {
     // reciprocals of the weights ([11..14]) and of the determinant ([15]);
     // LSQB for the 1/r gradient of alpha_g in the sources
     // (src/sr_source.F90:100-117), then that of the determinant ([11])
-    const double* dxn;      // [12][ld] centroid of neighbour f minus the
+    const double* dxn;      // [12][ldt] centroid of neighbour f minus the
                             // cell's (x, y, z of face 1, then 2, 3, 4; FP64
                             // gradients, else null)
     // (null where nothing reads them: no FP64 kernels, no gradients)
-    const double* lsqa;     // [NLSQ][ld]
-    const double* lsqb;     // [NLSQB][ld]
+    const double* lsqa;     // [NLSQ][ldt]
+    const double* lsqb;     // [NLSQB][ldt]
     const int *g_par, *g_id, *g_type;   // [nghosts] ghost list (reference order)
     // overset fringe (nfringe = 0: none): cells, 4 donor cells each and
     // barycentric weights, [4][nfringe] column-major
     // unique faces (FP32-arithmetic variants; nface = 0: cell-centric
     // fluxes): owner cell and local face of each, and per cell and local
-    // face the signed face id + 1 (negative when the cell is not the owner)
+    // face the signed face id + 1 (negative when the cell is not the owner).
+    // Faces between two cells of the FP64 wall layers, or of one and a ghost,
+    // feed only FP64 kernels and are not in the list (0 in cface)
     int nface;
     long long fld;          // leading dimension of the face-flux columns
     const int* f_i;
@@ -114,12 +124,13 @@ struct DevMesh {
     // what the face kernels read of a face, in face order: the cell on its
     // other side, the owner's area vector and the face centroid minus the
     // centroids of owner and neighbour in the arithmetic of the fluxes, and
-    // the viscous face centroid; filled on the device from the cell columns
+    // the viscous face centroid; filled at set-up
     const int* f_j;
     const float* fgeo;      // [9][fld] area vector, offset from owner, from neighbour
     const double* fgcv;     // [3][fld]
     // centroid differences and face centroid offsets in float for the FP32
-    // gradients (FP32-arithmetic variants, no aliased ghosts; else null)
+    // gradients (FP32-arithmetic variants without aliased ghosts and without
+    // the FP64 tables of every cell; else null)
     const float *dxnf, *fxof;   // [12][ld] as dxn, fxo
     const int* cface;       // [4][ld]
     // face modes 2 (colouring) and 3 (atomics): the face fluxes are added

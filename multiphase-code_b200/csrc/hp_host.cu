@@ -189,14 +189,20 @@ static void plan_arena(hp_handle* h, Arena& a, int neles, int nghosts, long long
     // geometry tables of the FP64 gradients and fluxes (the wall layers' too);
     // first order and the Jameson flux (myflux 3) have no gradients
     const bool fp64 = gb == D || h->nwall > 0, grad = h->prm.myorder == 2 && h->prm.myflux != 3;
-    auto table = [&](bool read, int ncol) { return read ? (double*)a.take(ncol * (size_t)ld * D) : nullptr; };
-    m.sc = table(true, 12);
-    m.fch = table(true, 12);
+    const bool cells = gb == D || nface == 0;   // read by cell (see DevMesh::ldt)
+    m.trows_n = cells ? neles : h->ngwall;
+    m.trows = !cells;
+    m.ldt = cells ? ld : (h->ngwall + 63) / 64 * 64;
+    auto table = [&](bool read, int ncol) { return read ? (double*)a.take(ncol * (size_t)m.ldt * D) : nullptr; };
+    m.sc = table(cells || fp64, 12);
+    m.scq = nullptr;
+    if (h->neq == 22) m.scq = cells ? m.sc : (double*)a.take(12 * (size_t)ld * D);
+    m.fch = table(cells || fp64, 12);
     m.fxo = table(fp64 && grad, 12);
     m.dxn = table(fp64 && grad, 12);
     m.nrm = table(fp64 && h->prm.myflux == 3, 16);
     m.area = table(fp64 && h->prm.myflux != 3, 4);
-    m.fcv = table(!h->prm.inviscid, 12);
+    m.fcv = table((cells || fp64) && !h->prm.inviscid, 12);
     m.lsqa = table(fp64 && grad, NLSQ);
     m.lsqb = table(fp64, NLSQB);
     m.g_par = (int*)a.take((nghosts + 1) * (size_t)I); m.g_id = (int*)a.take((nghosts + 1) * (size_t)I);
@@ -238,8 +244,10 @@ static void plan_arena(hp_handle* h, Arena& a, int neles, int nghosts, long long
     s.agrad = nullptr;
     if (gb != D && !h->aliased && grad) {
         if (h->prm.precision == HP_PREC_MIXED) s.agrad = (double*)a.take(3 * (size_t)ld * gb);
-        m.dxnf = (const float*)a.take(12 * (size_t)ld * sizeof(float));
-        m.fxof = (const float*)a.take(12 * (size_t)ld * sizeof(float));
+        if (!(cells && fp64)) {   // (else the FP64 kernels' tables have every cell)
+            m.dxnf = (const float*)a.take(12 * (size_t)ld * sizeof(float));
+            m.fxof = (const float*)a.take(12 * (size_t)ld * sizeof(float));
+        }
     }
     m.nface = nface;
     m.fld = ((long long)nface + 63) / 64 * 64;
@@ -287,9 +295,9 @@ struct Layout {
 };
 
 // Cells within `layers` layers of a wall ghost (types 5 and 6), breadth
-// first over the interior neighbours: wall (ascending), the same with their
-// interior neighbours added (grad, ascending), and the per-slot class (1: a
-// layer cell with a neighbour outside the layers, 2: one without).
+// first over the interior neighbours: wall (ascending), the same followed by
+// their other interior neighbours (grad, ascending), and the per-slot class (1:
+// a layer cell with a neighbour outside the layers, 2: one without).
 static void wall_layers(const Layout& L, int neles, int nghosts, long long ld, int layers,
                         std::vector<int>& wall, std::vector<int>& grad, std::vector<unsigned char>& cls) {
     std::vector<int> gtype((size_t)nghosts, 0);
@@ -328,8 +336,9 @@ static void wall_layers(const Layout& L, int neles, int nghosts, long long ld, i
                 if (j < neles) ing[j] = 1;
             }
         }
+    grad = wall;
     for (int t = 0; t < neles; t++)
-        if (ing[t]) grad.push_back(t);
+        if (ing[t] && layer[t] == 0) grad.push_back(t);
     // class 2: every interior neighbour is a layer cell too, so no FP32 face
     // needs the cell's FP32 gradients
     for (int t : wall) {
@@ -364,6 +373,66 @@ static bool ghosts_aliased(const hp_mesh* mesh) {
             if (j < 1 || j > ntot || (j > neles && !seen[j])) return true;
         }
     return false;
+}
+
+// Layer (1, 2, ... layers; 0: none) of each element, counted over interior
+// neighbours from the elements next to a wall ghost (types 5 and 6).  No
+// aliased ghosts.
+static std::vector<int> mesh_layers(const hp_mesh* mesh, int layers) {
+    const int neles = mesh->neles, ntot = neles + mesh->nghosts;
+    std::vector<int> gtype((size_t)ntot + 1, 0), layer(neles, 0), front;
+    for (int g = 0; g < mesh->nghosts; g++) gtype[mesh->ghost[4 * (size_t)g + 1]] = mesh->ghost[4 * (size_t)g + 2];
+    auto nb = [&](int e, int k) { return mesh->elem[9 * (size_t)e + 4 + k]; };   // 1-based
+    for (int e = 0; e < neles; e++)
+        for (int k = 0; k < 4; k++) {
+            const int j = nb(e, k);
+            if (j > neles && (gtype[j] == 5 || gtype[j] == 6)) {
+                layer[e] = 1;
+                front.push_back(e);
+                break;
+            }
+        }
+    for (int n = 2; n <= layers && !front.empty(); n++) {
+        std::vector<int> next;
+        for (int e : front)
+            for (int k = 0; k < 4; k++) {
+                const int j = nb(e, k);
+                if (j <= neles && layer[j - 1] == 0) { layer[j - 1] = n; next.push_back(j - 1); }
+            }
+        front.swap(next);
+    }
+    return layer;
+}
+
+// Faces that a handle of the FP32-arithmetic variants lists for this mesh (0:
+// neighbours that are not mutual), layer cells, and layer cells with their
+// neighbours.
+static long long mesh_faces(const hp_mesh* mesh, int layers, long long& nwall, long long& ngwall) {
+    const int neles = mesh->neles;
+    std::vector<int> layer(neles, 0);
+    if (layers > 0) layer = mesh_layers(mesh, layers);
+    std::vector<char> ing(neles, 0);
+    long long n = 0;
+    bool mutual = true;
+    for (int e = 0; e < neles; e++)
+        for (int k = 0; k < 4; k++) {
+            const int j = mesh->elem[9 * (size_t)e + 4 + k] - 1;
+            if (layer[e]) {
+                ing[e] = 1;
+                if (j < neles) ing[j] = 1;
+            }
+            if (j < neles) {
+                const int32_t* r = mesh->elem + 9 * (size_t)j + 4;
+                if (r[0] != e + 1 && r[1] != e + 1 && r[2] != e + 1 && r[3] != e + 1) mutual = false;
+                if (j < e) continue;
+            }
+            if (!(layer[e] && (j >= neles || layer[j]))) n++;
+        }
+    for (int e = 0; e < neles; e++) {
+        nwall += layer[e] > 0;
+        ngwall += ing[e];
+    }
+    return mutual ? std::max(n, 1LL) : 0;
 }
 
 // One case of a handle: validates its connectivity, computes its geometry
@@ -558,33 +627,13 @@ static int fill_case(const hp_mesh* mesh, const hp_params* params, Layout& L, Ca
         std::vector<uint8_t> group(neles + 1, 2);
         const bool fp32_arith = params->precision == HP_PREC_MIXED || params->precision == HP_PREC_FP32;
         if (fp32_arith && params->wall_fp64_layers > 0) {
-            std::vector<int> gtype_of(ntot + 1, 0);
-            for (int g = 0; g < nghosts; g++) gtype_of[gid[g]] = gtyp[g];
-            std::vector<int> layer(neles + 1, 0), front;
+            const std::vector<int> layer = mesh_layers(mesh, params->wall_fp64_layers);
             for (int e = 1; e <= neles; e++)
-                for (int k = 0; k < 4; k++) {
-                    const int j = nc[k][e];
-                    if (j > neles && j <= ntot && (gtype_of[j] == 5 || gtype_of[j] == 6)) {
-                        layer[e] = 1;
-                        front.push_back(e);
-                        break;
-                    }
-                }
-            for (int k = 2; k <= params->wall_fp64_layers && !front.empty(); k++) {
-                std::vector<int> next;
-                for (int e : front)
-                    for (int f = 0; f < 4; f++) {
-                        const int j = nc[f][e];
-                        if (j <= neles && layer[j] == 0) { layer[j] = k; next.push_back(j); }
-                    }
-                front.swap(next);
-            }
-            for (int e = 1; e <= neles; e++)
-                if (layer[e] > 0) {
+                if (layer[e - 1] > 0) {
                     group[e] = 0;
                     for (int f = 0; f < 4; f++) {
                         const int j = nc[f][e];
-                        if (j <= neles && layer[j] == 0) group[j] = 1;
+                        if (j <= neles && layer[j - 1] == 0) group[j] = 1;
                     }
                 }
         }
@@ -663,69 +712,85 @@ static int fill_case(const hp_mesh* mesh, const hp_params* params, Layout& L, Ca
 namespace {
 inline unsigned blocks_for(long long n, int b) { return (unsigned)((n + b - 1) / b); }
 
-// Set-up, one thread per cell: the neighbour centroid differences of the
-// gradient LSQ (m.dxn), the face centroids minus the cell's own (m.fxo), and
-// float copies of both, the subtractions that the step's kernels would do; and
+// Face geometry of every cell as the host computed it, for set-up.
+struct FaceGeo { const double *sc, *fch, *fcv; };   // [12][ld] each
+
+// Set-up, one thread per table row: area vectors and centroids (where the
+// tables are not the host's columns themselves), the neighbour centroid
+// differences of the gradient LSQ (m.dxn) and the face centroids minus the
+// cell's own (m.fxo), the subtractions that the step's kernels would do; and
 // the range bits of m.fk: weights, determinants and face areas in [2^-100,
 // 2^101), centroid differences zero or in [2^-100, 2^100), components of area
 // vectors zero or at least 2^-800.
-__global__ void __launch_bounds__(128) k_offsets(DevMesh m) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= m.neles) return;
-    const long long ld = m.ld;
+__global__ void __launch_bounds__(128) k_table_rows(DevMesh m, FaceGeo src) {
+    const int r = blockIdx.x * blockDim.x + threadIdx.x;
+    if (r >= m.trows_n) return;
+    const int i = m.trows ? m.gcells[r] : r;
+    const long long ld = m.ld, lt = m.ldt;
     const double* x[3] = {m.xc, m.yc, m.zc};
+    if (m.trows)
+        for (int k = 0; k < 12; k++) {
+            const_cast<double*>(m.sc)[k * lt + r] = src.sc[k * ld + i];
+            const_cast<double*>(m.fch)[k * lt + r] = src.fch[k * ld + i];
+            if (m.fcv) const_cast<double*>(m.fcv)[k * lt + r] = src.fcv[k * ld + i];
+        }
     unsigned out = 0;
     for (int f = 0; f < 4; f++) {
         const int j = m.nc[f * ld + i];
-        for (int d = 0; d < 3; d++) {
-            const double dx = x[d][j] - x[d][i], fo = m.fch[(4 * d + f) * ld + i] - x[d][i];
-            if (m.dxn) {
-                const_cast<double*>(m.dxn)[(3 * f + d) * ld + i] = dx;
-                const_cast<double*>(m.fxo)[(4 * d + f) * ld + i] = fo;
-            }
-            if (m.dxnf) {
-                const_cast<float*>(m.dxnf)[(3 * f + d) * ld + i] = (float)dx;
-                const_cast<float*>(m.fxof)[(4 * d + f) * ld + i] = (float)fo;
-            }
-            const double a = fabs(dx);
-            if (a != 0.0 && !(a >= 0x1p-100 && a < 0x1p100)) out |= FK_LSQA_RANGE | FK_LSQB_RANGE;
-        }
-    }
-    for (int f = 0; f < 4; f++) {
         double a2 = 0.0;
         for (int d = 0; d < 3; d++) {
-            const double a = fabs(m.sc[(3 * f + d) * ld + i]);
-            a2 += a * a;
+            const double dx = x[d][j] - x[d][i];
+            if (m.dxn) {
+                const_cast<double*>(m.dxn)[(3 * f + d) * lt + r] = dx;
+                const_cast<double*>(m.fxo)[(4 * d + f) * lt + r] = src.fch[(4 * d + f) * ld + i] - x[d][i];
+            }
+            const double b = fabs(dx), a = fabs(src.sc[(3 * f + d) * ld + i]);
+            if (b != 0.0 && !(b >= 0x1p-100 && b < 0x1p100)) out |= FK_LSQA_RANGE | FK_LSQB_RANGE;
             if (a != 0.0 && !(a >= 0x1p-800)) out |= FK_AREA_RANGE;
+            a2 += a * a;
         }
         const double area = sqrt(a2);
         if (!(area >= 0x1p-100 && area < 0x1p101)) out |= FK_AREA_RANGE;
     }
     for (int t = 0; t < 5; t++) {
         const int k = t < 4 ? t : 10;
-        const double a = m.lsqa ? m.lsqa[k * ld + i] : 1.0, b = m.lsqb ? m.lsqb[k * ld + i] : 1.0;
+        const double a = m.lsqa ? m.lsqa[k * lt + r] : 1.0, b = m.lsqb ? m.lsqb[k * lt + r] : 1.0;
         if (!(a >= 0x1p-100 && a < 0x1p101)) out |= FK_LSQA_RANGE;
         if (!(b >= 0x1p-100 && b < 0x1p101)) out |= FK_LSQB_RANGE;
     }
     if (out) const_cast<unsigned*>(m.fk)[i] |= out;
 }
 
-// Set-up, one thread per face: the face-ordered tables (after k_offsets).
-__global__ void __launch_bounds__(128) k_face_tables(DevMesh m) {
+// Set-up, one thread per cell: what the FP32 gradients read, as floats.
+__global__ void __launch_bounds__(128) k_cell_floats(DevMesh m, FaceGeo src) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= m.neles) return;
+    const long long ld = m.ld;
+    const double* x[3] = {m.xc, m.yc, m.zc};
+    for (int f = 0; f < 4; f++) {
+        const int j = m.nc[f * ld + i];
+        for (int d = 0; d < 3; d++) {
+            const_cast<float*>(m.dxnf)[(3 * f + d) * ld + i] = (float)(x[d][j] - x[d][i]);
+            const_cast<float*>(m.fxof)[(4 * d + f) * ld + i] = (float)(src.fch[(4 * d + f) * ld + i] - x[d][i]);
+        }
+    }
+}
+
+// Set-up, one thread per face: the face-ordered tables.
+__global__ void __launch_bounds__(128) k_face_tables(DevMesh m, FaceGeo src) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= m.nface) return;
     const long long ld = m.ld, fl = m.fld;
-    const int i = m.f_i[t], f = m.f_code[t] & 3;
+    const int i = m.f_i[t], f = m.f_code[t] & 3, j = m.nc[f * ld + i];
     float* g = const_cast<float*>(m.fgeo);
-    const int j = m.nc[f * ld + i];
     const_cast<int*>(m.f_j)[t] = j;
     const double* x[3] = {m.xc, m.yc, m.zc};
     for (int d = 0; d < 3; d++) {
-        const double fc = m.fch[(4 * d + f) * ld + i];
-        g[d * fl + t] = (float)m.sc[(3 * f + d) * ld + i];
+        const double fc = src.fch[(4 * d + f) * ld + i];
+        g[d * fl + t] = (float)src.sc[(3 * f + d) * ld + i];
         g[(3 + d) * fl + t] = (float)(fc - x[d][i]);
         g[(6 + d) * fl + t] = (float)(fc - x[d][j]);
-        if (m.fgcv) const_cast<double*>(m.fgcv)[d * fl + t] = m.fcv[(4 * d + f) * ld + i];
+        if (m.fgcv) const_cast<double*>(m.fgcv)[d * fl + t] = src.fcv[(4 * d + f) * ld + i];
     }
 }
 }  // namespace
@@ -844,6 +909,16 @@ extern "C" int hp_create_batch(const hp_mesh* meshes, int32_t ncase, const hp_pa
     if (cudaGetDevice(&dev) != cudaSuccess) { delete h; return fail(nullptr, HP_E_CUDA, "no CUDA device"); }
     h->device = dev;
     const size_t D = sizeof(double), I = sizeof(int), gb = h->var->grad_bytes;
+    // --- FP64 wall layers of the FP32-arithmetic variants ---
+    std::vector<int> hwall, hgwall;
+    std::vector<unsigned char> hwclass;
+    if (gb != D && p.wall_fp64_layers > 0) {
+        if (h->aliased) {
+            delete h;
+            return fail(nullptr, HP_E_UNSUPPORTED, "FP64 wall layers: aliased ghost ids");
+        }
+        wall_layers(L, neles, nghosts, ld, p.wall_fp64_layers, hwall, hgwall, hwclass);
+    }
     // --- unique faces for the face-based fluxes of the FP32-arithmetic
     // variants: a face belongs to its lower-id element (or to its element
     // when the other side is a ghost); meshes whose neighbour lists are not
@@ -869,10 +944,10 @@ extern "C" int hp_create_batch(const hp_mesh* meshes, int32_t ncase, const hp_pa
             }
         if (!mutual) { hf_i.clear(); hf_code.clear(); hcface.clear(); }
     }
-    const int nface = (int)hf_i.size();
+    int nface = (int)hf_i.size();
     // face mode 2: greedy colouring of the faces in id order, so that no two
     // faces of a colour touch the same element (tets: at most 7 colours)
-    std::vector<int> hf_color;
+    std::vector<int> hf_color, face_color;
     int ncolor = 0, fcoff[33] = {0};
     if (nface > 0 && h->prm.face_mode == 2) {
         std::vector<uint32_t> used((size_t)ld, 0u);
@@ -887,6 +962,44 @@ extern "C" int hp_create_batch(const hp_mesh* meshes, int32_t ncase, const hp_pa
             if (j < neles) used[j] |= 1u << c;
             ncolor = std::max(ncolor, c + 1);
         }
+        face_color = std::move(col);
+    }
+    // without the faces that only FP64 kernels would read (two layer cells, or
+    // one and a ghost); the others keep their order and colours.  One face
+    // stays where every cell is a layer cell: the handle still runs the
+    // face-based kernels, and no cell reads that face.
+    if (nface > 0 && !hwall.empty()) {
+        int n = 0;
+        std::vector<int> id(nface, -1);
+        for (int t = 0; t < nface; t++) {
+            const int i = hf_i[t], j = L.nc[(size_t)hf_code[t] * ld + i];
+            const bool fp64_only = hwclass[i] && (j >= neles || hwclass[j]);
+            if (fp64_only && !(n == 0 && t == nface - 1)) continue;
+            if (!fp64_only) id[t] = n;
+            hf_i[n] = i;
+            hf_code[n] = hf_code[t];
+            if (!face_color.empty()) face_color[n] = face_color[t];
+            n++;
+        }
+        for (int& c : hcface)
+            if (c) {
+                const int k = id[(c > 0 ? c : -c) - 1];
+                c = k < 0 ? 0 : c > 0 ? k + 1 : -(k + 1);
+            }
+        nface = n;
+        hf_i.resize(n);
+        hf_code.resize(n);
+        face_color.resize(face_color.empty() ? 0 : n);
+        // (a colour may have lost all its faces)
+        int seen[32] = {0}, to[32] = {0};
+        for (int c : face_color) seen[c] = 1;
+        ncolor = 0;
+        for (int c = 0; c < 32; c++)
+            if (seen[c]) to[c] = ncolor++;
+        for (int& c : face_color) c = to[c];
+    }
+    if (nface > 0 && h->prm.face_mode == 2) {
+        const std::vector<int>& col = face_color;
         for (int t = 0; t < nface; t++) fcoff[col[t] + 1]++;
         for (int c = 0; c < ncolor; c++) fcoff[c + 1] += fcoff[c];
         hf_color.assign(nface, 0);
@@ -894,16 +1007,6 @@ extern "C" int hp_create_batch(const hp_mesh* meshes, int32_t ncase, const hp_pa
         for (int t = 0; t < nface; t++) hf_color[pos[col[t]]++] = t;
     } else if (nface > 0 && h->prm.face_mode == 3) {
         hf_color.assign(nface, 0);   // unused by the atomic scatter; keeps the array defined
-    }
-    // --- FP64 wall layers of the FP32-arithmetic variants ---
-    std::vector<int> hwall, hgwall;
-    std::vector<unsigned char> hwclass;
-    if (gb != D && p.wall_fp64_layers > 0) {
-        if (h->aliased) {
-            delete h;
-            return fail(nullptr, HP_E_UNSUPPORTED, "FP64 wall layers: aliased ghost ids");
-        }
-        wall_layers(L, neles, nghosts, ld, p.wall_fp64_layers, hwall, hgwall, hwclass);
     }
     h->nwall = (int)hwall.size();
     h->ngwall = (int)hgwall.size();
@@ -981,12 +1084,7 @@ extern "C" int hp_create_batch(const hp_mesh* meshes, int32_t ncase, const hp_pa
     if (e == cudaSuccess) e = up(m.dl, L.dl.data(), ld * D);
     if (e == cudaSuccess) e = up(m.eps2, L.eps2.data(), ld * D);
     if (e == cudaSuccess) e = up(m.dd, L.dd.data(), ld * D);
-    if (e == cudaSuccess) e = up(m.sc, L.sc.data(), 12 * ld * D);
-    if (e == cudaSuccess && m.fcv) e = up(m.fcv, L.fcv.data(), 12 * ld * D);
-    if (e == cudaSuccess && m.lsqa) e = up(m.lsqa, L.la.data(), NLSQ * ld * D);
-    if (e == cudaSuccess && m.lsqb) e = up(m.lsqb, L.lb.data(), NLSQB * ld * D);
     if (e == cudaSuccess) e = up(m.fk, L.fk.data(), ld * sizeof(unsigned));
-    if (e == cudaSuccess) e = up(m.fch, L.fch.data(), 12 * ld * D);
     if (e == cudaSuccess && nghosts) e = up(m.g_par, L.gpar.data(), nghosts * (size_t)I);
     if (e == cudaSuccess && nghosts) e = up(m.g_id, L.gid.data(), nghosts * (size_t)I);
     if (e == cudaSuccess && nghosts) e = up(m.g_type, L.gtyp.data(), nghosts * (size_t)I);
@@ -995,13 +1093,6 @@ extern "C" int hp_create_batch(const hp_mesh* meshes, int32_t ncase, const hp_pa
     if (e == cudaSuccess && nface) e = up(m.f_i, hf_i.data(), nface * (size_t)I);
     if (e == cudaSuccess && nface) e = up(m.f_code, hf_code.data(), nface * (size_t)I);
     if (e == cudaSuccess && nface) e = up(m.cface, hcface.data(), 4 * (size_t)ld * I);
-    if (e == cudaSuccess) {
-        k_offsets<<<blocks_for(neles, 128), 128, 0, st>>>(m);
-        if (nface) k_face_tables<<<blocks_for(nface, 128), 128, 0, st>>>(m);
-        if (gb == D) h->var->setup(m, st);
-        else wall_fp64.setup(m, st);
-        e = cudaGetLastError();
-    }
     m.face_mode = nface > 0 ? h->prm.face_mode : 0;
     m.ncolor = ncolor;
     for (int c = 0; c <= ncolor; c++) m.fcoff[c] = fcoff[c];
@@ -1009,7 +1100,39 @@ extern "C" int hp_create_batch(const hp_mesh* meshes, int32_t ncase, const hp_pa
     if (e == cudaSuccess && h->nwall) e = up(m.wcells, hwall.data(), hwall.size() * (size_t)I);
     if (e == cudaSuccess && h->nwall) e = up(m.gcells, hgwall.data(), hgwall.size() * (size_t)I);
     if (e == cudaSuccess && h->nwall) e = up(m.wclass, hwclass.data(), (size_t)ld);
-    // hwall, hgwall and hwclass are local vectors
+    // geometry tables.  Tables by cell take the host's columns; otherwise those
+    // stand in the state's columns (44 doubles a cell and more) while the rows
+    // and the face-ordered tables are formed.
+    FaceGeo geo{m.sc, m.fch, m.fcv};
+    if (m.trows) geo = FaceGeo{h->ds.cn, h->ds.cn + 12 * ld, P.inviscid ? nullptr : h->ds.cn + 24 * ld};
+    if (e == cudaSuccess) e = up(geo.sc, L.sc.data(), 12 * ld * D);
+    if (e == cudaSuccess) e = up(geo.fch, L.fch.data(), 12 * ld * D);
+    if (e == cudaSuccess && geo.fcv) e = up(geo.fcv, L.fcv.data(), 12 * ld * D);
+    if (e == cudaSuccess && m.trows && m.scq) e = up(m.scq, L.sc.data(), 12 * ld * D);
+    std::vector<double> rows_a, rows_b;   // LSQ terms of the rows
+    auto up_lsq = [&](const double* dst, const std::vector<double>& col, int n, std::vector<double>& rows) {
+        if (!dst) return;
+        const double* from = col.data();
+        if (m.trows) {
+            rows.assign((size_t)n * m.ldt, 0.0);
+            for (int k = 0; k < n; k++)
+                for (int r = 0; r < h->ngwall; r++) rows[k * m.ldt + r] = col[k * ld + hgwall[r]];
+            from = rows.data();
+        }
+        if (e == cudaSuccess) e = up(dst, from, (size_t)n * m.ldt * D);
+    };
+    up_lsq(m.lsqa, L.la, NLSQ, rows_a);
+    up_lsq(m.lsqb, L.lb, NLSQB, rows_b);
+    if (e == cudaSuccess) {
+        if (m.trows_n) k_table_rows<<<blocks_for(m.trows_n, 128), 128, 0, st>>>(m, geo);
+        if (m.dxnf) k_cell_floats<<<blocks_for(neles, 128), 128, 0, st>>>(m, geo);
+        if (nface) k_face_tables<<<blocks_for(nface, 128), 128, 0, st>>>(m, geo);
+        if (gb == D) h->var->setup(m, st);
+        else wall_fp64.setup(m, st);
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess && m.trows) e = cudaMemsetAsync(h->ds.cn, 0, 36 * (size_t)ld * D, st);
+    // hwall, hgwall, hwclass and the rows are local vectors
     if (e == cudaSuccess && h->nwall) e = cudaStreamSynchronize(st);
     if (e == cudaSuccess && ncase > 1) {
         std::vector<int> cid(neles);
@@ -1613,30 +1736,47 @@ extern "C" int hp_estimate_bytes(const hp_mesh* mesh, const hp_params* params, i
 extern "C" int hp_estimate_batch_bytes(const hp_mesh* meshes, int32_t ncase, const hp_params* params,
                                        int64_t* bytes) {
     if (!meshes || !params || !bytes || ncase < 1) return HP_E_ARG;
-    long long ne = 0, ng = 0;
-    bool sizes_only = false;
+    const bool fp32 = params->precision == HP_PREC_MIXED || params->precision == HP_PREC_FP32;
+    const int layers = fp32 && params->wall_fp64_layers > 0 ? params->wall_fp64_layers : 0;
+    long long ne = 0, ng = 0, nface = 0, nwall = 0, ngwall = 0;
+    bool sizes_only = false, listed = true;
     hp_handle probe_h;
     probe_h.prm = *params;
     for (int c = 0; c < ncase; c++) {
-        if (meshes[c].neles <= 0 || meshes[c].nghosts < 0) return HP_E_ARG;
-        ne += meshes[c].neles;
-        ng += meshes[c].nghosts;
-        if (!meshes[c].elem || (meshes[c].nghosts > 0 && !meshes[c].ghost)) sizes_only = true;
-        else if (ghosts_aliased(meshes + c)) probe_h.aliased = 1;
+        const hp_mesh* mesh = meshes + c;
+        if (mesh->neles <= 0 || mesh->nghosts < 0) return HP_E_ARG;
+        ne += mesh->neles;
+        ng += mesh->nghosts;
+        if (!mesh->elem || (mesh->nghosts > 0 && !mesh->ghost)) {
+            sizes_only = true;
+        } else if (ghosts_aliased(mesh)) {
+            probe_h.aliased = 1;
+        } else if (fp32) {
+            const long long n = mesh_faces(mesh, layers, nwall, ngwall);
+            nface += n;
+            listed = listed && n > 0;
+        }
     }
     const long long ld = (ne + ng + 63) / 64 * 64;
-    const size_t gb = (params->precision == HP_PREC_MIXED || params->precision == HP_PREC_FP32) ? sizeof(float)
-                                                                                                : sizeof(double);
+    const size_t gb = fp32 ? sizeof(float) : sizeof(double);
     probe_h.neq = params->five_phase ? 22 : 10;
-    if (gb != sizeof(double) && params->wall_fp64_layers > 0)   // bound: every cell in the layers
-        probe_h.nwall = probe_h.ngwall = (int)ne;
-    *bytes = 0;
-    for (int pass = 0; pass < (sizes_only ? 2 : 1); pass++) {   // sizes alone: the larger of both kinds of ghosts
-        if (pass) probe_h.aliased = !probe_h.aliased;
-        const bool faces = gb != sizeof(double) && params->face_mode != 1 && !probe_h.aliased;
+    auto plan = [&](bool aliased, long long faces) {
+        probe_h.aliased = aliased;
         Arena probe;
-        plan_arena(&probe_h, probe, (int)ne, (int)ng, ld, gb, ncase, faces ? (int)((4 * ne + ng) / 2) : 0);
+        plan_arena(&probe_h, probe, (int)ne, (int)ng, ld, gb, ncase, (int)faces);
         *bytes = std::max(*bytes, (int64_t)(probe.used + 256));
+    };
+    *bytes = 0;
+    const bool aliased = probe_h.aliased;
+    if (sizes_only) {   // an upper bound: either kind of ghosts, every cell in the layers
+        probe_h.nwall = probe_h.ngwall = layers ? (int)ne : 0;
+        plan(true, 0);
+        plan(false, 0);
+        if (fp32 && params->face_mode != 1) plan(false, (4 * ne + ng) / 2);
+    } else {
+        probe_h.nwall = aliased ? 0 : (int)nwall;
+        probe_h.ngwall = aliased ? 0 : (int)ngwall;
+        plan(aliased, aliased || !listed || params->face_mode == 1 ? 0 : nface);
     }
     return HP_OK;
 }

@@ -235,6 +235,8 @@ __device__ __forceinline__ T qshfl(T v, int q) {
 }
 
 #define COL(ptr, k) ((ptr) + (size_t)(k) * (size_t)m.ld)
+// geometry table column, indexed by table row (see DevMesh::ldt)
+#define TAB(ptr, k) ((ptr) + (size_t)(k) * (size_t)m.ldt)
 // Primitive column k, indexed by prim_off(c).  983,040 cells against plain
 // columns: FP32 viscous terms 218 -> 180 us, FP32 gradients 326 -> 314 us
 // (three launches), FP64 viscous terms 560 -> 551 us, k_flux4 2007 -> 1998 us.
@@ -944,15 +946,6 @@ __device__ __forceinline__ bool grad_cell(int ib) { return ib == 1 || ib == HP_I
 // Venkatakrishnan limiter (src/sr_VK.F90:32-272).  grad_cell() cells.
 // FPR: read the primitives in R (the float copy of the FP32-arithmetic
 // variants) instead of the FP64 columns; false on aliased meshes.
-// FP64 wall layers of the FP32 variants: a face whose two cells are layer
-// cells (or a layer cell's boundary face) feeds only FP64 kernels, so the
-// FP32 face kernels skip it.
-__device__ __forceinline__ bool wall_face(const DevMesh& m, int i, int f) {
-    if (sizeof(R) == sizeof(double) || m.nwall == 0 || !ldg(m.wclass + i)) return false;
-    const int j = ldg(COL(m.nc, f) + i);
-    return j >= m.neles || ldg(m.wclass + j) != 0;
-}
-
 // FP32 fluxes with an FP64 state path (mixed): the gradient kernel forms the
 // sources' alpha_g gradient and the flux kernel recovers the next stage's
 // primitives.  The all-FP32 variant keeps its passes apart: its recovery
@@ -988,7 +981,7 @@ __device__ __forceinline__ void alpha_gradient(const R xa[4], const R ya[4], con
 }
 #endif
 
-template <bool FPR>
+template <bool FPR, bool FLT>
 __device__ __forceinline__ void k_grad_body(DevMesh m, DevState<R> s, DevParams P, int bid) {
     using PT = typename std::conditional<FPR, R, double>::type;
     const PT* const prb = reinterpret_cast<const PT*>(FPR ? (const void*)s.prr : (const void*)s.pr);
@@ -1001,14 +994,20 @@ __device__ __forceinline__ void k_grad_body(DevMesh m, DevState<R> s, DevParams 
     int n[4];
 #pragma unroll
     for (int f = 0; f < 4; f++) n[f] = ldg(COL(m.nc, f) + i);
-    // FPR: centroid differences from the set-up table (the same subtractions)
+    // FPR: centroid differences from a set-up table (the same subtractions): the
+    // float copies (FLT) or, where the FP64 kernels have them for every cell,
+    // theirs
     R xa[4], ya[4], za[4];
 #pragma unroll
     for (int f = 0; f < 4; f++) {
-        if constexpr (FPR) {
+        if constexpr (FPR && FLT) {
             xa[f] = (R)ldg(COL(m.dxnf, 3 * f) + i);
             ya[f] = (R)ldg(COL(m.dxnf, 3 * f + 1) + i);
             za[f] = (R)ldg(COL(m.dxnf, 3 * f + 2) + i);
+        } else if constexpr (FPR) {
+            xa[f] = (R)ldg(TAB(m.dxn, 3 * f) + i);
+            ya[f] = (R)ldg(TAB(m.dxn, 3 * f + 1) + i);
+            za[f] = (R)ldg(TAB(m.dxn, 3 * f + 2) + i);
         } else {
             xa[f] = (R)(ldg(m.xc + n[f]) - ldg(m.xc + i));
             ya[f] = (R)(ldg(m.yc + n[f]) - ldg(m.yc + i));
@@ -1021,10 +1020,10 @@ __device__ __forceinline__ void k_grad_body(DevMesh m, DevState<R> s, DevParams 
 #define DW(x, f) div_rn((x), wt[f], rw[f])
 #if HP_LSQ_TABLE
 #pragma unroll
-    for (int f = 0; f < 4; f++) { wt[f] = (R)ldg(COL(m.lsqa, f) + i); rw[f] = rcp(wt[f]); }
-    const R a1 = (R)ldg(COL(m.lsqa, 4) + i), a2 = (R)ldg(COL(m.lsqa, 5) + i), a3 = (R)ldg(COL(m.lsqa, 6) + i);
-    const R b1 = (R)ldg(COL(m.lsqa, 7) + i), b2 = (R)ldg(COL(m.lsqa, 8) + i), b3 = (R)ldg(COL(m.lsqa, 9) + i);
-    const R dnr = (R)ldg(COL(m.lsqa, 10) + i);
+    for (int f = 0; f < 4; f++) { wt[f] = (R)ldg(TAB(m.lsqa, f) + i); rw[f] = rcp(wt[f]); }
+    const R a1 = (R)ldg(TAB(m.lsqa, 4) + i), a2 = (R)ldg(TAB(m.lsqa, 5) + i), a3 = (R)ldg(TAB(m.lsqa, 6) + i);
+    const R b1 = (R)ldg(TAB(m.lsqa, 7) + i), b2 = (R)ldg(TAB(m.lsqa, 8) + i), b3 = (R)ldg(TAB(m.lsqa, 9) + i);
+    const R dnr = (R)ldg(TAB(m.lsqa, 10) + i);
 #else
 #pragma unroll
     for (int f = 0; f < 4; f++) { wt[f] = xa[f] * xa[f] + ya[f] * ya[f] + za[f] * za[f]; rw[f] = rcp(wt[f]); }
@@ -1093,14 +1092,18 @@ __device__ __forceinline__ void k_grad_body(DevMesh m, DevState<R> s, DevParams 
     R fx[4], fy[4], fz[4];
 #pragma unroll
     for (int f = 0; f < 4; f++) {
-        if constexpr (FPR) {
+        if constexpr (FPR && FLT) {
             fx[f] = (R)ldg(COL(m.fxof, f) + i);
             fy[f] = (R)ldg(COL(m.fxof, 4 + f) + i);
             fz[f] = (R)ldg(COL(m.fxof, 8 + f) + i);
+        } else if constexpr (FPR) {
+            fx[f] = (R)ldg(TAB(m.fxo, f) + i);
+            fy[f] = (R)ldg(TAB(m.fxo, 4 + f) + i);
+            fz[f] = (R)ldg(TAB(m.fxo, 8 + f) + i);
         } else {
-            fx[f] = (R)(ldg(COL(m.fch, f) + i) - ldg(m.xc + i));
-            fy[f] = (R)(ldg(COL(m.fch, 4 + f) + i) - ldg(m.yc + i));
-            fz[f] = (R)(ldg(COL(m.fch, 8 + f) + i) - ldg(m.zc + i));
+            fx[f] = (R)(ldg(TAB(m.fch, f) + i) - ldg(m.xc + i));
+            fy[f] = (R)(ldg(TAB(m.fch, 4 + f) + i) - ldg(m.yc + i));
+            fz[f] = (R)(ldg(TAB(m.fch, 8 + f) + i) - ldg(m.zc + i));
         }
     }
     const int lv[4] = {8, 9, 11, 12};   // pg, pp, rog, rop rows of gv
@@ -1126,9 +1129,9 @@ __device__ __forceinline__ void k_grad_body(DevMesh m, DevState<R> s, DevParams 
     }
     s.phi[i] = (double)phi;
 }
-template <bool FPR>
+template <bool FPR, bool FLT>
 __global__ void __launch_bounds__(128) k_grad(DevMesh m, DevState<R> s, DevParams P) {
-    k_grad_body<FPR>(m, s, P, blockIdx.x);
+    k_grad_body<FPR, FLT>(m, s, P, blockIdx.x);
 }
 
 // ---------------------------------------------------------------------------
@@ -1305,9 +1308,10 @@ enum { LIM_LD = 128, LIMC_N = 13, LIMC_LD = 32 };
 // LIST: the face is face t of the face list and its geometry comes from the
 // face-ordered FP32 tables: consecutive threads read consecutive words, where
 // the cell columns of four different f's gave a warp a quarter of each sector.
+// Otherwise t is the cell's table row.
 template <int F, int Z, class PT, bool NC = true, bool LIST = false>
 __device__ __forceinline__ void face_eval(const DevMesh& m, const DevState<R>& s, const DevParams& P,
-                                          int i, int f, FaceOut& o, unsigned& bad, const PT* pr, int t = 0) {
+                                          int i, int f, FaceOut& o, unsigned& bad, const PT* pr, int t) {
 #define FGEO(k) (R)ldg(m.fgeo + (size_t)(k) * m.fld + t)
     const int neigh = LIST ? ldg(m.f_j + t) : ldg(COL(m.nc, f) + i);
     const unsigned kind = (ldg(m.fk + i) >> (4 * f)) & 0xFu;
@@ -1317,24 +1321,24 @@ __device__ __forceinline__ void face_eval(const DevMesh& m, const DevState<R>& s
         // the Jameson flux has little else to do, and its handles have no
         // gradient tables (formed here: 1694 -> 1719 us, 983,040 cells, four
         // launches)
-        enx = ldg(COL(m.nrm, 4 * f) + i);
-        eny = ldg(COL(m.nrm, 4 * f + 1) + i);
-        enz = ldg(COL(m.nrm, 4 * f + 2) + i);
-        area = ldg(COL(m.nrm, 4 * f + 3) + i);
+        enx = ldg(TAB(m.nrm, 4 * f) + t);
+        eny = ldg(TAB(m.nrm, 4 * f + 1) + t);
+        enz = ldg(TAB(m.nrm, 4 * f + 2) + t);
+        area = ldg(TAB(m.nrm, 4 * f + 3) + t);
     } else if constexpr (sizeof(R) == 8) {
         // the area from a set-up table, and one reciprocal for the three
         // quotients (ranges tested at set-up).  The normals as a table too, 96
         // B a cell, would take 23 us off three launches of 1976 (983,040
         // cells).
-        const R scx = ldg(COL(m.sc, 3 * f) + i), scy = ldg(COL(m.sc, 3 * f + 1) + i), scz = ldg(COL(m.sc, 3 * f + 2) + i);
-        area = ldg(COL(m.area, f) + i);
+        const R scx = ldg(TAB(m.sc, 3 * f) + t), scy = ldg(TAB(m.sc, 3 * f + 1) + t), scz = ldg(TAB(m.sc, 3 * f + 2) + t);
+        area = ldg(TAB(m.area, f) + t);
         const R rarea = F == 0 ? R(0) : R(1) / area;
         enx = mquo<F>(scx, area, rarea);
         eny = mquo<F>(scy, area, rarea);
         enz = mquo<F>(scz, area, rarea);
     } else {
-        const R scx = LIST ? FGEO(0) : (R)ldg(COL(m.sc, 3 * f) + i), scy = LIST ? FGEO(1) : (R)ldg(COL(m.sc, 3 * f + 1) + i),
-                scz = LIST ? FGEO(2) : (R)ldg(COL(m.sc, 3 * f + 2) + i);
+        const R scx = LIST ? FGEO(0) : (R)ldg(TAB(m.sc, 3 * f) + t), scy = LIST ? FGEO(1) : (R)ldg(TAB(m.sc, 3 * f + 1) + t),
+                scz = LIST ? FGEO(2) : (R)ldg(TAB(m.sc, 3 * f + 2) + t);
         area = sqrt(scx * scx + scy * scy + scz * scz);
         const R rarea = mrcp<F>(area, bad);
         enx = mdiv<F>(scx, area, rarea, bad);
@@ -1438,7 +1442,7 @@ __device__ __forceinline__ void face_eval(const DevMesh& m, const DevState<R>& s
             xf0 = FGEO(3); yf0 = FGEO(4); zf0 = FGEO(5);
             xfn = FGEO(6); yfn = FGEO(7); zfn = FGEO(8);
         } else {
-            const double xf = ldg(COL(m.fch, f) + i), yf = ldg(COL(m.fch, 4 + f) + i), zf = ldg(COL(m.fch, 8 + f) + i);
+            const double xf = ldg(TAB(m.fch, f) + t), yf = ldg(TAB(m.fch, 4 + f) + t), zf = ldg(TAB(m.fch, 8 + f) + t);
             xf0 = (R)(xf - ldg(m.xc + i)); yf0 = (R)(yf - ldg(m.yc + i)); zf0 = (R)(zf - ldg(m.zc + i));
             xfn = (R)(xf - ldg(m.xc + neigh)); yfn = (R)(yf - ldg(m.yc + neigh)); zfn = (R)(zf - ldg(m.zc + neigh));
         }
@@ -1683,7 +1687,7 @@ __device__ __noinline__ void stale_flux(const DevMesh& m, const DevState<R>& s, 
         }
         FaceOut o;
         unsigned bad_ = 0;
-        face_eval<0, Z>(m, s, P, cell, face, o, bad_, s.pr);
+        face_eval<0, Z>(m, s, P, cell, face, o, bad_, s.pr, cell);
         if (!o.wall && (gas ? o.takeg : o.takep)) {
             for (int k = 0; k < 5; k++) out[k] = o.F[(gas ? 0 : 5) + k];
             return;
@@ -1780,7 +1784,7 @@ __device__ __forceinline__ void k_flux_body(DevMesh m, DevState<R> s, DevParams 
     for (int f = 0; f < 4 && !FACE && !ACC; f++) {
         FaceOut o;
         unsigned bad_ = 0;
-        face_eval<0, Z>(m, s, P, i, f, o, bad_, s.pr);
+        face_eval<0, Z>(m, s, P, i, f, o, bad_, s.pr, i);
         if (o.wall) {
             rhs[1] = rhs[1] + (double)o.w[0]; rhs[2] = rhs[2] + (double)o.w[1];
             rhs[3] = rhs[3] + (double)o.w[2]; rhs[6] = rhs[6] + (double)o.w[3];
@@ -1860,13 +1864,13 @@ __device__ __forceinline__ void k_flux_body(DevMesh m, DevState<R> s, DevParams 
 #if HP_LSQ_TABLE
             R wt[4], rw[4];
 #pragma unroll
-            for (int f = 0; f < 4; f++) { wt[f] = (R)ldg(COL(m.lsqb, f) + i); rw[f] = rcp(wt[f]); }
-            const R a1 = (R)ldg(COL(m.lsqb, 4) + i), a2 = (R)ldg(COL(m.lsqb, 5) + i), a3 = (R)ldg(COL(m.lsqb, 6) + i);
-            const R b1 = (R)ldg(COL(m.lsqb, 7) + i), b2 = (R)ldg(COL(m.lsqb, 8) + i), b3 = (R)ldg(COL(m.lsqb, 9) + i);
+            for (int f = 0; f < 4; f++) { wt[f] = (R)ldg(TAB(m.lsqb, f) + i); rw[f] = rcp(wt[f]); }
+            const R a1 = (R)ldg(TAB(m.lsqb, 4) + i), a2 = (R)ldg(TAB(m.lsqb, 5) + i), a3 = (R)ldg(TAB(m.lsqb, 6) + i);
+            const R b1 = (R)ldg(TAB(m.lsqb, 7) + i), b2 = (R)ldg(TAB(m.lsqb, 8) + i), b3 = (R)ldg(TAB(m.lsqb, 9) + i);
             R c1 = DW(pa[0] * xa[0], 0) + DW(pa[1] * xa[1], 1) + DW(pa[2] * xa[2], 2) + DW(pa[3] * xa[3], 3);
             R c2 = DW(pa[0] * ya[0], 0) + DW(pa[1] * ya[1], 1) + DW(pa[2] * ya[2], 2) + DW(pa[3] * ya[3], 3);
             R c3 = DW(pa[0] * za[0], 0) + DW(pa[1] * za[1], 1) + DW(pa[2] * za[2], 2) + DW(pa[3] * za[3], 3);
-            const R dnr = (R)ldg(COL(m.lsqb, 10) + i);
+            const R dnr = (R)ldg(TAB(m.lsqb, 10) + i);
             const R rdnr = rcp(dnr);
             dpx = div_rn(det3(c1, c2, c3, b1, a2, b3, b2, b3, a3), dnr, rdnr);
             dpy = div_rn(det3(a1, b1, b2, c1, c2, c3, b2, b3, a3), dnr, rdnr);
@@ -1965,9 +1969,9 @@ __device__ __forceinline__ unsigned grad4_limiter(const DevMesh& m, const DevSta
     R phl = R(0);
 #pragma unroll
     for (int f = 0; f < 4; f++) {
-        R fx = (R)(lc ? lc[f * LIMC_LD] : ldg(COL(m.fxo, f) + i));
-        R fy = (R)(lc ? lc[(4 + f) * LIMC_LD] : ldg(COL(m.fxo, 4 + f) + i));
-        R fz = (R)(lc ? lc[(8 + f) * LIMC_LD] : ldg(COL(m.fxo, 8 + f) + i));
+        R fx = (R)(lc ? lc[f * LIMC_LD] : ldg(TAB(m.fxo, f) + i));
+        R fy = (R)(lc ? lc[(4 + f) * LIMC_LD] : ldg(TAB(m.fxo, 4 + f) + i));
+        R fz = (R)(lc ? lc[(8 + f) * LIMC_LD] : ldg(TAB(m.fxo, 8 + f) + i));
         R d = fx * lg[0] + fy * lg[1] + fz * lg[2];
         R ph;
         if (d > R(0)) ph = fvenkat(dmax, d, epssq);
@@ -2099,13 +2103,13 @@ __device__ __forceinline__ unsigned grad4_body(const DevMesh& m, const DevState<
 #if HP_LSQ_TABLE
 #pragma unroll
     for (int f = 0; f < 4; f++) {
-        wt[f] = (R)ldg(COL(m.lsqa, f) + i);
-        rw[f] = mrcp_tab<F>(wt[f], (R)ldg(COL(m.lsqa, 11 + f) + i), bad);
+        wt[f] = (R)ldg(TAB(m.lsqa, f) + i);
+        rw[f] = mrcp_tab<F>(wt[f], (R)ldg(TAB(m.lsqa, 11 + f) + i), bad);
     }
-    const R a1 = (R)ldg(COL(m.lsqa, 4) + i), a2 = (R)ldg(COL(m.lsqa, 5) + i), a3 = (R)ldg(COL(m.lsqa, 6) + i);
-    const R b1 = (R)ldg(COL(m.lsqa, 7) + i), b2 = (R)ldg(COL(m.lsqa, 8) + i), b3 = (R)ldg(COL(m.lsqa, 9) + i);
-    const R dnr = (R)ldg(COL(m.lsqa, 10) + i);
-    const R rdnr_tab = (R)ldg(COL(m.lsqa, 15) + i);
+    const R a1 = (R)ldg(TAB(m.lsqa, 4) + i), a2 = (R)ldg(TAB(m.lsqa, 5) + i), a3 = (R)ldg(TAB(m.lsqa, 6) + i);
+    const R b1 = (R)ldg(TAB(m.lsqa, 7) + i), b2 = (R)ldg(TAB(m.lsqa, 8) + i), b3 = (R)ldg(TAB(m.lsqa, 9) + i);
+    const R dnr = (R)ldg(TAB(m.lsqa, 10) + i);
+    const R rdnr_tab = (R)ldg(TAB(m.lsqa, 15) + i);
 #else
 #pragma unroll
     for (int f = 0; f < 4; f++) { wt[f] = xa[f] * xa[f] + ya[f] * ya[f] + za[f] * za[f]; rw[f] = mrcp<F>(wt[f], bad); }
@@ -2160,16 +2164,23 @@ __device__ __forceinline__ unsigned grad4_body(const DevMesh& m, const DevState<
 
 // LIST = 1: the cells of m.gcells (the FP64 wall layers and their
 // neighbours) instead of all cells.
+// LIST = 1: the cells of m.gcells; 2: the leading cells of a mesh whose tables
+// have rows for those alone (see DevMesh::ldt); 0: all cells, ldt = ld (with
+// ldt read here too, 1648 against 1621 us for four launches over 983,040
+// cells).
 template <int LIST>
 __device__ __forceinline__ void k_grad4_body(DevMesh m, DevState<R> s, DevParams P, int bid) {
     const long long gt = (long long)bid * blockDim.x + threadIdx.x;
     const int q = (int)(gt & 3);
-    const int ncell = LIST ? m.ngwall : m.neles;
+    const int ncell = LIST == 1 ? m.ngwall : m.neles;
     const long long c = gt >> 2;
     const bool valid = c < ncell;
     const int k = valid ? (int)c : ncell - 1;
-    const int i = LIST ? ldg(m.gcells + k) : k;
+    const int i = LIST == 1 ? ldg(m.gcells + k) : k, tr = LIST == 1 && m.trows ? k : i;
     const bool active = valid && grad_cell(ldg(m.iblank + i));
+    const size_t tl = LIST ? (size_t)m.ldt : (size_t)m.ld;
+    (void)tr;
+    (void)tl;
 #if GRAD4_STAGED
     if constexpr (sizeof(R) == sizeof(double)) {
         __shared__ __align__(16) double sgeo[GEO_N * GEO_LD];
@@ -2183,7 +2194,7 @@ __device__ __forceinline__ void k_grad4_body(DevMesh m, DevState<R> s, DevParams
         // group 0: geometry values q, q + 4, ... of the lane's cell
 #pragma unroll
         for (int k = q; k < GEO_N; k += 4)
-            cp_async8(sgeo + k * GEO_LD + cl, k < 12 ? COL(m.dxn, k) + i : COL(m.lsqa, k - 12) + i);
+            cp_async8(sgeo + k * GEO_LD + cl, (k < 12 ? m.dxn + k * tl : m.lsqa + (k - 12) * tl) + tr);
         cp_async_commit();
         // groups 1-4: fields q, q + 4, q + 8, q + 12
         const int pcol[13] = {P_UG, P_VG, P_WG, P_TG, P_UP, P_VP, P_WP, P_TP, P_PG, P_PP, P_PHIG, P_ROG, P_ROP};
@@ -2207,7 +2218,7 @@ __device__ __forceinline__ void k_grad4_body(DevMesh m, DevState<R> s, DevParams
 #pragma unroll
         for (int f = 0; f < 4; f++) cp_async8(slim + (1 + f) * LIM_LD + tid, ql + po(nn[f]));
 #pragma unroll
-        for (int d = 0; d < 3; d++) cp_async8(slimc + (4 * d + q) * LIMC_LD + cl, COL(m.fxo, 4 * d + q) + i);
+        for (int d = 0; d < 3; d++) cp_async8(slimc + (4 * d + q) * LIMC_LD + cl, m.fxo + (4 * d + q) * tl + tr);
         if (q == 0) cp_async8(slimc + 12 * LIMC_LD + cl, m.eps2 + i);
         cp_async_commit();
         const Grad4Stage st{sgeo + cl, sgat + tid, slim + tid, slimc + cl};
@@ -2246,7 +2257,7 @@ enum { TAIL_DL = 0, TAIL_VOL = 1, TAIL_LSQB = 2, TAIL_VIS = TAIL_LSQB + NLSQB, T
 __device__ __forceinline__ const double* tail_col(const DevMesh& m, const DevState<R>& s, int k) {
     if (k == TAIL_DL) return m.dl;
     if (k == TAIL_VOL) return m.vol;
-    if (k < TAIL_VIS) return m.lsqb + (size_t)(k - TAIL_LSQB) * m.ld;
+    if (k < TAIL_VIS) return TAB(m.lsqb, k - TAIL_LSQB);
     if (k < TAIL_D24) return s.vis + (size_t)(k - TAIL_VIS) * m.ld;
     if (k < TAIL_CU) return s.d24 + (size_t)(k - TAIL_D24) * m.ld;
     if (k < TAIL_CN) return s.cu + (size_t)(k - TAIL_CU) * m.ld;
@@ -2263,7 +2274,7 @@ __device__ __forceinline__ const double* tail_col(const DevMesh& m, const DevSta
 // must wait for that vote).
 template <int F, int Z, bool NC = true, bool PF = false>
 __device__ __forceinline__ bool flux4_body(const DevMesh& m, const DevState<R>& s, const DevParams& P, int stage,
-                                           int i, int q, bool active, R* sres, const double* pf = nullptr) {
+                                           int i, int tr, int q, bool active, R* sres, const double* pf = nullptr) {
     unsigned bad = 0;
     const R* pr = s.prr;
     // PF: the cell's own values after the face evaluation come from the
@@ -2277,7 +2288,7 @@ __device__ __forceinline__ bool flux4_body(const DevMesh& m, const DevState<R>& 
     int flags;
     {
         FaceOut o;
-        face_eval<F, Z, R, NC>(m, s, P, i, q, o, bad, s.prr);
+        face_eval<F, Z, R, NC>(m, s, P, i, q, o, bad, s.prr, tr);
         if (o.wall) {
 #pragma unroll
             for (int k = 0; k < 10; k++)
@@ -2367,7 +2378,7 @@ __device__ __forceinline__ bool flux4_body(const DevMesh& m, const DevState<R>& 
         // their ranges tested) at set-up
 #undef DW
 #if HP_LSQ_TABLE
-#define LB(k) TL(TAIL_LSQB + (k), ldg(COL(m.lsqb, k) + i))
+#define LB(k) TL(TAIL_LSQB + (k), ldg(TAB(m.lsqb, k) + tr))
         if (F != 0) bad |= ldg(m.fk + i) & (FK_LSQB_RANGE | FK_AREA_RANGE);
         // face q's three quotients, by one reciprocal of its weight; every lane
         // then sums them over the faces
@@ -2495,7 +2506,7 @@ __device__ __forceinline__ void k_flux4_body(DevMesh m, DevState<R> s, DevParams
     const long long c = gt >> 2;
     const bool valid = c < ncell;
     const int k = valid ? (int)c : ncell - 1;
-    const int i = LIST ? ldg(m.wcells + k) : k;
+    const int i = LIST ? ldg(m.wcells + k) : k, tr = LIST && m.trows ? k : i;
     bool active = valid && ldg(m.iblank + i) == 1;
     if (sizeof(R) != sizeof(double) && m.nwall > 0) active = active && !ldg(m.wclass + i);
     __shared__ __align__(16) R sres[10 * FLUX4_T];
@@ -2515,23 +2526,24 @@ __device__ __forceinline__ void k_flux4_body(DevMesh m, DevState<R> s, DevParams
             }
         } else {
             const int cs = (int)(threadIdx.x >> 2) & (TAIL_LD - 1);
-            for (int k = q; k < TAIL_N; k += 4) cp_async8(stail + k * TAIL_LD + cs, tail_col(m, s, k) + i);
+            for (int k = q; k < TAIL_N; k += 4)
+                cp_async8(stail + k * TAIL_LD + cs, tail_col(m, s, k) + (k >= TAIL_LSQB && k < TAIL_VIS ? tr : i));
         }
         cp_async_commit();
         const double* pf = stail + ((threadIdx.x >> 2) & (TAIL_LD - 1));
         if constexpr (HP_FAST(2)) {
-            if (!flux4_body<1, Z, NC, true>(m, s, P, stage, i, q, active, sres, pf))
-                flux4_body<0, Z, NC, true>(m, s, P, stage, i, q, active, sres, pf);
+            if (!flux4_body<1, Z, NC, true>(m, s, P, stage, i, tr, q, active, sres, pf))
+                flux4_body<0, Z, NC, true>(m, s, P, stage, i, tr, q, active, sres, pf);
         } else {
-            flux4_body<0, Z, NC, true>(m, s, P, stage, i, q, active, sres, pf);
+            flux4_body<0, Z, NC, true>(m, s, P, stage, i, tr, q, active, sres, pf);
         }
         return;
     }
 #endif
     if constexpr (HP_FAST(2)) {
-        if (!flux4_body<1, Z, NC>(m, s, P, stage, i, q, active, sres)) flux4_body<0, Z, NC>(m, s, P, stage, i, q, active, sres);
+        if (!flux4_body<1, Z, NC>(m, s, P, stage, i, tr, q, active, sres)) flux4_body<0, Z, NC>(m, s, P, stage, i, tr, q, active, sres);
     } else {
-        flux4_body<0, Z, NC>(m, s, P, stage, i, q, active, sres);
+        flux4_body<0, Z, NC>(m, s, P, stage, i, tr, q, active, sres);
     }
     __syncwarp();   // the fused step reuses sres for its next virtual block
 }
@@ -2549,7 +2561,6 @@ __device__ __forceinline__ void k_faceflux_body(DevMesh m, DevState<R> s, DevPar
     const int t = bid * blockDim.x + threadIdx.x;
     if (t >= m.nface) return;
     const int i = ldg(m.f_i + t), f = ldg(m.f_code + t) & 3;
-    if (wall_face(m, i, f)) return;
     FaceOut o{};
     unsigned bad = 0;
     face_eval<0, Z, R, NC, true>(m, s, P, i, f, o, bad, s.prr, t);
@@ -2719,14 +2730,14 @@ __device__ __forceinline__ void visc_face(const DevMesh& m, const DevState<R>& s
 #endif
 template <int F, class PT>
 __device__ __forceinline__ void visc_face_ph(const DevMesh& m, const DevState<R>& s, const DevParams& P,
-                                             int i, int f, const int nci[4], int ph, double c[4], unsigned& bad,
+                                             int i, int tr, int f, const int nci[4], int ph, double c[4], unsigned& bad,
                                              const PT* pr) {
     const int c0 = ph ? P_UP : P_UG;          // u, v, w, T columns of the phase: c0 .. c0 + 3
     const R c23 = (R)P.c23;
-    const R scx = (R)ldg(COL(m.sc, 3 * f) + i), scy = (R)ldg(COL(m.sc, 3 * f + 1) + i),
-            scz = (R)ldg(COL(m.sc, 3 * f + 2) + i);
-    const double xf = ldg(COL(m.fcv, f) + i), yf = ldg(COL(m.fcv, 4 + f) + i),
-                 zf = ldg(COL(m.fcv, 8 + f) + i);
+    const R scx = (R)ldg(TAB(m.sc, 3 * f) + tr), scy = (R)ldg(TAB(m.sc, 3 * f + 1) + tr),
+            scz = (R)ldg(TAB(m.sc, 3 * f + 2) + tr);
+    const double xf = ldg(TAB(m.fcv, f) + tr), yf = ldg(TAB(m.fcv, 4 + f) + tr),
+                 zf = ldg(TAB(m.fcv, 8 + f) + tr);
     const int neigh = nci[f];
     R ff[4];
 #pragma unroll
@@ -2805,8 +2816,8 @@ __device__ __forceinline__ void visc_face_ph(const DevMesh& m, const DevState<R>
 
 // area vector and centroid of face f of cell i from the cell columns
 #define VISC_GEO(i, f) \
-    (R)ldg(COL(m.sc, 3 * (f)) + (i)), (R)ldg(COL(m.sc, 3 * (f) + 1) + (i)), (R)ldg(COL(m.sc, 3 * (f) + 2) + (i)), \
-    ldg(COL(m.fcv, (f)) + (i)), ldg(COL(m.fcv, 4 + (f)) + (i)), ldg(COL(m.fcv, 8 + (f)) + (i))
+    (R)ldg(TAB(m.sc, 3 * (f)) + (i)), (R)ldg(TAB(m.sc, 3 * (f) + 1) + (i)), (R)ldg(TAB(m.sc, 3 * (f) + 2) + (i)), \
+    ldg(TAB(m.fcv, (f)) + (i)), ldg(TAB(m.fcv, 4 + (f)) + (i)), ldg(TAB(m.fcv, 8 + (f)) + (i))
 
 // one thread per cell (aliased meshes)
 __global__ void __launch_bounds__(128) k_visc(DevMesh m, DevState<R> s, DevParams P) {
@@ -2889,7 +2900,7 @@ __device__ __forceinline__ void k_visc8_body(DevMesh m, DevState<R> s, DevParams
     const long long c = ((gt >> 6) << 3) + ((gt & 31) >> 2);
     const bool valid = c < ncell;
     const int k = valid ? (int)c : ncell - 1;
-    const int i = LIST ? ldg(m.wcells + k) : k;
+    const int i = LIST ? ldg(m.wcells + k) : k, tr = LIST && m.trows ? k : i;
     const bool active = valid && ldg(m.iblank + i) == 1;
     int nci[4];
 #pragma unroll
@@ -2897,8 +2908,8 @@ __device__ __forceinline__ void k_visc8_body(DevMesh m, DevState<R> s, DevParams
     for (int pass = HP_FAST(4) ? 1 : 0; pass >= 0; pass--) {
         double c[4];
         unsigned bad = 0;
-        if (pass) visc_face_ph<1>(m, s, P, i, q, nci, ph, c, bad, s.prr);
-        else visc_face_ph<0>(m, s, P, i, q, nci, ph, c, bad, s.prr);
+        if (pass) visc_face_ph<1>(m, s, P, i, tr, q, nci, ph, c, bad, s.prr);
+        else visc_face_ph<0>(m, s, P, i, tr, q, nci, ph, c, bad, s.prr);
         double acc[4];
 #pragma unroll
         for (int k = 0; k < 4; k++) acc[k] = 0.0;
@@ -2924,7 +2935,6 @@ __device__ __forceinline__ void k_facevisc_body(DevMesh m, DevState<R> s, DevPar
     const int t = bid * blockDim.x + threadIdx.x;
     if (t >= m.nface) return;
     const int i = ldg(m.f_i + t), f = ldg(m.f_code + t) & 3;
-    if (wall_face(m, i, f)) return;
     int nci[4];
 #pragma unroll
     for (int k = 0; k < 4; k++) nci[k] = ldg(COL(m.nc, k) + i);
@@ -3181,8 +3191,8 @@ __global__ void __launch_bounds__(128) k_qrs_flux(DevMesh m, DevState<R> s, DevP
     for (int f = 0; f < 4; f++) {
         if ((kinds >> (4 * f)) & FK_WALL) continue;
         const int n = ldg(COL(m.nc, f) + i);
-        const double scx = ldg(COL(m.sc, 3 * f) + i), scy = ldg(COL(m.sc, 3 * f + 1) + i),
-                     scz = ldg(COL(m.sc, 3 * f + 2) + i);
+        const double scx = ldg(COL(m.scq, 3 * f) + i), scy = ldg(COL(m.scq, 3 * f + 1) + i),
+                     scz = ldg(COL(m.scq, 3 * f + 2) + i);
         const double area = sqrt(scx * scx + scy * scy + scz * scz);
         const double enx = scx / area, eny = scy / area, enz = scz / area;
 #pragma unroll
@@ -3255,20 +3265,20 @@ __global__ void __launch_bounds__(128) k_qrs_flux(DevMesh m, DevState<R> s, DevP
 // evaluate per face and stage, compiled with the same flags.
 __global__ void __launch_bounds__(128) k_face_areas(DevMesh m) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= m.neles) return;
+    if (i >= m.trows_n) return;
 #pragma unroll
     for (int f = 0; f < 4; f++) {
-        const double scx = ldg(COL(m.sc, 3 * f) + i), scy = ldg(COL(m.sc, 3 * f + 1) + i),
-                     scz = ldg(COL(m.sc, 3 * f + 2) + i);
+        const double scx = ldg(TAB(m.sc, 3 * f) + i), scy = ldg(TAB(m.sc, 3 * f + 1) + i),
+                     scz = ldg(TAB(m.sc, 3 * f + 2) + i);
         const double area = sqrt(scx * scx + scy * scy + scz * scz);
         if (m.nrm) {
             double* out = const_cast<double*>(m.nrm);
-            COL(out, 4 * f)[i] = scx / area;
-            COL(out, 4 * f + 1)[i] = scy / area;
-            COL(out, 4 * f + 2)[i] = scz / area;
-            COL(out, 4 * f + 3)[i] = area;
+            TAB(out, 4 * f)[i] = scx / area;
+            TAB(out, 4 * f + 1)[i] = scy / area;
+            TAB(out, 4 * f + 2)[i] = scz / area;
+            TAB(out, 4 * f + 3)[i] = area;
         } else {
-            COL(const_cast<double*>(m.area), f)[i] = area;
+            TAB(const_cast<double*>(m.area), f)[i] = area;
         }
     }
 }
@@ -3278,7 +3288,7 @@ static inline unsigned grid_for(long long n, int block) {
 }
 
 static void setup(const DevMesh& m, cudaStream_t st) {
-    if (m.area || m.nrm) k_face_areas<<<grid_for(m.neles, 128), 128, 0, st>>>(m);
+    if (m.area || m.nrm) k_face_areas<<<grid_for(m.trows_n, 128), 128, 0, st>>>(m);
 }
 
 #define MARK(k) do { if (hook && hook->mark) hook->mark(hook->ctx, (k)); } while (0)
@@ -3431,8 +3441,9 @@ static void enqueue_step(const DevMesh& m, const void* stp, const DevParams& P, 
         // primitiveplusbc only)
         if (P.myorder == 2 && P.myflux != 3) {
             MARK(KK_GRAD);
-            if (m.aliased) k_grad<false><<<gf, b, 0, st>>>(m, s, P);
-            else if (sizeof(R) != sizeof(double)) k_grad<true><<<gf, b, 0, st>>>(m, s, P);
+            if (m.aliased) k_grad<false, false><<<gf, b, 0, st>>>(m, s, P);
+            else if (sizeof(R) != sizeof(double) && m.dxnf) k_grad<true, true><<<gf, b, 0, st>>>(m, s, P);
+            else if (sizeof(R) != sizeof(double)) k_grad<true, false><<<gf, b, 0, st>>>(m, s, P);
             else k_grad4<0><<<g4, 128, 0, st>>>(m, s, P);
             if (m.aliased) { MARK(KK_SERIAL); k_phi_copy_serial<<<1, 1, 0, st>>>(m, s); }
             // FP64 wall layers: FP64 gradients and limiter of those cells and

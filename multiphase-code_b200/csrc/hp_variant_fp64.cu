@@ -58,7 +58,7 @@ static DevMesh prefix_view(const DevMesh& m, int n) {
 }
 static void wall_grad(const DevMesh& m, const DevState<double>& s, const DevParams& P, cudaStream_t st) {
     if (m.ngwall <= 0) return;
-    if (m.wprefix) k_grad4<0><<<grid_for(4ll * m.ngwall, 128), 128, 0, st>>>(prefix_view(m, m.ngwall), s, P);
+    if (m.wprefix) k_grad4<2><<<grid_for(4ll * m.ngwall, 128), 128, 0, st>>>(prefix_view(m, m.ngwall), s, P);
     else k_grad4<1><<<grid_for(4ll * m.ngwall, 128), 128, 0, st>>>(m, s, P);
 }
 template <int Z>
