@@ -3485,16 +3485,13 @@ static void enqueue_step(const DevMesh& m, const void* stp, const DevParams& P, 
 // over virtual blocks of 128 threads; a grid-wide barrier separates the
 // phases.  Results are those of the separate launches bit for bit (every
 // reduction is order-free: min, max, integer sums).  For small meshes, where
-// the fixed cost of ~20 dependent launches is a large part of a step.
+// the fixed cost of 16 and more dependent launches is a large part of a step.
 // Not for aliased meshes, the five-phase model, face modes 2 and 3, overset
 // fringes, partition halos or FP64 wall layers (the host keeps the graph).
 // Built in the parity variant only (HP_FUSED_STEP): without FMA contraction
 // the bodies round the same inlined here as in their own kernels.
 
 #if HP_FUSED_STEP
-#ifndef HP_FUSED_MINB
-#define HP_FUSED_MINB 4
-#endif
 // spins of a barrier wait (each with a 64 ns sleep) before it gives up
 #ifndef HP_SYNC_SPIN_LIMIT
 #define HP_SYNC_SPIN_LIMIT (1ll << 24)
@@ -3532,9 +3529,8 @@ __device__ __forceinline__ bool grid_sync(GridSync* g) {
     return ok_s != 0;
 }
 
-template <int Z>
-__global__ void __launch_bounds__(128, HP_FUSED_MINB) k_step_fused(DevMesh m, DevState<R> s, DevParams P,
-                                                                   GridSync* g) {
+template <int Z, int MINB>
+__global__ void __launch_bounds__(128, MINB) k_step_fused(DevMesh m, DevState<R> s, DevParams P, GridSync* g) {
     const int nb = gridDim.x;
 #define PHASE(nthreads, CALL) \
     for (int vb = blockIdx.x; vb < (int)(((long long)(nthreads) + 127) / 128); vb += nb) { CALL; }
@@ -3583,6 +3579,18 @@ __global__ void __launch_bounds__(128, HP_FUSED_MINB) k_step_fused(DevMesh m, De
 #undef SYNC
 }
 
+// MINB blocks per SM.  With four, registers spill (580 bytes, HLLC-Zien 968);
+// with three nearly none do, and a block waits less between barriers, but the
+// grid makes more rounds over a phase.  Small meshes, where the four-lane
+// phases take at most four rounds of three blocks on each of 148 SMs, gain: a
+// step of 13,182 cells 176 -> 156 us, 48,000 cells 353 -> 335 (Zien 364 ->
+// 335); 63,888 cells 473 -> 487, 162,000 cells 979 -> 1058.
+static const void* fused_kernel(const DevMesh& m, const DevParams& P) {
+    const bool small = 4ll * m.neles <= 4ll * 3 * 148 * 128;
+    if (P.myflux == 1) return small ? (const void*)k_step_fused<1, 3> : (const void*)k_step_fused<1, 4>;
+    return small ? (const void*)k_step_fused<0, 3> : (const void*)k_step_fused<0, 4>;
+}
+
 // Blocks of the fused step on this device: as many as are co-resident
 // (cooperative launch), at most the largest phase's virtual blocks.
 static int fused_grid(const DevMesh& m, const DevParams& P) {
@@ -3590,9 +3598,7 @@ static int fused_grid(const DevMesh& m, const DevParams& P) {
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
         return 0;
-    cudaError_t e = P.myflux == 1
-                        ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_step_fused<1>, 128, 0)
-                        : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_step_fused<0>, 128, 0);
+    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fused_kernel(m, P), 128, 0);
     if (e != cudaSuccess || per_sm < 1) return 0;
     const long long need = (8ll * m.neles + 127) / 128;
     return (int)std::min<long long>((long long)sms * per_sm, std::max(need, 1ll));
@@ -3604,8 +3610,7 @@ static cudaError_t enqueue_fused(const DevMesh& m, const void* stp, const DevPar
     DevMesh mm = m;
     DevParams pp = P;
     void* args[] = {&mm, &s, &pp, &sync};
-    return P.myflux == 1 ? cudaLaunchCooperativeKernel((void*)k_step_fused<1>, grid, 128, args, 0, st)
-                         : cudaLaunchCooperativeKernel((void*)k_step_fused<0>, grid, 128, args, 0, st);
+    return cudaLaunchCooperativeKernel(fused_kernel(m, P), grid, 128, args, 0, st);
 }
 #else
 // variants without the fused step (built with FMA contraction)
