@@ -1950,6 +1950,7 @@ extern "C" int hp_info(const hp_handle* h, int64_t* kernels_per_step, int64_t* d
         int64_t per_stage = 1 + (h->nghosts ? 1 : 0) + grad + 1;
         if (h->aliased) per_stage += grad + 1;
         if (h->dm.nfringe > 0) per_stage += 1;
+        if (h->dm.nhalo > 0) per_stage += 1;
         if (h->dm.nface > 0)   // k_faceflux; or the scatter kernels of face modes 2 (one per colour), 3
             per_stage += h->dm.face_mode == 2 ? h->dm.ncolor : 1;
         if (h->dm.nface > 0 && !h->prm.inviscid && h->var->face_visc) n += 1;   // k_vis_gather
