@@ -80,9 +80,11 @@ typedef struct hp_params {
     double twall;            /* isothermal wall temperature (BC type 6) */
     int32_t precision;       /* HP_PREC_* */
     int32_t renumber;        /* 1: space-filling-curve cell order on device */
-    int32_t block_size;      /* threads per block of the one-thread-per-cell
-                                kernels: 0 (= 256) or a multiple of 32 in
-                                [64, 512]; hydraphase.tune picks it */
+    int32_t block_size;      /* threads per block of the primitive and ghost
+                                passes: a multiple of 32 in [64, 512], or 0:
+                                64, 128 or 256 by the number of cells (the
+                                other kernels' blocks are fixed);
+                                hydraphase.tune picks it */
     int32_t use_graph;       /* 1: capture each step in a CUDA graph; 2: one
                                 fused cooperative kernel per step (precision
                                 HP_PREC_FP64_PARITY on plain meshes: not aliased,

@@ -1264,8 +1264,6 @@ __global__ void k_gather_ghost_prims(const double* __restrict__ pr, Cols6 cols, 
     int v = (int)(t / ng), g = (int)(t - (long long)v * ng);
     dst[(size_t)v * ng + g] = pr[cols.c[v] * PR_TILE + prim_off(gid[g])];
 }
-// p[k*ld + start + i] = v and dst[k*ld + start + i] = src[k*ld + start + i],
-// k < ncol, i < count (one case's element or ghost range)
 // primitives of cells [start, start + count) set to zero
 __global__ void k_zero_prims(double* pr, int start, int count) {
     long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1281,6 +1279,8 @@ __global__ void k_gather_prims(const double* __restrict__ pr, int col0, int n, i
     const int k = (int)(t / n), i = (int)(t - (long long)k * n);
     dst[(size_t)k * n + i] = pr[(col0 + k) * PR_TILE + prim_off(idx[i])];
 }
+// p[k*ld + start + i] = v and dst[k*ld + start + i] = src[k*ld + start + i],
+// k < ncol, i < count (one case's element or ghost range)
 __global__ void k_fill_cols(double* __restrict__ p, long long ld, int ncol, int start, int count, double v) {
     long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= (long long)count * ncol) return;

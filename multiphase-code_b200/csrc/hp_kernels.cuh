@@ -1349,10 +1349,16 @@ __device__ __forceinline__ void face_eval(const DevMesh& m, const DevState<R>& s
     R tgL = (R)PLD(PCOL(pr, P_TG) + po(i)), phigL = (R)PLD(PCOL(pr, P_PHIG) + po(i));
     R upL = (R)PLD(PCOL(pr, P_UP) + po(i)), vpL = (R)PLD(PCOL(pr, P_VP) + po(i)), wpL = (R)PLD(PCOL(pr, P_WP) + po(i));
     R tpL = (R)PLD(PCOL(pr, P_TP) + po(i)), pgL = (R)PLD(PCOL(pr, P_PG) + po(i)), ppL = (R)PLD(PCOL(pr, P_PP) + po(i));
-    R ugR = (R)PLD(PCOL(pr, P_UG) + po(neigh)), vgR = (R)PLD(PCOL(pr, P_VG) + po(neigh)), wgR = (R)PLD(PCOL(pr, P_WG) + po(neigh));
+    R ugR = (R)PLD(PCOL(pr, P_UG) + po(neigh)),
+      vgR = (R)PLD(PCOL(pr, P_VG) + po(neigh)),
+      wgR = (R)PLD(PCOL(pr, P_WG) + po(neigh));
     R tgR = (R)PLD(PCOL(pr, P_TG) + po(neigh)), phigR = (R)PLD(PCOL(pr, P_PHIG) + po(neigh));
-    R upR = (R)PLD(PCOL(pr, P_UP) + po(neigh)), vpR = (R)PLD(PCOL(pr, P_VP) + po(neigh)), wpR = (R)PLD(PCOL(pr, P_WP) + po(neigh));
-    R tpR = (R)PLD(PCOL(pr, P_TP) + po(neigh)), pgR = (R)PLD(PCOL(pr, P_PG) + po(neigh)), ppR = (R)PLD(PCOL(pr, P_PP) + po(neigh));
+    R upR = (R)PLD(PCOL(pr, P_UP) + po(neigh)),
+      vpR = (R)PLD(PCOL(pr, P_VP) + po(neigh)),
+      wpR = (R)PLD(PCOL(pr, P_WP) + po(neigh));
+    R tpR = (R)PLD(PCOL(pr, P_TP) + po(neigh)),
+      pgR = (R)PLD(PCOL(pr, P_PG) + po(neigh)),
+      ppR = (R)PLD(PCOL(pr, P_PP) + po(neigh));
     // alpha_p.  The reference forms it as 1 - alpha_g after reconstruction
     // (src/sr_hllcbatten.F90:226-227), which the FP64 variants keep.  In FP32
     // that difference loses everything where the water is a trace: with
@@ -2266,12 +2272,12 @@ __device__ __forceinline__ const double* tail_col(const DevMesh& m, const DevSta
 
 // Residual + sources + RK update with four lanes per cell: lane q evaluates
 // face q; the four faces' fluxes meet in shared memory (sres), and lane q sums
-// variables q, q+4, q+8 over the faces in order, adds their sources and
-// updates them.  (Every lane re-assembling all ten through shuffles took 80
-// of them and 40 additions: 983,040 cells, 802 us a launch against 703.)  F selects the division
-// form (see mdiv).  The fast form returns false, before any store, when a lane
-// of the warp flagged an operand (cn is read and written here, so the stores
-// must wait for that vote).
+// variables q, q+4, q+8 over the faces in order, adds their sources and updates
+// them.  (Every lane re-assembling all ten through shuffles took 80 of them and
+// 40 additions: 983,040 cells, 802 us a launch against 703.)  F selects the
+// division form (see mdiv).  The fast form returns false, before any store,
+// when a lane of the warp flagged an operand (cn is read and written here, so
+// the stores must wait for that vote).
 template <int F, int Z, bool NC = true, bool PF = false>
 __device__ __forceinline__ bool flux4_body(const DevMesh& m, const DevState<R>& s, const DevParams& P, int stage,
                                            int i, int tr, int q, bool active, R* sres, const double* pf = nullptr) {
@@ -2541,7 +2547,8 @@ __device__ __forceinline__ void k_flux4_body(DevMesh m, DevState<R> s, DevParams
     }
 #endif
     if constexpr (HP_FAST(2)) {
-        if (!flux4_body<1, Z, NC>(m, s, P, stage, i, tr, q, active, sres)) flux4_body<0, Z, NC>(m, s, P, stage, i, tr, q, active, sres);
+        if (!flux4_body<1, Z, NC>(m, s, P, stage, i, tr, q, active, sres))
+            flux4_body<0, Z, NC>(m, s, P, stage, i, tr, q, active, sres);
     } else {
         flux4_body<0, Z, NC>(m, s, P, stage, i, tr, q, active, sres);
     }
@@ -3359,11 +3366,11 @@ static void enqueue_flux(const DevMesh& m, const DevState<R>& s, const DevParams
     }
 }
 
-// Threads per block of the one-thread-per-cell kernels where the caller leaves
-// the choice (block_size 0): 256, or fewer where that would leave SMs without
-// a block (148 of them).  These kernels wait on gathers, and the warps of one
-// SM queue for its load unit: a 2,058-cell step takes 86 us with 9 blocks of
-// 256 threads in the primitive passes and 82 us with 33 of 64.
+// Threads per block of the primitive and ghost passes where the caller leaves
+// the choice (block_size 0): 256, or fewer where that would leave some of the
+// device's 148 SMs without a block.  These kernels wait on gathers, and the
+// warps of one SM queue for its load unit: a 2,058-cell step takes 86 us with 9
+// blocks of 256 threads in the primitive passes and 82 us with 33 of 64.
 static int cell_block(const DevMesh& m, int block) {
     if (block > 0) return block;
     return m.neles >= 148 * 256 ? 256 : m.neles >= 148 * 128 ? 128 : 64;
@@ -3382,9 +3389,9 @@ static void enqueue_start(const DevMesh& m, const void* stp, const DevParams& P,
 static void enqueue_step(const DevMesh& m, const void* stp, const DevParams& P, cudaStream_t st,
                          int block, const StepHook* hook) {
     const DevState<R>& s = *static_cast<const DevState<R>*>(stp);
-    // one-thread-per-cell kernels: `block` threads per block (64..512,
-    // 0 = 256); four-lane kernels and the one-thread kernels of aliased
-    // meshes: 128 (their launch bounds)
+    // primitive and ghost passes: cell_block threads per block; JST kernels,
+    // four-lane kernels and the one-thread kernels of aliased meshes: 128 (their
+    // launch bounds)
     const int cb = cell_block(m, block), b = 128;
     const unsigned ge = grid_for(m.neles, cb), gf = grid_for(m.neles, b);
     const unsigned gg = grid_for(m.nghosts > 0 ? m.nghosts : 1, cb);

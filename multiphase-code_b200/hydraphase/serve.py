@@ -121,8 +121,8 @@ class Server:
     batch_cells: cases below this size are grouped into multi-mesh batches of
         at most this many cells (0: every case on its own handle)
     max_batch: cases per batch at most
-    block_size: threads per block of the per-cell kernels: an int, a dict
-        from hydraphase.tune.size_class() to an int, or None (256)
+    block_size: threads per block of the primitive and ghost passes: an int,
+        a dict from hydraphase.tune.size_class() to an int, or None (by size)
     face_mode: hp_params.face_mode, an int or a dict by size class (None: 0)
     step_mode: hp_params.use_graph (1: graph, 2: fused step), an int or a
         dict by size class (None: 1)

@@ -4,9 +4,8 @@ for each mesh-size class, and caches the choices.
 Two levels are tuned:
 
 * **Kernels** (`tune_block_size`, `tune_face_mode`, `tune_step_mode`). These are the threads
-  per block of the one-thread-per-cell kernels (primitive recovery, JST
-  smoothing, ghost fill, and the gradients and face gathers of the
-  FP32-arithmetic variants) and, for those variants, how the HLLC fluxes
+  per block of the primitive and ghost passes and, for the FP32-arithmetic
+  variants, how the HLLC fluxes
   reach the cells: once per face with the face records gathered per cell in
   face order (mode 0), once from each side with four lanes per cell (mode 1,
   one kernel fewer per stage), once per face added to per-cell sums colour by
@@ -15,9 +14,9 @@ Two levels are tuned:
   vary between runs, with atomic adds (mode 3). Every candidate runs device-timed steps (CUDA
   events) of a representative case of the class: the best of three runs from
   the initial state, each of at least 20 ms (up to 200 steps).  The fastest
-  is kept. The four-lane kernels have their block size fixed by their launch
+  is kept. The other kernels have their block size fixed by their launch
   bounds, tuned per precision variant at build time. Last, whether a step
-  replays its ~20 kernels from a CUDA graph or runs as one fused cooperative
+  replays its 16 and more kernels from a CUDA graph or runs as one fused cooperative
   kernel (grid-wide barriers between the phases), which saves the fixed
   cost of the launches on small meshes.
 * **Serving** (`tune_serving`). These are the units in flight, the
@@ -105,7 +104,7 @@ def _ms_per_step(c, spec, steps: int, min_ms: float = 20.0, max_steps: int = 200
 
 def tune_block_size(spec, precision: int = PREC_MIXED, candidates=BLOCK_CANDIDATES, steps: int = 6,
                     use_cache: bool = True) -> tuple[int, dict]:
-    """Threads per block of the per-cell kernels for the size class of
+    """Threads per block of the primitive and ghost passes for the size class of
     `spec`; returns (best, {candidate: ms per step})."""
     key = _key(precision, size_class(spec.mesh.neles), "block_size")
     if use_cache:
