@@ -89,7 +89,7 @@ struct DevMesh {
     const double* sc;       // [12][ldt] face area vectors sc1x..sc4z
     const double* scq;      // [12][ld] the same for every cell (five-phase model, else null)
     const double* fch;      // [12][ldt] face centroids, 0.3333 factor (HLLC, VK): x of faces 1-4, then y, z
-    const double* fxo;      // [12][ldt] the same minus the cell's centroid (FP64 gradients, else null)
+    const double* fxo;      // [12][ldt] the same minus the cell's centroid (k_grad4, else null)
     // face areas or, for the Jameson flux, unit normal (x, y, z) and area of
     // face 1, then 2, 3, 4; formed on the device by the variant that reads them
     // (Variant::setup), null when the handle runs no FP64 flux kernel

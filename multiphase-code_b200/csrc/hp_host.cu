@@ -198,8 +198,8 @@ static void plan_arena(hp_handle* h, Arena& a, int neles, int nghosts, long long
     m.scq = nullptr;
     if (h->neq == 22) m.scq = cells ? m.sc : (double*)a.take(12 * (size_t)ld * D);
     m.fch = table(cells || fp64, 12);
-    m.fxo = table(fp64 && grad, 12);
-    m.dxn = table(fp64 && grad, 12);
+    m.fxo = table(fp64 && grad && !h->aliased, 12);   // (k_grad4's; aliased meshes run k_grad)
+    m.dxn = table(fp64 && grad && !h->aliased, 12);
     m.nrm = table(fp64 && h->prm.myflux == 3, 16);
     m.area = table(fp64 && h->prm.myflux != 3, 4);
     m.fcv = table((cells || fp64) && !h->prm.inviscid, 12);
@@ -367,12 +367,14 @@ static bool ghosts_aliased(const hp_mesh* mesh) {
         if (par < 1 || par > neles) return true;
     }
     // neighbours in the ghost range must be ghost slots that exist
+    int bad = 0;
+#pragma omp parallel for schedule(static) reduction(| : bad)
     for (long long e = 0; e < neles; e++)
         for (int k = 4; k < 8; k++) {
             const int j = mesh->elem[9 * e + k];
-            if (j < 1 || j > ntot || (j > neles && !seen[j])) return true;
+            bad |= j < 1 || j > ntot || (j > neles && !seen[j]);
         }
-    return false;
+    return bad != 0;
 }
 
 // Layer (1, 2, ... layers; 0: none) of each element, counted over interior
@@ -412,26 +414,33 @@ static long long mesh_faces(const hp_mesh* mesh, int layers, long long& nwall, l
     std::vector<int> layer(neles, 0);
     if (layers > 0) layer = mesh_layers(mesh, layers);
     std::vector<char> ing(neles, 0);
-    long long n = 0;
-    bool mutual = true;
+    long long n = 0, nw = 0, ng = 0;
+    int mutual = 1;
+#pragma omp parallel for schedule(static) reduction(+ : n) reduction(& : mutual)
     for (int e = 0; e < neles; e++)
         for (int k = 0; k < 4; k++) {
             const int j = mesh->elem[9 * (size_t)e + 4 + k] - 1;
             if (layer[e]) {
                 ing[e] = 1;
-                if (j < neles) ing[j] = 1;
+                if (j < neles && layer[j] == 0) {
+#pragma omp atomic write
+                    ing[j] = 1;
+                }
             }
             if (j < neles) {
                 const int32_t* r = mesh->elem + 9 * (size_t)j + 4;
-                if (r[0] != e + 1 && r[1] != e + 1 && r[2] != e + 1 && r[3] != e + 1) mutual = false;
+                mutual &= r[0] == e + 1 || r[1] == e + 1 || r[2] == e + 1 || r[3] == e + 1;
                 if (j < e) continue;
             }
             if (!(layer[e] && (j >= neles || layer[j]))) n++;
         }
+#pragma omp parallel for schedule(static) reduction(+ : nw, ng)
     for (int e = 0; e < neles; e++) {
-        nwall += layer[e] > 0;
-        ngwall += ing[e];
+        nw += layer[e] > 0;
+        ng += ing[e];
     }
+    nwall += nw;
+    ngwall += ng;
     return mutual ? std::max(n, 1LL) : 0;
 }
 

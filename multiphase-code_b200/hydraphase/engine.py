@@ -14,7 +14,7 @@ from dataclasses import dataclass
 
 import numpy as np
 
-from ._lib import (KERNEL_KINDS, HpDiag, HpMesh, HpOverset, HpParams, HydraError, PREC_FP64_PARITY, lib)
+from ._lib import (KERNEL_KINDS, HpDiag, HpMesh, HpOverset, HpParams, HydraError, PREC_FP32, PREC_FP64_PARITY, PREC_MIXED, lib)
 
 FLOW_FIELDS = (
     "pmax", "pmin", "tgmax", "tgmin", "ugmax", "ugmin", "vgmax", "vgmin", "wgmax", "wgmin",
@@ -146,19 +146,28 @@ def write_tecplot(path: str, mesh: MeshArrays, fields: np.ndarray):
     _check(lib().hp_write_tecplot(path.encode(), ctypes.byref(hm), _dp(f)))
 
 
+def _estimate_mesh(mesh: MeshArrays, params: HpParams, keep: list) -> HpMesh:
+    if params.wall_fp64_layers > 0 and params.precision in (PREC_MIXED, PREC_FP32):
+        return _hp_mesh(mesh, keep)
+    return HpMesh(mesh.nodes, mesh.neles, mesh.nghosts, 0, None, None, None, None, None)
+
+
 def estimate_batch_bytes(meshes, params: HpParams) -> int:
-    """Device bytes a Batch of these meshes would hold."""
+    """Device bytes a Batch of these meshes would hold (see estimate_bytes)."""
     keep = []
-    arr = (HpMesh * len(meshes))(*[_hp_mesh(m, keep) for m in meshes])
+    arr = (HpMesh * len(meshes))(*[_estimate_mesh(m, params, keep) for m in meshes])
     b = ctypes.c_int64()
     _check(lib().hp_estimate_batch_bytes(arr, len(meshes), ctypes.byref(params), ctypes.byref(b)))
     return int(b.value)
 
 
 def estimate_bytes(mesh: MeshArrays, params: HpParams) -> int:
-    """Device bytes a Case of this mesh and precision would hold."""
+    """Device bytes a Case of this mesh and precision would hold: an upper bound
+    from the mesh's sizes, at once; with FP64 wall layers, whose cells have to
+    be counted for it to be close, a pass over the mesh (25 ms a million
+    cells)."""
     keep = []
-    hm = _hp_mesh(mesh, keep)
+    hm = _estimate_mesh(mesh, params, keep)
     b = ctypes.c_int64()
     _check(lib().hp_estimate_bytes(ctypes.byref(hm), ctypes.byref(params), ctypes.byref(b)))
     return int(b.value)

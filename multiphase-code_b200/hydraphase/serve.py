@@ -212,6 +212,7 @@ class Server:
         active: list[_Active] = []
         rep = ServeReport()
         used = 0
+        waiting = None             # (unit, params, bytes) at the head of the queue
         t0 = time.perf_counter()
         now = lambda: time.perf_counter() - t0
         import os
@@ -227,12 +228,17 @@ class Server:
                 # FIFO admission against slots and bytes
                 while queue and len(setting_up) + len(active) < self.max_active:
                     unit = self._take_unit(queue)
-                    cells = sum(r.spec.mesh.neles for r in unit)
-                    p = self._params(unit[0].spec, cells)
-                    b = estimate_bytes(unit[0].spec.mesh, p) if len(unit) == 1 else \
-                        estimate_batch_bytes([r.spec.mesh for r in unit], p)
+                    # (a unit that waits for room is estimated once)
+                    if not (waiting and len(waiting[0]) == len(unit) and
+                            all(r is q for r, q in zip(waiting[0], unit))):
+                        p = self._params(unit[0].spec, sum(r.spec.mesh.neles for r in unit))
+                        b = estimate_bytes(unit[0].spec.mesh, p) if len(unit) == 1 else \
+                            estimate_batch_bytes([r.spec.mesh for r in unit], p)
+                        waiting = (unit, p, b)
+                    _, p, b = waiting
                     if used + b > self.budget and (setting_up or active):
                         break
+                    waiting = None
                     del queue[:len(unit)]
                     used += b
                     rep.peak_bytes = max(rep.peak_bytes, used)
