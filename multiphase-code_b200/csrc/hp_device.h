@@ -102,13 +102,14 @@ struct DevMesh {
     // (src/sr_derivative.F90:163-176,255), then the correctly rounded
     // reciprocals of the weights ([11..14]) and of the determinant ([15]);
     // LSQB for the 1/r gradient of alpha_g in the sources
-    // (src/sr_source.F90:100-117), then that of the determinant ([11])
+    // (src/sr_source.F90:100-117), then that of the determinant ([11]) and,
+    // with the Jameson flux, those of the weights ([12..15])
     const double* dxn;      // [12][ldt] centroid of neighbour f minus the
-                            // cell's (x, y, z of face 1, then 2, 3, 4; FP64
-                            // gradients, else null)
+                            // cell's (x, y, z of face 1, then 2, 3, 4; k_grad4
+                            // and the sources beside the Jameson flux, else null)
     // (null where nothing reads them: no FP64 kernels, no gradients)
     const double* lsqa;     // [NLSQ][ldt]
-    const double* lsqb;     // [NLSQB][ldt]
+    const double* lsqb;     // [NLSQB or NLSQB + 4][ldt]
     const int *g_par, *g_id, *g_type;   // [nghosts] ghost list (reference order)
     // overset fringe (nfringe = 0: none): cells, 4 donor cells each and
     // barycentric weights, [4][nfringe] column-major

@@ -199,12 +199,12 @@ static void plan_arena(hp_handle* h, Arena& a, int neles, int nghosts, long long
     if (h->neq == 22) m.scq = cells ? m.sc : (double*)a.take(12 * (size_t)ld * D);
     m.fch = table(cells || fp64, 12);
     m.fxo = table(fp64 && grad && !h->aliased, 12);   // (k_grad4's; aliased meshes run k_grad)
-    m.dxn = table(fp64 && grad && !h->aliased, 12);
+    m.dxn = table(fp64 && (grad || h->prm.myflux == 3) && !h->aliased, 12);
     m.nrm = table(fp64 && h->prm.myflux == 3, 16);
     m.area = table(fp64 && h->prm.myflux != 3, 4);
     m.fcv = table((cells || fp64) && !h->prm.inviscid, 12);
     m.lsqa = table(fp64 && grad, NLSQ);
-    m.lsqb = table(fp64, NLSQB);
+    m.lsqb = table(fp64, h->prm.myflux == 3 ? NLSQB + 4 : NLSQB);
     m.g_par = (int*)a.take((nghosts + 1) * (size_t)I); m.g_id = (int*)a.take((nghosts + 1) * (size_t)I);
     m.g_type = (int*)a.take((nghosts + 1) * (size_t)I);
     DevState<double>& s = h->ds;
@@ -290,7 +290,7 @@ struct Layout {
         gpar.assign(ng, 0); gid.assign(ng, 0); gtyp.assign(ng, 0); perm.assign(ne, 0); ghost_id.assign(ng, 0);
         for (auto* v : {&x, &y, &z, &vol, &dl, &dd, &eps2}) v->assign(ld, 0.0);
         for (auto* v : {&sc, &fch, &fcv}) v->assign(12 * ld, 0.0);
-        la.assign(NLSQ * ld, 0.0); lb.assign(NLSQB * ld, 0.0);
+        la.assign(NLSQ * ld, 0.0); lb.assign((NLSQB + 4) * ld, 0.0);
     }
 };
 
@@ -572,7 +572,7 @@ static int fill_case(const hp_mesh* mesh, const hp_params* params, Layout& L, Ca
         }
     }
     // --- static least-squares terms of the gradient and source operators ---
-    std::vector<double> lsqa(NLSQ * (size_t)(neles + 1), 0.0), lsqb(NLSQB * (size_t)(neles + 1), 0.0);
+    std::vector<double> lsqa(NLSQ * (size_t)(neles + 1), 0.0), lsqb((NLSQB + 4) * (size_t)(neles + 1), 0.0);
     auto LA = [&](int k, int i) -> double& { return lsqa[(size_t)k * (neles + 1) + i]; };
     auto LB = [&](int k, int i) -> double& { return lsqb[(size_t)k * (neles + 1) + i]; };
 #pragma omp parallel for schedule(static)
@@ -611,6 +611,7 @@ static int fill_case(const hp_mesh* mesh, const hp_params* params, Layout& L, Ca
         LB(4, i) = a1; LB(5, i) = a2; LB(6, i) = a3; LB(7, i) = b1; LB(8, i) = b2; LB(9, i) = b3;
         LB(10, i) = det3(a1, b1, b2, b1, a2, b3, b2, b3, a3);
         LB(11, i) = 1.0 / LB(10, i);
+        for (int f = 0; f < 4; f++) LB(NLSQB + f, i) = 1.0 / wb[f];   // (read with the Jameson flux)
     }
     cr.aliased = ghosts_aliased(mesh) ? 1 : 0;
     // --- internal order: space-filling curve over element centroids ---
@@ -706,7 +707,7 @@ static int fill_case(const hp_mesh* mesh, const hp_params* params, Layout& L, Ca
                 hsc[k * ld + t] = SC(k, i); hfch[k * ld + t] = FCH(k, i); hfcv[k * ld + t] = FCV(k, i);
             }
             for (int k = 0; k < NLSQ; k++) hla[k * ld + t] = LA(k, i);
-            for (int k = 0; k < NLSQB; k++) hlb[k * ld + t] = LB(k, i);
+            for (int k = 0; k < NLSQB + 4; k++) hlb[k * ld + t] = LB(k, i);
         } else {
             for (int k = 0; k < 4; k++) { hnc[k * ld + t] = map(nc[k][i]); hsnb[k * ld + t] = map(nc[k][i]); }
         }
@@ -749,10 +750,8 @@ __global__ void __launch_bounds__(128) k_table_rows(DevMesh m, FaceGeo src) {
         double a2 = 0.0;
         for (int d = 0; d < 3; d++) {
             const double dx = x[d][j] - x[d][i];
-            if (m.dxn) {
-                const_cast<double*>(m.dxn)[(3 * f + d) * lt + r] = dx;
-                const_cast<double*>(m.fxo)[(4 * d + f) * lt + r] = src.fch[(4 * d + f) * ld + i] - x[d][i];
-            }
+            if (m.dxn) const_cast<double*>(m.dxn)[(3 * f + d) * lt + r] = dx;
+            if (m.fxo) const_cast<double*>(m.fxo)[(4 * d + f) * lt + r] = src.fch[(4 * d + f) * ld + i] - x[d][i];
             const double b = fabs(dx), a = fabs(src.sc[(3 * f + d) * ld + i]);
             if (b != 0.0 && !(b >= 0x1p-100 && b < 0x1p100)) out |= FK_LSQA_RANGE | FK_LSQB_RANGE;
             if (a != 0.0 && !(a >= 0x1p-800)) out |= FK_AREA_RANGE;
@@ -1131,7 +1130,7 @@ extern "C" int hp_create_batch(const hp_mesh* meshes, int32_t ncase, const hp_pa
         if (e == cudaSuccess) e = up(dst, from, (size_t)n * m.ldt * D);
     };
     up_lsq(m.lsqa, L.la, NLSQ, rows_a);
-    up_lsq(m.lsqb, L.lb, NLSQB, rows_b);
+    up_lsq(m.lsqb, L.lb, P.myflux == 3 ? NLSQB + 4 : NLSQB, rows_b);
     if (e == cudaSuccess) {
         if (m.trows_n) k_table_rows<<<blocks_for(m.trows_n, 128), 128, 0, st>>>(m, geo);
         if (m.dxnf) k_cell_floats<<<blocks_for(neles, 128), 128, 0, st>>>(m, geo);

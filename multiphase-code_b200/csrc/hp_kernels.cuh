@@ -237,6 +237,11 @@ __device__ __forceinline__ T qshfl(T v, int q) {
 #define COL(ptr, k) ((ptr) + (size_t)(k) * (size_t)m.ld)
 // geometry table column, indexed by table row (see DevMesh::ldt)
 #define TAB(ptr, k) ((ptr) + (size_t)(k) * (size_t)m.ldt)
+// the same in the flux kernels.  In the whole-mesh kernel with the Jameson flux
+// (!WL: not one of the wall layers', so every cell has a row and ldt = ld) by
+// m.ld: 693 -> 670 us for three launches over 529,200 cells; with the HLLC
+// fluxes m.ldt is the faster of the two.
+#define FTAB(ptr, k) ((ptr) + (size_t)(k) * (size_t)(Z == 2 && !WL ? m.ld : m.ldt))
 // Primitive column k, indexed by prim_off(c).  983,040 cells against plain
 // columns: FP32 viscous terms 218 -> 180 us, FP32 gradients 326 -> 314 us
 // (three launches), FP64 viscous terms 560 -> 551 us, k_flux4 2007 -> 1998 us.
@@ -1309,7 +1314,7 @@ enum { LIM_LD = 128, LIMC_N = 13, LIMC_LD = 32 };
 // face-ordered FP32 tables: consecutive threads read consecutive words, where
 // the cell columns of four different f's gave a warp a quarter of each sector.
 // Otherwise t is the cell's table row.
-template <int F, int Z, class PT, bool NC = true, bool LIST = false>
+template <int F, int Z, class PT, bool NC = true, bool LIST = false, bool WL = false>
 __device__ __forceinline__ void face_eval(const DevMesh& m, const DevState<R>& s, const DevParams& P,
                                           int i, int f, FaceOut& o, unsigned& bad, const PT* pr, int t) {
 #define FGEO(k) (R)ldg(m.fgeo + (size_t)(k) * m.fld + t)
@@ -1321,24 +1326,26 @@ __device__ __forceinline__ void face_eval(const DevMesh& m, const DevState<R>& s
         // the Jameson flux has little else to do, and its handles have no
         // gradient tables (formed here: 1694 -> 1719 us, 983,040 cells, four
         // launches)
-        enx = ldg(TAB(m.nrm, 4 * f) + t);
-        eny = ldg(TAB(m.nrm, 4 * f + 1) + t);
-        enz = ldg(TAB(m.nrm, 4 * f + 2) + t);
-        area = ldg(TAB(m.nrm, 4 * f + 3) + t);
+        enx = ldg(FTAB(m.nrm, 4 * f) + t);
+        eny = ldg(FTAB(m.nrm, 4 * f + 1) + t);
+        enz = ldg(FTAB(m.nrm, 4 * f + 2) + t);
+        area = ldg(FTAB(m.nrm, 4 * f + 3) + t);
     } else if constexpr (sizeof(R) == 8) {
         // the area from a set-up table, and one reciprocal for the three
         // quotients (ranges tested at set-up).  The normals as a table too, 96
         // B a cell, would take 23 us off three launches of 1976 (983,040
         // cells).
-        const R scx = ldg(TAB(m.sc, 3 * f) + t), scy = ldg(TAB(m.sc, 3 * f + 1) + t), scz = ldg(TAB(m.sc, 3 * f + 2) + t);
-        area = ldg(TAB(m.area, f) + t);
+        const R scx = ldg(FTAB(m.sc, 3 * f) + t), scy = ldg(FTAB(m.sc, 3 * f + 1) + t),
+                scz = ldg(FTAB(m.sc, 3 * f + 2) + t);
+        area = ldg(FTAB(m.area, f) + t);
         const R rarea = F == 0 ? R(0) : R(1) / area;
         enx = mquo<F>(scx, area, rarea);
         eny = mquo<F>(scy, area, rarea);
         enz = mquo<F>(scz, area, rarea);
     } else {
-        const R scx = LIST ? FGEO(0) : (R)ldg(TAB(m.sc, 3 * f) + t), scy = LIST ? FGEO(1) : (R)ldg(TAB(m.sc, 3 * f + 1) + t),
-                scz = LIST ? FGEO(2) : (R)ldg(TAB(m.sc, 3 * f + 2) + t);
+        const R scx = LIST ? FGEO(0) : (R)ldg(FTAB(m.sc, 3 * f) + t),
+                scy = LIST ? FGEO(1) : (R)ldg(FTAB(m.sc, 3 * f + 1) + t),
+                scz = LIST ? FGEO(2) : (R)ldg(FTAB(m.sc, 3 * f + 2) + t);
         area = sqrt(scx * scx + scy * scy + scz * scz);
         const R rarea = mrcp<F>(area, bad);
         enx = mdiv<F>(scx, area, rarea, bad);
@@ -1448,7 +1455,7 @@ __device__ __forceinline__ void face_eval(const DevMesh& m, const DevState<R>& s
             xf0 = FGEO(3); yf0 = FGEO(4); zf0 = FGEO(5);
             xfn = FGEO(6); yfn = FGEO(7); zfn = FGEO(8);
         } else {
-            const double xf = ldg(TAB(m.fch, f) + t), yf = ldg(TAB(m.fch, 4 + f) + t), zf = ldg(TAB(m.fch, 8 + f) + t);
+            const double xf = ldg(FTAB(m.fch, f) + t), yf = ldg(FTAB(m.fch, 4 + f) + t), zf = ldg(FTAB(m.fch, 8 + f) + t);
             xf0 = (R)(xf - ldg(m.xc + i)); yf0 = (R)(yf - ldg(m.yc + i)); zf0 = (R)(zf - ldg(m.zc + i));
             xfn = (R)(xf - ldg(m.xc + neigh)); yfn = (R)(yf - ldg(m.yc + neigh)); zfn = (R)(zf - ldg(m.zc + neigh));
         }
@@ -2260,10 +2267,11 @@ __global__ void __launch_bounds__(128, HP_GRAD4_MINB) k_grad4(DevMesh m, DevStat
 enum { FLUX4_T = 128 };   // threads of the four-lane flux kernel's blocks
 enum { TAIL_DL = 0, TAIL_VOL = 1, TAIL_LSQB = 2, TAIL_VIS = TAIL_LSQB + NLSQB, TAIL_D24 = TAIL_VIS + 8,
        TAIL_CU = TAIL_D24 + 10, TAIL_CN = TAIL_CU + 10, TAIL_N = TAIL_CN + 10, TAIL_LD = 32 };
+template <int Z, bool WL>
 __device__ __forceinline__ const double* tail_col(const DevMesh& m, const DevState<R>& s, int k) {
     if (k == TAIL_DL) return m.dl;
     if (k == TAIL_VOL) return m.vol;
-    if (k < TAIL_VIS) return TAB(m.lsqb, k - TAIL_LSQB);
+    if (k < TAIL_VIS) return FTAB(m.lsqb, k - TAIL_LSQB);
     if (k < TAIL_D24) return s.vis + (size_t)(k - TAIL_VIS) * m.ld;
     if (k < TAIL_CU) return s.d24 + (size_t)(k - TAIL_D24) * m.ld;
     if (k < TAIL_CN) return s.cu + (size_t)(k - TAIL_CU) * m.ld;
@@ -2278,7 +2286,7 @@ __device__ __forceinline__ const double* tail_col(const DevMesh& m, const DevSta
 // division form (see mdiv).  The fast form returns false, before any store,
 // when a lane of the warp flagged an operand (cn is read and written here, so
 // the stores must wait for that vote).
-template <int F, int Z, bool NC = true, bool PF = false>
+template <int F, int Z, bool WL, bool NC = true, bool PF = false>
 __device__ __forceinline__ bool flux4_body(const DevMesh& m, const DevState<R>& s, const DevParams& P, int stage,
                                            int i, int tr, int q, bool active, R* sres, const double* pf = nullptr) {
     unsigned bad = 0;
@@ -2294,7 +2302,7 @@ __device__ __forceinline__ bool flux4_body(const DevMesh& m, const DevState<R>& 
     int flags;
     {
         FaceOut o;
-        face_eval<F, Z, R, NC>(m, s, P, i, q, o, bad, s.prr, tr);
+        face_eval<F, Z, R, NC, false, WL>(m, s, P, i, q, o, bad, s.prr, tr);
         if (o.wall) {
 #pragma unroll
             for (int k = 0; k < 10; k++)
@@ -2314,8 +2322,18 @@ __device__ __forceinline__ bool flux4_body(const DevMesh& m, const DevState<R>& 
     }
     // neighbour data for the alpha_g gradient of the sources
     const int nq = ldg(COL(m.nc, q) + i);
-    const double x0 = ldg(m.xc + i), y0 = ldg(m.yc + i), z0 = ldg(m.zc + i);
-    const R xq = (R)(ldg(m.xc + nq) - x0), yq = (R)(ldg(m.yc + nq) - y0), zq = (R)(ldg(m.zc + nq) - z0);
+    // (the Jameson flux, which gathers no centroids for its faces, takes the
+    // differences and the weight's reciprocal from tables: a step of 27,750
+    // cells 129.2 -> 128.1 us)
+    R xq, yq, zq, rwq = R(0);
+    if constexpr (sizeof(R) == 8 && Z == 2) {
+        xq = ldg(FTAB(m.dxn, 3 * q) + tr); yq = ldg(FTAB(m.dxn, 3 * q + 1) + tr); zq = ldg(FTAB(m.dxn, 3 * q + 2) + tr);
+        rwq = ldg(FTAB(m.lsqb, NLSQB + q) + tr);
+    } else {
+        xq = (R)(ldg(m.xc + nq) - ldg(m.xc + i));
+        yq = (R)(ldg(m.yc + nq) - ldg(m.yc + i));
+        zq = (R)(ldg(m.zc + nq) - ldg(m.zc + i));
+    }
     // alpha_g differences from the FP64 primitives (see k_grad)
     const R pq = (R)(PCOL(s.pr, P_PHIG)[po(nq)] - PCOL(s.pr, P_PHIG)[po(i)]);
     // residual of this lane's variables j = q, q + 4, q + 8 in face order 1..4
@@ -2384,12 +2402,13 @@ __device__ __forceinline__ bool flux4_body(const DevMesh& m, const DevState<R>& 
         // their ranges tested) at set-up
 #undef DW
 #if HP_LSQ_TABLE
-#define LB(k) TL(TAIL_LSQB + (k), ldg(TAB(m.lsqb, k) + tr))
+#define LB(k) TL(TAIL_LSQB + (k), ldg(FTAB(m.lsqb, k) + tr))
         if (F != 0) bad |= ldg(m.fk + i) & (FK_LSQB_RANGE | FK_AREA_RANGE);
         // face q's three quotients, by one reciprocal of its weight; every lane
         // then sums them over the faces
         mout<F, -800, 700>(pq, bad);
-        const R wq = LB(q), rwq = F == 0 ? R(0) : R(1) / wq;
+        const R wq = LB(q);
+        if constexpr (F != 0 && Z != 2) rwq = R(1) / wq;
         const R tx = mquo<F>(pq * xq, wq, rwq), ty = mquo<F>(pq * yq, wq, rwq), tz = mquo<F>(pq * zq, wq, rwq);
         const R c1 = qshfl(tx, 0) + qshfl(tx, 1) + qshfl(tx, 2) + qshfl(tx, 3);
         const R c2 = qshfl(ty, 0) + qshfl(ty, 1) + qshfl(ty, 2) + qshfl(ty, 3);
@@ -2502,17 +2521,18 @@ __device__ __forceinline__ bool flux4_body(const DevMesh& m, const DevState<R>& 
 }
 
 // LIST = 1: the cells of m.wcells (the FP64 wall layers) instead of all
-// cells.  The FP32 variants leave the cells of the wall layers (wclass) to
-// those FP64 kernels.
+// cells; 2: the leading cells, with the Jameson flux (with the HLLC fluxes 0
+// serves for them).  The FP32 variants leave the cells of the wall layers
+// (wclass) to those FP64 kernels.
 template <int Z, int LIST, bool NC = true>
 __device__ __forceinline__ void k_flux4_body(DevMesh m, DevState<R> s, DevParams P, int stage, int bid) {
     const long long gt = (long long)bid * blockDim.x + threadIdx.x;
     const int q = (int)(gt & 3);
-    const int ncell = LIST ? m.nwall : m.neles;
+    const int ncell = LIST == 1 ? m.nwall : m.neles;
     const long long c = gt >> 2;
     const bool valid = c < ncell;
     const int k = valid ? (int)c : ncell - 1;
-    const int i = LIST ? ldg(m.wcells + k) : k, tr = LIST && m.trows ? k : i;
+    const int i = LIST == 1 ? ldg(m.wcells + k) : k, tr = LIST == 1 && m.trows ? k : i;
     bool active = valid && ldg(m.iblank + i) == 1;
     if (sizeof(R) != sizeof(double) && m.nwall > 0) active = active && !ldg(m.wclass + i);
     __shared__ __align__(16) R sres[10 * FLUX4_T];
@@ -2523,34 +2543,34 @@ __device__ __forceinline__ void k_flux4_body(DevMesh m, DevState<R> s, DevParams
         // cells, the warp's 8 consecutive cells, 64 bytes per column; for a
         // cell list, lane q copies columns q, q + 4, ... of its own cell
         __shared__ __align__(16) double stail[TAIL_N * TAIL_LD];
-        if constexpr (LIST == 0) {
+        if constexpr (LIST != 1) {
             const int lane = (int)(threadIdx.x & 31), w8 = (int)((threadIdx.x >> 5) * 8);
             const long long c0 = ((long long)bid * blockDim.x + (threadIdx.x & ~31u)) >> 2;
             for (int t = lane; t < TAIL_N * 4; t += 32) {
                 const int k = t >> 2, part = t & 3;
-                cp_async16(stail + k * TAIL_LD + w8 + 2 * part, tail_col(m, s, k) + c0 + 2 * part);
+                cp_async16(stail + k * TAIL_LD + w8 + 2 * part, tail_col<Z, LIST != 0>(m, s, k) + c0 + 2 * part);
             }
         } else {
             const int cs = (int)(threadIdx.x >> 2) & (TAIL_LD - 1);
             for (int k = q; k < TAIL_N; k += 4)
-                cp_async8(stail + k * TAIL_LD + cs, tail_col(m, s, k) + (k >= TAIL_LSQB && k < TAIL_VIS ? tr : i));
+                cp_async8(stail + k * TAIL_LD + cs, tail_col<Z, LIST != 0>(m, s, k) + (k >= TAIL_LSQB && k < TAIL_VIS ? tr : i));
         }
         cp_async_commit();
         const double* pf = stail + ((threadIdx.x >> 2) & (TAIL_LD - 1));
         if constexpr (HP_FAST(2)) {
-            if (!flux4_body<1, Z, NC, true>(m, s, P, stage, i, tr, q, active, sres, pf))
-                flux4_body<0, Z, NC, true>(m, s, P, stage, i, tr, q, active, sres, pf);
+            if (!flux4_body<1, Z, LIST != 0, NC, true>(m, s, P, stage, i, tr, q, active, sres, pf))
+                flux4_body<0, Z, LIST != 0, NC, true>(m, s, P, stage, i, tr, q, active, sres, pf);
         } else {
-            flux4_body<0, Z, NC, true>(m, s, P, stage, i, tr, q, active, sres, pf);
+            flux4_body<0, Z, LIST != 0, NC, true>(m, s, P, stage, i, tr, q, active, sres, pf);
         }
         return;
     }
 #endif
     if constexpr (HP_FAST(2)) {
-        if (!flux4_body<1, Z, NC>(m, s, P, stage, i, tr, q, active, sres))
-            flux4_body<0, Z, NC>(m, s, P, stage, i, tr, q, active, sres);
+        if (!flux4_body<1, Z, LIST != 0, NC>(m, s, P, stage, i, tr, q, active, sres))
+            flux4_body<0, Z, LIST != 0, NC>(m, s, P, stage, i, tr, q, active, sres);
     } else {
-        flux4_body<0, Z, NC>(m, s, P, stage, i, tr, q, active, sres);
+        flux4_body<0, Z, LIST != 0, NC>(m, s, P, stage, i, tr, q, active, sres);
     }
     __syncwarp();   // the fused step reuses sres for its next virtual block
 }

@@ -65,7 +65,7 @@ template <int Z>
 static void wall_flux_z(const DevMesh& m, const DevState<double>& s, const DevParams& P, cudaStream_t st,
                         int stage) {
     const unsigned g = grid_for(4ll * m.nwall, 128);
-    if (m.wprefix) k_flux4<Z, 0><<<g, 128, 0, st>>>(prefix_view(m, m.nwall), s, P, stage);
+    if (m.wprefix) k_flux4<Z, Z == 2 ? 2 : 0><<<g, 128, 0, st>>>(prefix_view(m, m.nwall), s, P, stage);
     else k_flux4<Z, 1><<<g, 128, 0, st>>>(m, s, P, stage);
 }
 static void wall_flux(const DevMesh& m, const DevState<double>& s, const DevParams& P, cudaStream_t st,
